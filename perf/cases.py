@@ -31,7 +31,7 @@ def listed():
         # was linked against the reference and now links this library
         {"name": "api sign 1", "kind": "api_sign", "set": "sha256-128f-simple", "count": 1, "keys": 1,
          "min_len": 33, "max_len": 33},
-        {"name": "api verify 1", "kind": "api_verify", "set": "sha256-128f-simple", "count": 1, "keys": 1,
+        {"name": "api open 1", "kind": "api_open", "set": "sha256-128f-simple", "count": 1, "keys": 1,
          "min_len": 1024, "max_len": 1024},
         # the headline batch: one signing service, one key, 4096 short messages
         {"name": "sign 4096", "kind": "sign", "set": "sha256-128f-simple", "count": 4096, "keys": 1,
@@ -103,7 +103,7 @@ def _units(name, kind, count, keys, mlen):
     tree = (leaf << hp) + ((1 << hp) - 1) * th(2)
     if kind == "keygen":
         return count * tree
-    if "verify" in kind:
+    if kind in ("verify", "api_open"):
         steps = 7.5 * (2 * n) + 3 * 7.5
         return count * (_msg_units(name, False, mlen) + k * (th(1) + a * th(2)) + th(k) +
                         d * (steps * th(1) + th(ln) + hp * th(2)))
@@ -149,7 +149,7 @@ def _log_int(rng, lo, hi):
 
 def draw(rng):
     limit = max(work(x)["flops"] for x in listed())
-    kind = rng.choice(["api_sign", "api_verify", "sign", "sign", "verify", "verify", "keygen", "oneshot_sign", "long",
+    kind = rng.choice(["api_sign", "api_open", "sign", "sign", "verify", "verify", "keygen", "oneshot_sign", "long",
                        "mixed"])
     name = rng.choice(SET_NAMES)
     lo = rng.randint(1, 64)
@@ -162,7 +162,7 @@ def draw(rng):
     elif kind == "mixed":
         case.update(set2=rng.choice([x for x in SET_NAMES if x != name]), count=_log_int(rng, 4, 512), max_len=65536)
     elif kind in ("sign", "verify", "keygen"):
-        case["count"] = _log_int(rng, 2, 4096)
+        case["count"] = _log_int(rng, 6 if kind == "verify" else 2, 4096)
 
     def cost(x):  # verify inputs are signed first
         return work(dict(x, kind="sign"))["flops"] if x["kind"] == "verify" else work(x)["flops"]
@@ -196,7 +196,7 @@ def _dropin(name):
         L = ctypes.CDLL(c.dropin_path(name))
         p, z = ctypes.c_void_p, ctypes.c_size_t
         L.crypto_sign_signature.argtypes = [p, ctypes.POINTER(z), p, z, p]
-        L.crypto_sign_verify.argtypes = [p, z, p, z, p]
+        L.crypto_sign_open.argtypes = [p, ctypes.POINTER(ctypes.c_ulonglong), p, ctypes.c_ulonglong, p]
         _dropins[name] = L
     return _dropins[name]
 
@@ -247,8 +247,8 @@ class _Requests:
         b.download(self.sigs, None, self.status)
 
     def corrupt(self, rng):
-        """one byte of each tenth signature"""
-        bad = np.nonzero(rng.random(self.count) < 0.1)[0]
+        """one byte of each tenth signature (of every second one in a small batch)"""
+        bad = np.nonzero(rng.random(self.count) < (0.1 if self.count >= 32 else 0.5))[0]
         at = bad * self.z["sig"] + rng.integers(0, self.z["sig"], bad.size)
         self.sigs[at] ^= 1
 
@@ -277,13 +277,16 @@ def prepare(case, seed):
                 "count": case["count"], "sk": _pinned(case["count"] * z["sk"]), "pk": _pinned(case["count"] * z["pk"])}
     r = _Requests(rng, case["set"], case["count"], case["keys"], lo, hi)
     s = {"kind": kind, "r": r}
-    if "verify" in kind:
+    if kind in ("verify", "api_open"):
         b = r.batch(c.OP_SIGN)
         r.sign_into(b)
         b.close()
         if kind == "verify":
             r.corrupt(rng)
             s["batch"] = r.batch(c.OP_VERIFY)
+        else:
+            s["sm"] = np.concatenate([r.sigs, r.slab[:int(r.lens[0])]])
+            s["m"] = np.zeros_like(s["sm"])
     elif kind == "sign":
         s["batch"] = r.batch(c.OP_SIGN)
     else:
@@ -327,8 +330,9 @@ def run(state):
         rc = state["lib"].crypto_sign_signature(_at(r.sigs), ctypes.byref(n), _at(r.slab), int(r.lens[0]),
                                                 _at(state["rows"]))
         return [rc, n.value, r.sigs]
-    rc = state["lib"].crypto_sign_verify(_at(r.sigs), r.z["sig"], _at(r.slab), int(r.lens[0]), _at(r.pks))
-    return [rc]
+    n, m, sm = ctypes.c_ulonglong(), state["m"], state["sm"]
+    rc = state["lib"].crypto_sign_open(_at(m), ctypes.byref(n), _at(sm), sm.size, _at(r.pks))
+    return [rc, n.value, m[:n.value]]
 
 
 def exact(case, seed):
