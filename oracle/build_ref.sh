@@ -43,7 +43,7 @@ ARCH="${REF_ARCH:-sm_100}"
 SOURCES="common.cu address.cu rng.cu wots.cu utils.cu fors.cu sign.cu fips202.cu gpu_fips202.cu hash_shake256.cu thash_shake256.cu sha256.cu gpu_sha256.cu hash_sha256.cu thash_sha256.cu"
 LIBCRYPTO="${LIBCRYPTO:-$(ls /usr/lib/*-linux-gnu/libcrypto.so.3 2>/dev/null | head -1)}"
 
-if [ ! -d "$REF" ]; then
+if [ ! -f "$REF/sign.cu" ]; then
     [ "$IF_PRESENT" = 1 ] && exit 0
     echo "reference sources not found at $REF" >&2; exit 2
 fi
