@@ -662,7 +662,7 @@ struct Shake {
         for (int i = 0; i < L; i++) A[NL + 4 + i] = in[i];
         A[NL + 4 + L] = 0x1Full;
         A[16] ^= 0x8000000000000000ull;
-        keccak_f1600(A);
+        keccak_f1600_short(A);
 #pragma unroll
         for (int i = 0; i < NO; i++) out[i] = A[i];
     }
