@@ -61,7 +61,7 @@ __global__ void k_cmp_chain(uint32_t *out, int iters, uint32_t seed) {
         uint32_t m[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) m[i] = w[i] ^ st[i & 7];
-        cuspx::sha256_compress(st, m);
+        cuspx::sha256_compress<true>(st, m);
     }
     uint32_t acc = 0;
 #pragma unroll

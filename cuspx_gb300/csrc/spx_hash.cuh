@@ -136,7 +136,18 @@ SPX_DEV void sha256_iv(uint32_t s[8]) {
 // (Folding d into h + K + W a round early, e' = (d + h + K + W) + Sigma1 + Ch,
 // shortens the e chain by one step at one more ALU add a round; it measured
 // slower even for a warp alone on its SM: a lone verify 1.14 -> 1.20 ms.)
-template <int R0, int R1>
+//
+// AF: a' = t1 + Sigma0 + Maj as two adds on the FMA pipe instead of one IADD3,
+// 11 ALU instructions a round instead of 12.  WOTS+ chains of the simple sets,
+// bound by the ALU pipe: 18.2 -> 19.4 G F/s at n = 16, 18.0 -> 19.2 at n = 24,
+// 17.8 -> 18.7 at n = 32 (keygen of 4096 keys at 128f 1.17 -> 1.10 ms, 1024
+// signatures at 256f 25.8 -> 24.8 ms).  Robust sets keep IADD3: their second,
+// mask state leaves no registers for the longer chain (1024 signatures at
+// 192f-robust 27.4 -> 28.5 ms with AF).  Moving t1's adds as well gains
+// nothing at n <= 24 and loses 8% at n = 32, and moving the schedule's gains
+// nothing in any kernel: an IMAD takes an issue slot of its own, so two of
+// them for one IADD3 pay only where the ALU pipe is the tighter bound.
+template <int R0, int R1, bool AF>
 SPX_DEV void sha256_rounds(uint32_t st[8], uint32_t w[16]) {
     uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6], h = st[7];
 #pragma unroll
@@ -149,8 +160,11 @@ SPX_DEV void sha256_rounds(uint32_t st[8], uint32_t w[16]) {
                                                     sha_sigma1(w[(i - 2) & 15]));
         }
         // h + K is ready a round early, so the schedule word joins it on the FMA pipe
-        uint32_t t1 = add_fma(h + sha256_k(i), wi) + sha_Sigma1(e) + ((e & f) ^ (~e & g));
-        uint32_t t2 = sha_Sigma0(a) + ((a & b) | (c & (a | b)));
+        const uint32_t hk = add_fma(h + sha256_k(i), wi);
+        const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
+        const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
+        const uint32_t t1 = hk + S1 + ch;
+        const uint32_t na = AF ? add_fma(add_fma(S0, mj), t1) : t1 + (S0 + mj);
         h = g;
         g = f;
         f = e;
@@ -158,7 +172,7 @@ SPX_DEV void sha256_rounds(uint32_t st[8], uint32_t w[16]) {
         d = c;
         c = b;
         b = a;
-        a = t1 + t2;
+        a = na;
     }
     st[0] = a; st[1] = b; st[2] = c; st[3] = d; st[4] = e; st[5] = f; st[6] = g; st[7] = h;
 }
@@ -199,11 +213,12 @@ SPX_DEV void sha256_compress_kw(uint32_t s[8], const uint32_t *kw) {
 }
 
 // s <- compress(s, w); w is consumed (overwritten by the schedule).
+template <bool AF>
 SPX_DEV void sha256_compress(uint32_t s[8], uint32_t w[16]) {
     uint32_t t[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) t[i] = s[i];
-    sha256_rounds<0, 64>(t, w);
+    sha256_rounds<0, 64, AF>(t, w);
 #pragma unroll
     for (int i = 0; i < 8; i++) s[i] += t[i];
 }

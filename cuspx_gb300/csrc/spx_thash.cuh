@@ -73,6 +73,7 @@ struct Sha2 {
     static constexpr int W = N / 4;
     static constexpr bool kRobust = ROBUST;
     static constexpr int kShake = 0;
+    static constexpr bool kFmaA = !ROBUST;   // the round's form, see sha256_rounds
     // k_leaves occupancy floor for robust chains (which carry a second, mask
     // state); measured on GB300, capping registers to raise it spills and is
     // slower, so the default leaves the compiler's choice
@@ -99,7 +100,7 @@ struct Sha2 {
 #pragma unroll
         for (int i = 0; i < 16; i++) w[i] = i < W ? k.pub[i] : 0u;
         sha256_iv(k.mid);
-        sha256_compress(k.mid, w);
+        sha256_compress<kFmaA>(k.mid, w);
     }
 
     // SHA256(midstate; ADRS_c || in[L words]), truncated (thash_sha256.cu:16-34)
@@ -120,8 +121,8 @@ struct Sha2 {
         uint32_t s[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) s[i] = mid[i];
-        sha256_compress(s, m);
-        if (NB == 2) sha256_compress(s, m + 16);
+        sha256_compress<kFmaA>(s, m);
+        if (NB == 2) sha256_compress<kFmaA>(s, m + 16);
 #pragma unroll
         for (int i = 0; i < W; i++) out[i] = s[i];
     }
@@ -141,8 +142,8 @@ struct Sha2 {
         for (int i = W + 7; i < 16 * NB; i++) m[i] = 0;
         m[16 * NB - 1] = TOT * 8;
         sha256_iv(out);
-        sha256_compress(out, m);
-        if (NB == 2) sha256_compress(out, m + 16);
+        sha256_compress<kFmaA>(out, m);
+        if (NB == 2) sha256_compress<kFmaA>(out, m + 16);
     }
 
     template <int L>
@@ -192,7 +193,7 @@ struct Sha2 {
         f.a5 = a.w[5] & 0xff000000u;
 #pragma unroll
         for (int i = 0; i < 8; i++) f.st[i] = k.mid[i];
-        sha256_rounds<0, 5>(f.st, w);
+        sha256_rounds<0, 5, kFmaA>(f.st, w);
         if (ROBUST) {
             uint32_t x[16];
 #pragma unroll
@@ -200,7 +201,7 @@ struct Sha2 {
 #pragma unroll
             for (int i = 0; i < 5; i++) x[W + i] = a.w[i];
             sha256_iv(f.mst);
-            sha256_rounds<0, W + 5>(f.mst, x);
+            sha256_rounds<0, W + 5, kFmaA>(f.mst, x);
         }
     }
     // out = F(in) at hash address `hash` of the prepared chain
@@ -227,10 +228,10 @@ struct Sha2 {
             uint32_t t[8], ms[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) t[i] = f.mst[i];
-            sha256_rounds<W + 5, 64>(t, mw);
+            sha256_rounds<W + 5, 64, kFmaA>(t, mw);
 #pragma unroll
             for (int i = 0; i < 8; i++) ms[i] = t[i] + sha256_iv_word(i);
-            if (NB == 2) sha256_compress(ms, mw + 16);
+            if (NB == 2) sha256_compress<kFmaA>(ms, mw + 16);
 #pragma unroll
             for (int i = 0; i < W; i++) x[i] ^= ms[i];
         }
@@ -248,7 +249,7 @@ struct Sha2 {
         uint32_t t[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) t[i] = f.st[i];
-        sha256_rounds<5, 64>(t, m);
+        sha256_rounds<5, 64, kFmaA>(t, m);
 #pragma unroll
         for (int i = 0; i < W; i++) out[i] = t[i] + k.mid[i];
     }
@@ -266,7 +267,7 @@ struct Sha2 {
         m[15] = (N + 22) * 8;
         uint32_t s[8];
         sha256_iv(s);
-        sha256_compress(s, m);
+        sha256_compress<kFmaA>(s, m);
 #pragma unroll
         for (int i = 0; i < W; i++) out[i] = s[i];
     }
@@ -299,7 +300,7 @@ struct Sha2 {
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) w[i] = t.buf[i];
-        sha256_compress(t.st, w);
+        sha256_compress<kFmaA>(t.st, w);
         t.blocks++;
     }
     SPX_DEV static void t_word(TStream &t, uint32_t x, const KeyRegs<N> &k) {
@@ -429,7 +430,7 @@ struct Sha2 {
         for (uint64_t b = 0; b < nblocks; b++) {
             uint32_t w[16];
             next_block<P>(w, b, nblocks, bits, pre, m, mlen, nxt, have);
-            sha256_compress(st, w);
+            sha256_compress<kFmaA>(st, w);
         }
     }
 
@@ -477,21 +478,21 @@ struct Sha2 {
         sha256_iv(st);
 #pragma unroll
         for (int i = 0; i < 16; i++) w[i] = (i < W ? skprf[i] : 0u) ^ 0x36363636u;
-        sha256_compress(st, w);
+        sha256_compress<kFmaA>(st, w);
     }
     SPX_DEV static void hmac_finish(uint32_t R[W], const uint32_t inner[8], const uint32_t skprf[W]) {
         uint32_t st[8], w[16];
         sha256_iv(st);
 #pragma unroll
         for (int i = 0; i < 16; i++) w[i] = (i < W ? skprf[i] : 0u) ^ 0x5c5c5c5cu;
-        sha256_compress(st, w);
+        sha256_compress<kFmaA>(st, w);
 #pragma unroll
         for (int i = 0; i < 8; i++) w[i] = inner[i];
         w[8] = 0x80000000u;
 #pragma unroll
         for (int i = 9; i < 15; i++) w[i] = 0;
         w[15] = (64 + 32) * 8;
-        sha256_compress(st, w);
+        sha256_compress<kFmaA>(st, w);
 #pragma unroll
         for (int i = 0; i < W; i++) R[i] = st[i];
     }
@@ -550,7 +551,7 @@ struct Sha2 {
                 for (int i = 10; i < 15; i++) w[i] = 0;
                 w[15] = phase == 3 ? (64 + 32) * 8 : 36 * 8;
             }
-            sha256_compress(st, w);
+            sha256_compress<kFmaA>(st, w);
             if (phase == 0) {
                 phase = 1;
                 b = 0;
@@ -602,7 +603,7 @@ struct Sha2 {
             for (int i = 10; i < 15; i++) w[i] = 0;
             w[15] = 36 * 8;
             sha256_iv(s);
-            sha256_compress(s, w);
+            sha256_compress<kFmaA>(s, w);
             for (int i = 0; i < 32 && 32 * c + i < dgst_bytes; i++)
                 dg[32 * c + i] = (uint8_t)(s[i >> 2] >> (24 - 8 * (i & 3)));
         }

@@ -257,7 +257,7 @@ struct VerifySha2 : VerifySlot<4 * HF::W, 22, 64> {
     SPX_DEV static void run(Unit &u) {
 #pragma unroll
         for (int i = 0; i < 8; i++) u.out[i] = u.st[i];
-        sha256_rounds<0, 64>(u.out, u.blk);
+        sha256_rounds<0, 64, HF::kFmaA>(u.out, u.blk);
 #pragma unroll
         for (int i = 0; i < 8; i++) u.out[i] += u.st[i];
     }
