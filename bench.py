@@ -331,12 +331,13 @@ def main():
     vkern = vb.kernel_ms()
     vb.profile(False)
     tot = sum(m for _, m, _ in kern)
-    leaves = [(m / n) for name, m, n in kern if name == "k_leaves"][0]
+    # the chain kernel runs in chunks of trees: its time is all launches of a step
+    leaves = sum(m for name, m, _ in kern if name == "k_leaf_chains") / 3
     P = dict(n=16, d=22, hp=3)
-    leaf_ops = BATCH * P["d"] * (1 << P["hp"]) * leaf_units(SET) * OPS_PER_CMP
+    leaf_ops = BATCH * P["d"] * (1 << P["hp"]) * chain_units(SET) * OPS_PER_CMP
     achieved = leaf_ops / (leaves * 1e-3) / 1e12
     traffic = None
-    tfile = os.path.join(ROOT, "profiles", "k_leaves_sha256-128f_traffic.json")
+    tfile = os.path.join(ROOT, "profiles", "k_leaf_chains_sha256-128f_traffic.json")
     if os.path.exists(tfile):
         with open(tfile) as f:
             tj = json.load(f)
@@ -372,20 +373,20 @@ def main():
     # compression.  This engine skips two of its parts (the FORS secret PRF
     # and wots_sign's chain recomputation: ~6.5k of 113k compressions), and
     # the compiler issues fewer ALU instructions per compression than the
-    # model's ops (ncu: ALU instructions of one k_leaves launch / its
-    # compressions, profiles/k_leaves_sha256-128f_pipe.json).
+    # model's ops (ncu: ALU instructions of a k_leaf_chains launch / its
+    # compressions, profiles/k_leaf_chains_sha256-128f_pipe.json).
     m128 = unit_model(SET)
     executed = {"sign_compressions": m128["executed_sign"] + MSG_CMP_64B_SIGN,
                 "step_frac_of_mix_peak": value * (m128["executed_sign"] + MSG_CMP_64B_SIGN) * OPS_PER_CMP / peak_ops}
-    pfile = os.path.join(ROOT, "profiles", "k_leaves_sha256-128f_pipe.json")
+    pfile = os.path.join(ROOT, "profiles", "k_leaf_chains_sha256-128f_pipe.json")
     if os.path.exists(pfile):
         with open(pfile) as f:
             pj = json.load(f)
-        cmps = leaf_ops / OPS_PER_CMP   # compressions of one k_leaves launch
-        executed["k_leaves_alu_instr_per_cmp"] = pj["alu_instr_per_cmp"]
-        executed["k_leaves_alu_pipe_frac"] = cmps * pj["alu_instr_per_cmp"] / (leaves * 1e-3) / peak_alu
+        cmps = leaf_ops / OPS_PER_CMP   # compressions of one step's chains
+        executed["k_leaf_chains_alu_instr_per_cmp"] = pj["alu_instr_per_cmp"]
+        executed["k_leaf_chains_alu_pipe_frac"] = cmps * pj["alu_instr_per_cmp"] / (leaves * 1e-3) / peak_alu
         executed["alu_source"] = "ALU-pipe instructions per compression from ncu (%s) x compressions/s of " \
-                                 "k_leaves / the measured ALU-only peak" % pj.get("capture", "k_leaves")
+                                 "k_leaf_chains / the measured ALU-only peak" % pj.get("capture", "k_leaf_chains")
 
     # ---- batched key generation (crypto_sign_seed_keypair per item) ----
     keygen = keygen_run(c, eng, sid, z, o, flush, args.steps, args.warmup, peak_ops) if rank == 0 else None
@@ -490,11 +491,11 @@ def main():
             "gpu_launches": (5 + 3) * args.steps,
             "kernels_ms": {name: round(m / n, 4) for name, m, n in kern},
             "verify_kernels_ms": {name: round(m / n, 4) for name, m, n in vkern},
-            "roofline": {"bound": "int_alu", "kernel": "k_leaves", "achieved": achieved,
+            "roofline": {"bound": "int_alu", "kernel": "k_leaf_chains", "achieved": achieved,
                          "peak": peak_ops / 1e12, "unit": "Tops/s", "frac": achieved / (peak_ops / 1e12),
                          "traffic": traffic,
-                         "work": "%d compressions x %d INT ops per launch" %
-                                 (BATCH * 176 * leaf_units(SET), OPS_PER_CMP),
+                         "work": "%d compressions x %d INT ops per step" %
+                                 (BATCH * 176 * chain_units(SET), OPS_PER_CMP),
                          "peak_source": "measured in this run on all SMs: SHA-256 round mix, 7 ALU ops "
                                         "(SHF/LOP3/IADD3) to 1 IMAD on the FMA pipe (cuspx_int_peak_mix 1)",
                          "peak_alu_only": peak_alu / 1e12,
@@ -757,10 +758,16 @@ def leaf_units(name):
     return ln * 16 + t
 
 
+def chain_units(name):
+    """Hash units of the WOTS+ chains of one XMSS leaf (leaf_units without T_len)."""
+    n = {"128": 16, "192": 24, "256": 32}[name.split("-")[1][:3]]
+    return (2 * n + 3) * 16
+
+
 def sign_sets(c, eng, peak_alu, peak_mix, count=1024, mlen=256):
     """Sign throughput of other simple sets at `count` signatures of `mlen`
-    random bytes (one key each, graph-launched batches), with k_leaves'
-    fraction of the integer peak for its hash: the SHA-256-round mix for
+    random bytes (one key each, graph-launched batches), with the chain
+    kernel's fraction of the integer peak for its hash: the SHA-256-round mix for
     SHA-256, the ALU pipe alone for Keccak-f (which puts nothing on the FMA
     pipe).  One signature per set is byte-compared with the CPU oracle."""
     import numpy as np
@@ -792,18 +799,18 @@ def sign_sets(c, eng, peak_alu, peak_mix, count=1024, mlen=256):
             sb.run(); sb.sync(); ms.append(sb.last_ms())
         sb.profile(True)
         sb.run(); sb.sync()
-        km = {k: m / n for k, m, n in sb.kernel_ms()}
+        km = {k: m for k, m, n in sb.kernel_ms()}
         sb.profile(False)
         sb.close()
         h, d = hypertree[name.split("-")[1]]
-        units = count * d * (1 << (h // d)) * leaf_units(name)
+        units = count * d * (1 << (h // d)) * chain_units(name)
         shake = name.startswith("shake")
         ops = units * (4560 if shake else OPS_PER_CMP)
-        leaves = km.get("k_leaves")
+        leaves = km.get("k_leaf_chains")
         peak = peak_alu if shake else peak_mix
         out[name] = {"sign_per_s": count / (min(ms) / 1e3), "ms_per_batch": min(ms),
-                     "k_leaves_ms": leaves,
-                     "k_leaves_frac": ops / (leaves * 1e-3) / peak if leaves else None,
+                     "k_leaf_chains_ms": leaves,
+                     "k_leaf_chains_frac": ops / (leaves * 1e-3) / peak if leaves else None,
                      "peak": "alu_only" if shake else "sha256_mix", "oracle_first_sig_agrees": ok}
     return out
 

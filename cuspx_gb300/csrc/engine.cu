@@ -79,15 +79,15 @@ void ensure_registered() { register_all(); }
 
 using namespace cuspx;
 
-// items per batch for which chain-parallel leaf scratch is allocated (the
-// largest chain_mode_max that can take effect)
-static const size_t kChainModeItems = 256;
+// Most bytes of WOTS+ chain ends that a sign or key-generation batch keeps:
+// larger batches run their trees in chunks of this size.  A chunk of 128f
+// trees is 480k leaves, 15 ms of chains, and its last, part-empty wave costs
+// about 0.5% of that; 's' sets (287 KB a tree at 128s) would otherwise want
+// 2 MB of it a signature.
+static const size_t kEndsBytes = (size_t)256 << 20;
 // items per verify batch that the speculative chain table covers (the
 // largest verify_spec_max; 64 x 22 x 35 x 16 x 16 B = 12.6 MB at 128f)
 static const int kSpecItems = 64;
-// keys per key-generation batch that the chain-parallel scratch covers
-// (16384 x 2^hp x len x n: 73 MB at 128f)
-static const size_t kKeygenChainItems = 16384;
 // messages of at least this many bytes (32 SHA-256 blocks) are hashed by the
 // two-warp message kernels of the SHA-256 sets
 static const uint64_t kPairMsgBytes = 2048;
@@ -165,8 +165,8 @@ struct cuspx_batch {
     bool long_msgs = false;    // the last upload held a message of >= kPairMsgBytes (SHA-256:
                                // hash those over two warps; both kernels read the device
                                // lengths, so the split is right whatever the flag says)
-    uint8_t *ends = nullptr;   // chain-parallel leaf scratch
-    uint32_t ends_cap = 0;
+    uint8_t *ends = nullptr;   // chain-parallel leaf scratch, for ends_trees trees
+    uint32_t ends_trees = 0;
     size_t count = 0;
     bool use_keyrow = false, use_aux = false, use_siglen = false;
     const uint8_t *bound_keys = nullptr;   // external device key table (not owned)
@@ -669,6 +669,12 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
             return fail(ctx, CUSPX_ECUDA, "side stream");
         }
     }
+    // chain ends of up to `trees` XMSS trees, in whole groups of 32 leaves
+    auto ends = [&](size_t trees) {
+        const size_t tree = ((size_t)1 << P.hp) * P.len * n;
+        b->ends_trees = (uint32_t)std::min(trees, kEndsBytes / tree);
+        A((void **)&b->ends, (((size_t)b->ends_trees << P.hp) + 31) / 32 * 32 * P.len * n);
+    };
     const size_t keyrow_bytes = op == CUSPX_OP_VERIFY ? 2 * n : 4 * n;
     A((void **)&b->keys, b->key_cap * keyrow_bytes);
     A((void **)&b->status, cap * sizeof(int32_t));
@@ -676,9 +682,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
         A((void **)&b->out, cap * 2 * n);
         A((void **)&b->leaves, cap * ((size_t)1 << P.hp) * n);
         A((void **)&b->roots, cap * n);
-        // chain-parallel scratch
-        b->ends_cap = (uint32_t)std::min<size_t>(cap, kKeygenChainItems);
-        A((void **)&b->ends, (size_t)b->ends_cap * ((size_t)1 << P.hp) * P.len * n);
+        ends(cap);
     } else {
         A((void **)&b->keyrow, cap * sizeof(uint32_t));
         A((void **)&b->msg, msg_capacity + 64);
@@ -692,9 +696,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
             A((void **)&b->leaves, cap * P.d * ((size_t)1 << P.hp) * n);
             A((void **)&b->roots, cap * P.d * n);
             A((void **)&b->chains, cap * P.d * P.len * 16 * n);
-            // chain-parallel scratch for small batches
-            b->ends_cap = (uint32_t)std::min<size_t>(cap, kChainModeItems);
-            A((void **)&b->ends, (size_t)b->ends_cap * P.d * ((size_t)1 << P.hp) * P.len * n);
+            ends(cap * P.d);
         } else {
             A((void **)&b->aux, cap * P.sig_bytes);
             A((void **)&b->siglen, cap * sizeof(uint64_t));
@@ -825,7 +827,7 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.chains = b->chains;
         A.status = b->status;
         A.ends = b->ends;
-        A.ends_cap = b->ends_cap;
+        A.ends_trees = b->ends_trees;
         ops.sign(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0,
                  (CUSPX_SIGN_FORK && b->fork.side) ? &b->fork : nullptr);
     } else if (b->op == CUSPX_OP_VERIFY) {
@@ -845,7 +847,7 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.ctr = b->ctr;
         ops.verify(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0, &b->vlists, &b->vfork);
     } else {
-        KeygenArgs K{cnt, b->keys, b->out, b->leaves, b->roots, b->ends, b->ends_cap};
+        KeygenArgs K{cnt, b->keys, b->out, b->leaves, b->roots, b->ends, b->ends_trees};
         ops.keygen(P, K, tu, b->s, pt);
     }
 }

@@ -11,8 +11,9 @@
 //                                        schedule warp + rounds warp per message
 //   k_fors_sign     2^g lanes / FORS tree leaves (PRF+F), per-lane subtree stack,
 //                                        g shuffle levels, auth path, root
-//   k_leaves        thread / XMSS leaf   WOTS+ key (len chains x 15 F) streamed into
-//                                        T_len; the signing leaf records its chains
+//   k_leaf_chains   thread / WOTS+ chain PRF and 15 F; the signing leaf records its chains
+//   k_leaf_tstream  thread / XMSS leaf   T_len over the chain ends (k_leaf_tlen in small
+//                                        batches; k_leaves: both per leaf, without scratch)
 //   k_trees         warp / XMSS tree     level-by-level reduction in shared memory,
 //                                        auth path, root (k_trees_lane: lane / tree)
 //   k_sign_finish   block / signature    FORS pk (T_k), WOTS signatures gathered
@@ -27,7 +28,7 @@
 // (k_vsort_chains + k_vsort_layer, spx_vsort.cuh); or per-layer
 // k_verify_chains + k_verify_root, or k_verify_ht (one thread per item over
 // all layers).
-// Key generation reuses k_leaves / k_trees on the top layer.
+// Key generation reuses the leaf and tree kernels on the top layer.
 //
 // Reference structure followed (CPU form): crypto_sign_signature sign.cu:1924-1994,
 // fors_sign fors.cu:107-143, treehash utils.cu:189-241, wots_gen_leaf sign.cu:87-102,
@@ -94,8 +95,8 @@ struct SignArgs {
     uint8_t *roots;            // count x d x n
     uint8_t *chains;           // count x d x len x 16 x n  (signing leaf's chain values)
     int32_t *status;           // count
-    uint8_t *ends = nullptr;   // chain-parallel scratch: ends_cap x d x 2^hp x len x n, or null
-    uint32_t ends_cap = 0;
+    uint8_t *ends = nullptr;   // chain-parallel scratch: ends_trees x 2^hp x len x n, or null
+    uint32_t ends_trees = 0;
 };
 
 // tree/leaf indices of hypertree layer L (sign.cu:1987-1988)
@@ -425,7 +426,11 @@ struct LeafArgs {
     const SignWork *work;  // null for key generation (tree 0, no signing leaf)
     uint8_t *leaves;     // [item][layer-layer0][leaf] n bytes
     uint8_t *chains;     // [item][layer][chain][16] n bytes, or null
-    uint8_t *ends;       // chain-parallel mode: [item][layer-layer0][leaf][chain] n bytes
+    // chain-parallel kernels: a launch takes trees tree0 .. tree0 + trees - 1,
+    // tree t being layer layer0 + t % nlayers of item t / nlayers
+    uint8_t *ends;       // the launch's chain ends (chain_end), n bytes each
+    uint32_t tree0, trees;
+    bool interleaved;
 };
 
 template <class HF>
@@ -485,33 +490,54 @@ __global__ void __launch_bounds__(256, HF::kLeafMinBlocks) k_leaves(SetParams P,
 }
 
 // ===========================================================================
-// XMSS leaves, chain-parallel mode (small batches): one thread per WOTS+
-// chain (wots_gen_pk's loop body, wots.cu:181-184) writes its chain end;
-// then one thread per leaf hashes the len ends with T_len.  35x (n=16) the
-// threads of k_leaves, so a few signatures still fill the GPU; the cost is
-// the chain-end round trip through memory and an idle T_len pass for most
-// lanes, which is why big batches use k_leaves.
+// XMSS leaves, chain-parallel: one thread per WOTS+ chain (wots_gen_pk's loop
+// body, wots.cu:181-184) writes its chain end; then one thread per leaf hashes
+// the len ends with T_len.
+//
+// k_leaf_chains is bound by the ALU pipe.  A chain's state is its context and
+// value alone (64 registers at 128f against 117 with the T stream of
+// k_leaves), so 8 warps instead of 4 share a scheduler, and a batch is
+// millions of equal threads, so no wave is left part empty: 19.2 G
+// compressions/s at 1024 signatures of 128f, against 17.1 in k_leaves (5.25 +
+// 0.13 ms for T_len, against 5.99); 256s-robust, 100 signatures, 43.8 against
+// 45.9 ms; SHAKE-256f, 1024, 63.4 against 66.2 ms.  The ends cross memory
+// once (99 KB a signature at 128f, 0.4% of the time at HBM rate).  Launched in
+// chunks of whole trees that the ends scratch holds.
 // ===========================================================================
+// the tree (item and layer) and leaf of the launch's leaf x
+SPX_DEV void leaf_pos(const SetParams &P, const LeafArgs &A, uint32_t x, uint32_t &item, int &L, uint32_t &j) {
+    const uint32_t t = A.tree0 + (x >> P.hp);
+    j = x & ((1u << P.hp) - 1u);
+    item = t / (uint32_t)A.nlayers;
+    L = A.layer0 + (int)(t - item * (uint32_t)A.nlayers);
+}
+
+// where chain c's end of the launch's leaf x goes: the chains of a leaf in
+// succession (k_leaf_tlen: one thread stages a leaf's values), or those of 32
+// leaves interleaved (k_leaf_tstream: a warp reads 32 leaves' value c at once)
+template <int N>
+SPX_DEV uint8_t *chain_end(const LeafArgs &A, uint32_t x, uint32_t c) {
+    constexpr uint32_t LEN = 2 * N + 3;
+    const uint64_t at = A.interleaved ? ((uint64_t)(x >> 5) * LEN + c) * 32 + (x & 31u) : (uint64_t)x * LEN + c;
+    return A.ends + at * N;
+}
+
 template <class HF>
-__global__ void k_leaf_chains(SetParams P, LeafArgs A) {
-    constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nleaf = 1u << P.hp;
-    const uint64_t per_item = (uint64_t)A.nlayers * nleaf * LEN;
-    if (gid >= (uint64_t)A.count * per_item) return;
-    const uint32_t item = (uint32_t)(gid / per_item);
-    uint32_t rem = (uint32_t)(gid % per_item);
-    const int c = (int)(rem % LEN);
-    rem /= LEN;
-    const uint32_t j = rem & (nleaf - 1);
-    const int Lr = (int)(rem >> P.hp);
-    const int L = A.layer0 + Lr;
+__global__ void __launch_bounds__(128) k_leaf_chains(SetParams P, LeafArgs A) {
+    constexpr int W = HF::W, N = 4 * W;
+    constexpr uint32_t LEN = 2 * N + 3;
+    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t x = gid / LEN, c = gid - x * LEN;
+    if (x >> P.hp >= A.trees) return;
+    uint32_t item, j;
+    int L;
+    leaf_pos(P, A, x, item, L, j);
     const uint8_t *sk = A.sk.row(item);
     KeyRegs<N> key;
     uint64_t tree_L = 0;
     uint32_t idx_L = 0xffffffffu;
     if (A.work) {
-        const SignWork wk = A.work[item];
+        const SignWork &wk = A.work[item];
         key_from_work<HF>(key, sk, sk + 2 * N, wk);
         layer_index(P, wk.tree, wk.idx_leaf, L, tree_L, idx_L);
     } else {
@@ -536,7 +562,7 @@ __global__ void k_leaf_chains(SetParams P, LeafArgs A) {
         HF::f_step(v, v, fc, s, key);
         if (rec) HF::store(chain + (uint64_t)(s + 1) * N, v);
     }
-    HF::store(A.ends + gid * N, v);
+    HF::store(chain_end<N>(A, x, c), v);
 }
 
 // T_l of m n-byte values in global memory under ADRS pa into out, by one
@@ -547,54 +573,67 @@ template <class HF>
 SPX_DEV void slot_tl(uint32_t *S, const KeyRegs<4 * HF::W> &key, const uint8_t *pub, const Adrs &pa,
                      const uint8_t *vals, int m, uint32_t out[HF::W]);
 
-// thread per WOTS+ leaf: T_len over its chain ends, through a slot of
-// slot_words shared words per thread (slot_tl; small sign batches, where the
-// thread's serial latency is what counts), or with slot_words 0 through the
-// T stream of HF::kSmemWords shared words per thread (key generation's
-// large batches, where the smaller footprint keeps more warps resident).
+// key, address and output of a T_len thread: the launch's leaf x
 template <class HF>
-__global__ void k_leaf_tlen(SetParams P, LeafArgs A, uint32_t slot_words) {
-    constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
-    extern __shared__ uint32_t smem[];
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nleaf = 1u << P.hp;
-    if (gid >= (uint64_t)A.count * A.nlayers * nleaf) return;
-    const uint32_t item = (uint32_t)(gid / ((uint64_t)A.nlayers * nleaf));
-    const uint32_t rem = (uint32_t)(gid % ((uint64_t)A.nlayers * nleaf));
-    const int L = A.layer0 + (int)(rem >> P.hp);
-    const uint32_t j = rem & (nleaf - 1);
+SPX_DEV const uint8_t *tlen_pos(const SetParams &P, const LeafArgs &A, uint32_t x, KeyRegs<4 * HF::W> &key, Adrs &pa,
+                                uint8_t *&leaf) {
+    constexpr int N = 4 * HF::W;
+    uint32_t item, j;
+    int L;
+    leaf_pos(P, A, x, item, L, j);
     const uint8_t *sk = A.sk.row(item);
-    KeyRegs<N> key;
     uint64_t tree_L = 0;
     uint32_t idx_L = 0;
     if (A.work) {
-        const SignWork wk = A.work[item];
+        const SignWork &wk = A.work[item];
         key_from_work<HF>(key, sk, sk + 2 * N, wk);
         layer_index(P, wk.tree, wk.idx_leaf, L, tree_L, idx_L);
     } else {
         HF::key_init(key, sk, sk + 2 * N);
     }
-    Adrs pa;
     adrs_zero(pa);
     adrs_layer(pa, L);
     adrs_tree(pa, tree_L);
     adrs_type(pa, ADDR_WOTSPK);
     adrs_keypair(pa, j);
+    leaf = A.leaves + ((((uint64_t)item * A.nlayers + (L - A.layer0)) << P.hp) + j) * N;
+    return sk;
+}
+
+// thread per leaf, small sign batches, where the thread's serial latency is
+// what counts: T_len through a slot of slot_words shared words (slot_tl)
+template <class HF>
+__global__ void k_leaf_tlen(SetParams P, LeafArgs A, uint32_t slot_words) {
+    constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
+    extern __shared__ uint32_t smem[];
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >> P.hp >= A.trees) return;
+    KeyRegs<N> key;
+    Adrs pa;
+    uint8_t *to;
+    const uint8_t *sk = tlen_pos<HF>(P, A, x, key, pa, to);
     uint32_t leaf[W];
-    const uint8_t *e = A.ends + gid * LEN * N;
-    if (slot_words) {
-        slot_tl<HF>(smem + threadIdx.x * slot_words, key, sk + 2 * N, pa, e, LEN, leaf);
-    } else {
-        typename HF::TStream ts;
-        HF::t_init(ts, smem + threadIdx.x * HF::kSmemWords, key, pa);
-        for (int c = 0; c < LEN; c++) {
-            uint32_t v[W];
-            HF::load(v, e + (uint64_t)c * N);
-            HF::t_absorb(ts, v, key);
-        }
-        HF::t_final(leaf, ts);
-    }
-    HF::store(A.leaves + gid * N, leaf);
+    slot_tl<HF>(smem + threadIdx.x * slot_words, key, sk + 2 * N, pa, chain_end<N>(A, x, 0), LEN, leaf);
+    HF::store(to, leaf);
+}
+
+// thread per leaf, large batches: T_len over the interleaved ends, block by
+// block in registers (HF::t_values).  A warp's 32 leaves read value c as one
+// run of 32 n bytes.  4096 keys at 128f: 0.036 ms, against 0.058 ms through
+// the T stream's shared buffer and a leaf's own 560 bytes.
+template <class HF>
+__global__ void __launch_bounds__(128) k_leaf_tstream(SetParams P, LeafArgs A) {
+    constexpr int W = HF::W, N = 4 * W, NW = N / 8, LEN = 2 * N + 3;
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >> P.hp >= A.trees) return;
+    KeyRegs<N> key;
+    Adrs pa;
+    uint8_t *to;
+    tlen_pos<HF>(P, A, x, key, pa, to);
+    const uint2 *e = reinterpret_cast<const uint2 *>(chain_end<N>(A, x, 0));
+    uint32_t leaf[W];
+    HF::template t_values<LEN>(leaf, key, pa, [&](uint32_t q) { return e[(q / NW) * (32 * NW) + q % NW]; });
+    HF::store(to, leaf);
 }
 
 // ===========================================================================

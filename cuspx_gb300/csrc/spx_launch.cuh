@@ -40,8 +40,8 @@ struct KeygenArgs {
     uint8_t *pk;       // count x 2n: written
     uint8_t *leaves;   // count x 2^hp x n scratch
     uint8_t *roots;    // count x n scratch
-    uint8_t *ends;     // chain-parallel scratch (count x 2^hp x len x n) or null
-    uint32_t ends_cap; // items the chain-parallel scratch holds
+    uint8_t *ends;        // chain-parallel scratch (ends_trees x 2^hp x len x n) or null
+    uint32_t ends_trees;
 };
 
 // Optional per-kernel timing: an event is recorded on the launch stream
@@ -160,7 +160,7 @@ struct Family {
         // is a request's (one took ~50 ms of host time and held back every
         // queued request of its class).
         cudaFuncAttributes fa;
-        const void *rest[] = {(const void *)k_sign_msg<HF>, (const void *)k_leaf_chains<HF>,
+        const void *rest[] = {(const void *)k_sign_msg<HF>, (const void *)k_leaf_chains<HF>, (const void *)k_leaf_tstream<HF>,
                               (const void *)k_trees_lane<HF>, (const void *)k_sign_finish<HF>,
                               (const void *)k_verify_msg<HF>, (const void *)k_verify_fors<HF>,
                               (const void *)k_verify_chains<HF>, (const void *)k_vsort_chains<HF>,
@@ -227,27 +227,38 @@ struct Family {
         k_trees<HF><<<ceil_div(warps, wpb), 32 * wpb, per_warp * wpb, s>>>(P, T);
     }
 
-    // XMSS leaves: one thread per leaf (k_leaves), or for small batches one
-    // thread per chain then one per leaf (k_leaf_chains + k_leaf_tlen)
-    static void leaves(const SetParams &P, const LeafArgs &L, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
-                       bool chain_mode) {
-        const uint64_t nleaves = (uint64_t)L.count * L.nlayers * (1u << P.hp);
-        if (chain_mode) {
-            constexpr int LEN = 2 * N + 3;
-            k_leaf_chains<HF><<<ceil_div(nleaves * LEN, 128), 128, 0, s>>>(P, L);
-            CUSPX_MARK(pt, "k_leaf_chains", s);
-            if (L.work) {   // signing: 32 threads per block, each with a slot of 1-5 KB
-                const uint32_t sw = VsortSmem<HF>::slot_stride(0);
-                k_leaf_tlen<HF><<<ceil_div(nleaves, 32), 32, (size_t)32 * sw * 4, s>>>(P, L, sw);
-            } else {
-                k_leaf_tlen<HF><<<ceil_div(nleaves, 64), 64, (size_t)64 * HF::kSmemWords * 4, s>>>(P, L, 0u);
-            }
-            CUSPX_MARK(pt, "k_leaf_tlen", s);
+    // XMSS leaves.  With chain-end scratch: a thread per chain, then a thread
+    // per leaf, in chunks of as many trees as the scratch holds; `latency`
+    // picks the T_len kernel of small sign batches (128f, one signature: 25
+    // against 41 us; 37: 25 against 43 us), whose shared slots keep one warp an
+    // SM, while large ones run the streaming one with every warp resident.
+    // Without scratch (ends_trees 0): a thread per leaf (k_leaves).
+    static void leaves(const SetParams &P, LeafArgs L, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
+                       uint32_t ends_trees, bool latency) {
+        const uint64_t trees = (uint64_t)L.count * L.nlayers;
+        if (ends_trees == 0) {
+            const int b = tu.leaf_block;
+            k_leaves<HF><<<ceil_div(trees << P.hp, b), b, (size_t)b * HF::kSmemWords * 4, s>>>(P, L);
+            CUSPX_MARK(pt, "k_leaves", s);
             return;
         }
-        const int b = tu.leaf_block;
-        k_leaves<HF><<<ceil_div(nleaves, b), b, (size_t)b * HF::kSmemWords * 4, s>>>(P, L);
-        CUSPX_MARK(pt, "k_leaves", s);
+        constexpr int LEN = 2 * N + 3;
+        L.interleaved = !latency;
+        for (uint64_t t = 0; t < trees; t += ends_trees) {
+            L.tree0 = (uint32_t)t;
+            L.trees = (uint32_t)(trees - t < ends_trees ? trees - t : ends_trees);
+            const uint64_t nl = (uint64_t)L.trees << P.hp;
+            k_leaf_chains<HF><<<ceil_div(nl * LEN, 128), 128, 0, s>>>(P, L);
+            CUSPX_MARK(pt, "k_leaf_chains", s);
+            if (latency) {   // 32 threads per block, each with a slot of 1-5 KB
+                const uint32_t sw = VsortSmem<HF>::slot_stride(0);
+                k_leaf_tlen<HF><<<ceil_div(nl, 32), 32, (size_t)32 * sw * 4, s>>>(P, L, sw);
+                CUSPX_MARK(pt, "k_leaf_tlen", s);
+            } else {
+                k_leaf_tstream<HF><<<ceil_div(nl, 128), 128, 0, s>>>(P, L);
+                CUSPX_MARK(pt, "k_leaf_tstream", s);
+            }
+        }
     }
 
     static void sign(const SetParams &P, const SignArgs &A, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
@@ -283,8 +294,9 @@ struct Family {
         }
         if (split) cudaEventRecord(fk->join, sf);
         {
-            LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends};
-            leaves(P, L, tu, s, pt, A.ends && A.count <= (uint32_t)tu.chain_mode_max && A.count <= A.ends_cap);
+            LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false};
+            leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? A.ends_trees : 0,
+                   A.count <= (uint32_t)tu.chain_mode_max && A.count <= 256);
         }
         {
             TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig};
@@ -437,12 +449,8 @@ struct Family {
     static void keygen(const SetParams &P, const KeygenArgs &K, const Tuning &tu, cudaStream_t s, PhaseTimer *pt) {
         if (K.count == 0) return;
         KeyRef kr{K.sk, nullptr, (uint32_t)(4 * N)};
-        LeafArgs L{K.count, P.d - 1, 1, kr, nullptr, K.leaves, nullptr, K.ends};
-        // the top layer alone is 2^hp leaves per key, so one lane per leaf
-        // leaves SMs idle up to thousands of keys (4096 keys: 1.27 ms one
-        // lane per leaf, 1.17 ms one lane per chain); chain lanes whenever
-        // the scratch holds the batch, unless chain_mode_max is 0
-        leaves(P, L, tu, s, pt, K.ends && tu.chain_mode_max > 0 && K.count <= K.ends_cap);
+        LeafArgs L{K.count, P.d - 1, 1, kr, nullptr, K.leaves, nullptr, K.ends, 0, 0, false};
+        leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? K.ends_trees : 0, false);
         TreeArgs T{K.count, P.d - 1, 1, kr, nullptr, K.leaves, K.roots, nullptr};
         trees(P, T, tu, s);
         CUSPX_MARK(pt, "k_trees", s);

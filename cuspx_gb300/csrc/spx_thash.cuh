@@ -344,6 +344,58 @@ struct Sha2 {
         for (int i = 0; i < W; i++) out[i] = t.st[i];
     }
 
+    // T_l of M n-byte values: midstate; ADRS_c || values, block by block.
+    // ld(q) gives bytes 8q .. 8q + 7 of the values (memory order).  A value
+    // word straddles two stream words (the values start at byte 22), so block
+    // j needs value words 16j - 6 .. 16j + 10; a robust set's mask block b
+    // covers value words 8b .. 8b + 7.
+    template <int M, class LD>
+    SPX_DEV static void t_values(uint32_t out[W], const KeyRegs<N> &k, const Adrs &a, LD ld) {
+        constexpr int NB = (22 + M * N + 9 + 63) / 64, Q = M * N / 8, MB = (M * N + 31) / 32;
+        uint32_t st[8], mk[24];
+#pragma unroll
+        for (int i = 0; i < 24; i++) mk[i] = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) st[i] = k.mid[i];
+#pragma unroll 1
+        for (int j = 0; j < NB; j++) {
+            uint32_t v[18], w[16];   // v[i]: value word 16j - 6 + i
+#pragma unroll
+            for (int i = 0; i < 9; i++) {
+                const int q = 8 * j - 3 + i;
+                uint2 x = make_uint2(0u, 0u);
+                if (q >= 0 && q < Q) x = ld((uint32_t)q);
+                v[2 * i] = bswap32(x.x);
+                v[2 * i + 1] = bswap32(x.y);
+            }
+            if constexpr (ROBUST) {
+                // mk: mask blocks 2j - 1 (kept from the last block), 2j, 2j + 1
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    if (2 * j + h < MB) mask_block(mk + 8 + 8 * h, k.pub, a, 2 * j + h);
+#pragma unroll
+                for (int i = 0; i < 18; i++) {
+                    const int x = 16 * j - 6 + i;
+                    if (x >= 0 && x < M * W) v[i] ^= mk[2 + i];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++) mk[i] = mk[16 + i];
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) w[i] = __funnelshift_l(v[i + 1], v[i], 16);
+            if (j == 0) {
+#pragma unroll
+                for (int i = 0; i < 5; i++) w[i] = a.w[i];
+                w[5] |= a.w[5] & 0xffff0000u;
+            }
+            if (j == (5 + M * W) / 16) w[(5 + M * W) % 16] |= 0x8000u;
+            if (j == NB - 1) w[15] = (uint32_t)(64 + 22 + M * N) * 8u;
+            sha256_compress<kFmaA>(st, w);
+        }
+#pragma unroll
+        for (int i = 0; i < W; i++) out[i] = st[i];
+    }
+
     // ---- message hashing over a message in global memory -----------------
     // word q (big-endian) of the padded stream "prefix(P words) || m || 0x80
     // || 0* || bitlen64"; m must be 4-byte aligned and readable up to the
@@ -789,6 +841,61 @@ struct Shake {
         t_flush(t);
 #pragma unroll
         for (int i = 0; i < NL; i++) { out[2 * i] = (uint32_t)t.A[i]; out[2 * i + 1] = (uint32_t)(t.A[i] >> 32); }
+    }
+
+    // T_l of M n-byte values: PUB_SEED || ADRS || values, block by block.
+    // ld(q) gives lane q of the values.  A robust set's mask lane q belongs to
+    // value lane q, so block j takes mask blocks j - 1 and j.
+    template <int M, class LD>
+    SPX_DEV static void t_values(uint32_t out[W], const KeyRegs<N> &k, const Adrs &a, LD ld) {
+        constexpr int PL = NL + 4, Q = M * NL, NB = (PL + Q) / 17 + 1, MB = (Q + 16) / 17;
+        uint64_t A[25], S[25], last[PL];   // last: the mask block before's last PL lanes
+        uint64_t al[4];
+        adrs_lanes(a, al);
+#pragma unroll
+        for (int i = 0; i < 25; i++) A[i] = S[i] = 0;
+        if constexpr (ROBUST) {
+#pragma unroll
+            for (int i = 0; i < NL; i++) S[i] = vlane(k.pub, i);
+#pragma unroll
+            for (int i = 0; i < 4; i++) S[NL + i] = al[i];
+            S[PL] = 0x1Full;
+            S[16] ^= 0x8000000000000000ull;
+#pragma unroll
+            for (int i = 0; i < PL; i++) last[i] = 0;
+        }
+#pragma unroll 1
+        for (int j = 0; j < NB; j++) {
+            if (ROBUST && j < MB) keccak_f1600(S);
+#pragma unroll
+            for (int i = 0; i < 17; i++) {
+                const int q = 17 * j + i - PL;
+                uint64_t x = 0;
+                if (q >= 0 && q < Q) {
+                    const uint2 y = ld((uint32_t)q);
+                    x = lane_of(y.x, y.y);
+                    if constexpr (ROBUST) x ^= i < PL ? last[i < PL ? i : 0] : S[i - PL < 0 ? 0 : i - PL];
+                }
+                A[i] ^= x;
+            }
+            if (ROBUST) {
+#pragma unroll
+                for (int i = 0; i < PL; i++) last[i] = S[17 - PL + i];
+            }
+            if (j == 0) {
+#pragma unroll
+                for (int i = 0; i < NL; i++) A[i] ^= vlane(k.pub, i);
+#pragma unroll
+                for (int i = 0; i < 4; i++) A[NL + i] ^= al[i];
+            }
+            if (j == NB - 1) {
+                A[(PL + Q) % 17] ^= 0x1Full;
+                A[16] ^= 0x8000000000000000ull;
+            }
+            keccak_f1600(A);
+        }
+#pragma unroll
+        for (int i = 0; i < NL; i++) { out[2 * i] = (uint32_t)A[i]; out[2 * i + 1] = (uint32_t)(A[i] >> 32); }
     }
 
     // ---- message hashing --------------------------------------------------

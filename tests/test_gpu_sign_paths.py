@@ -1,0 +1,68 @@
+"""Sign batches through each way their work is laid out: chain lanes with the
+streaming T_len (batches above chain_mode_max) in one or more chunks of trees.
+They are byte-identical to the small-batch path, which
+test_gpu_parity.py pins to the oracle, and to the oracle itself.
+"""
+import random
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HASHES = ("sha256", "shake256")
+SETS = ["%s-%s-%s" % (h, s, m) for h in HASHES for s in ("128s", "128f", "192s", "192f", "256s", "256f")
+        for m in ("simple", "robust")]
+
+
+@pytest.fixture(scope="module")
+def engine():
+    import cuspx_gb300
+    eng = cuspx_gb300.Engine(0)
+    yield eng
+    eng.close()
+
+
+def _oracle(name):
+    import spx_oracle
+    return spx_oracle.Oracle(name)
+
+
+def _requests(engine, sid, count, keys, seed):
+    import cuspx_gb300 as c
+    rng = random.Random(seed)
+    n = c.set_sizes(sid)["seed"]
+    pks, sks = engine.keypair_batch(sid, [rng.randbytes(n) for _ in range(keys)])
+    row = [i % keys if keys == count else rng.randrange(keys) for i in range(count)]
+    msgs = [rng.randbytes(rng.randrange(0, 150)) for _ in range(count)]
+    return [pks[r] for r in row], [sks[r] for r in row], msgs
+
+
+def _in_pieces(engine, sid, sks, msgs, piece=60):
+    """signatures through batches small enough for the latency mapping"""
+    out = []
+    for i in range(0, len(msgs), piece):
+        sigs, st = engine.sign_batch(sid, sks[i:i + piece], msgs[i:i + piece])
+        assert not any(st)
+        out += sigs
+    return out
+
+
+@pytest.mark.parametrize("setname", SETS)
+def test_streaming_leaves_match_latency_path(engine, setname):
+    sid = engine.set_id(setname)
+    pks, sks, msgs = _requests(engine, sid, 65, 65, 5)
+    sigs, st = engine.sign_batch(sid, sks, msgs)
+    assert not any(st)
+    assert sigs == _in_pieces(engine, sid, sks, msgs)
+    assert sigs[64] == _oracle(setname).sign(msgs[64], sks[64])
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-128s-simple", 140), ("shake256-192s-simple", 70)])
+def test_leaf_chunks(engine, setname, count):
+    """more trees than the chain-end scratch holds (256 MiB: 935 trees of
+    128s, 428 of 192s), the last chunk part full"""
+    sid = engine.set_id(setname)
+    pks, sks, msgs = _requests(engine, sid, count, count, 6)
+    sigs, st = engine.sign_batch(sid, sks, msgs)
+    assert not any(st)
+    assert sigs == _in_pieces(engine, sid, sks, msgs, 30)
