@@ -167,6 +167,8 @@ struct cuspx_batch {
                                // lengths, so the split is right whatever the flag says)
     uint8_t *ends = nullptr;   // chain-parallel leaf scratch, for ends_trees trees
     uint32_t ends_trees = 0;
+    uint8_t *fors_nodes = nullptr;
+    uint64_t fors_lanes = 0;
     size_t count = 0;
     bool use_keyrow = false, use_aux = false, use_siglen = false;
     const uint8_t *bound_keys = nullptr;   // external device key table (not owned)
@@ -697,6 +699,11 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
             A((void **)&b->roots, cap * P.d * n);
             A((void **)&b->chains, cap * P.d * P.len * 16 * n);
             ends(cap * P.d);
+            // FORS subtree roots of trees spread over more than a warp
+            // (fors_lanes stops below twice 2048 lanes an SM)
+            b->fors_lanes = std::min<uint64_t>((uint64_t)cap * P.k << std::min(P.a, kForsMaxLanes),
+                                               (uint64_t)device_sms() * 4096);
+            A((void **)&b->fors_nodes, b->fors_lanes * n);
         } else {
             A((void **)&b->aux, cap * P.sig_bytes);
             A((void **)&b->siglen, cap * sizeof(uint64_t));
@@ -828,6 +835,8 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.status = b->status;
         A.ends = b->ends;
         A.ends_trees = b->ends_trees;
+        A.fors_nodes = b->fors_nodes;
+        A.fors_lanes = b->fors_lanes;
         ops.sign(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0,
                  (CUSPX_SIGN_FORK && b->fork.side) ? &b->fork : nullptr);
     } else if (b->op == CUSPX_OP_VERIFY) {

@@ -11,6 +11,7 @@
 //                                        schedule warp + rounds warp per message
 //   k_fors_sign     2^g lanes / FORS tree leaves (PRF+F), per-lane subtree stack,
 //                                        g shuffle levels, auth path, root
+//   k_fors_top      block / FORS tree    the levels above 2^g > 32 lanes
 //   k_leaf_chains   thread / WOTS+ chain PRF and 15 F; the signing leaf records its chains
 //   k_leaf_tstream  thread / XMSS leaf   T_len over the chain ends (k_leaf_tlen in small
 //                                        batches; k_leaves: both per leaf, without scratch)
@@ -97,6 +98,8 @@ struct SignArgs {
     int32_t *status;           // count
     uint8_t *ends = nullptr;   // chain-parallel scratch: ends_trees x 2^hp x len x n, or null
     uint32_t ends_trees = 0;
+    uint8_t *fors_nodes = nullptr;   // FORS subtree roots: fors_lanes x n, or null
+    uint64_t fors_lanes = 0;
 };
 
 // tree/leaf indices of hypertree layer L (sign.cu:1987-1988)
@@ -321,15 +324,27 @@ __global__ void __launch_bounds__(128) k_sign_msg_wide(SetParams P, SignArgs A, 
 }
 
 // ===========================================================================
-// FORS sign: a group of G = 2^g lanes per (signature, tree), g in 0..5.  Lane
-// l of a group owns the contiguous subtree of 2^(a-g) leaves starting at
-// l*2^(a-g) and reduces it with a shared-memory stack (treehash,
-// utils.cu:189-241); the G subtree roots are then reduced over g shuffle
-// levels inside the group.  g = 0 is one lane per tree (no idle lanes in the
-// reduction, best for big batches); g = 5 is one warp per tree (lowest
-// latency, best for few signatures or tall trees).  Auth-path nodes are
+// FORS sign: G = 2^g lanes per (signature, tree), g in 0..min(a, 10).  Lane l
+// owns the contiguous subtree of 2^(a-g) leaves starting at l*2^(a-g) and
+// reduces it with a shared-memory stack (treehash, utils.cu:189-241).  Up to
+// g = 5 the G subtree roots are then reduced over g shuffle levels inside the
+// group; g = 0 is one lane per tree (no idle lanes in the reduction, best
+// where the trees alone fill the GPU).  Above, the roots go to A.fors_nodes
+// and k_fors_top reduces them: a tall tree of a small batch is then spread
+// over up to 1024 lanes instead of a warp (one signature at 256s-robust,
+// a = 14: 32 lanes of 512 leaves each took 15.3 ms).  Auth-path nodes are
 // written by whichever lane holds them.
 // ===========================================================================
+constexpr int kForsWarpLanes = 5, kForsMaxLanes = 10;   // log2
+
+// FORS tree address of tree t: layer 0, tree, key pair idx_leaf, type FORSTREE
+SPX_DEV void fors_adrs(Adrs &ad, const SignWork &wk) {
+    adrs_zero(ad);
+    adrs_tree(ad, wk.tree);
+    adrs_keypair(ad, wk.idx_leaf);
+    adrs_type(ad, ADDR_FORSTREE);
+}
+
 template <class HF>
 __global__ void k_fors_sign(SetParams P, SignArgs A, int g) {
     constexpr int W = HF::W, N = 4 * W;
@@ -345,7 +360,7 @@ __global__ void k_fors_sign(SetParams P, SignArgs A, int g) {
     if (!valid) tid = 0;
     const uint32_t item = (uint32_t)(tid / P.k);
     const int t = (int)(tid % P.k);
-    const SignWork wk = A.work[item];
+    const SignWork &wk = A.work[item];
     const uint8_t *sk = A.sk.row(item);
     KeyRegs<N> key;
     key_from_work<HF>(key, sk, sk + 2 * N, wk);
@@ -354,47 +369,22 @@ __global__ void k_fors_sign(SetParams P, SignArgs A, int g) {
     const uint32_t per = 1u << sub;
     const uint32_t off = (uint32_t)t << P.a;   // idx_offset
     uint8_t *sigt = A.sig + (uint64_t)item * P.sig_bytes + N + (uint64_t)t * (P.a + 1) * N;
+    Adrs ad;
+    fors_adrs(ad, wk);
 
-    Adrs ad;  // FORS tree address: layer 0, tree, key pair idx_leaf, type FORSTREE
-    adrs_zero(ad);
-    adrs_tree(ad, wk.tree);
-    adrs_keypair(ad, wk.idx_leaf);
-    adrs_type(ad, ADDR_FORSTREE);
-
-    // per-lane stack: sub+1 entries of W words (heights in registers/local)
-    uint32_t *stk = smem + threadIdx.x * (sub + 1) * W;
-    int heights[17];
-    int sp = 0;
     uint32_t v[W];
-    for (uint32_t jj = 0; jj < per; jj++) {
-        const uint32_t j = lane * per + jj;
-        adrs_height(ad, 0);
-        adrs_index(ad, off + j);
-        uint32_t skv[W];
-        HF::PRF(skv, ad, key);
-        if (valid && j == idx) HF::store(sigt, skv);
-        HF::F(v, skv, ad, key);
-        if (valid && (idx ^ 1u) == j) HF::store(sigt + N, v);
-        int hgt = 0;
-        // merge equal-height nodes on the stack
-        while (sp > 0 && heights[sp - 1] == hgt) {
-            uint32_t l[W];
-#pragma unroll
-            for (int q = 0; q < W; q++) l[q] = stk[(sp - 1) * W + q];
-            const uint32_t tidx = j >> (hgt + 1);
-            adrs_height(ad, hgt + 1);
-            adrs_index(ad, tidx + (off >> (hgt + 1)));
-            HF::H(v, l, v, ad, key);
-            sp--;
-            hgt++;
-            if (valid && ((idx >> hgt) ^ 1u) == tidx) HF::store(sigt + N + (uint64_t)hgt * N, v);
-        }
-#pragma unroll
-        for (int q = 0; q < W; q++) stk[sp * W + q] = v[q];
-        heights[sp] = hgt;
-        sp++;
-    }
+    HF::fors_subtree(v, ad, key, lane * per, sub, off, smem + threadIdx.x * (sub + 1) * W,
+                     [&](uint32_t j, const uint32_t *x) {
+                         if (valid && j == idx) HF::store(sigt, x);
+                     },
+                     [&](int hgt, uint32_t i, const uint32_t *x) {
+                         if (valid && ((idx >> hgt) ^ 1u) == i) HF::store(sigt + N + (uint64_t)hgt * N, x);
+                     });
     // v = this lane's subtree root at height `sub`, index lane
+    if (g > kForsWarpLanes) {
+        if (valid) HF::store(A.fors_nodes + gid * N, v);
+        return;
+    }
     for (int s = 0; s < g; s++) {
         const int hgt = sub + s;
         const uint32_t q = lane >> s;
@@ -410,6 +400,72 @@ __global__ void k_fors_sign(SetParams P, SignArgs A, int g) {
         }
     }
     if (valid && lane == 0) HF::store(A.fors_roots + ((uint64_t)item * P.k + t) * N, v);
+}
+
+// Block per FORS tree: the 2^g subtree roots of k_fors_sign (g > 5) reduced
+// level by level, in place in shared memory (2^g W words): a node's thread
+// reads both children before any thread writes the level.
+template <class HF>
+__global__ void __launch_bounds__(256) k_fors_top(SetParams P, SignArgs A, int g) {
+    constexpr int W = HF::W, N = 4 * W;
+    extern __shared__ uint32_t nodes[];
+    const uint32_t item = blockIdx.x / P.k;
+    const int t = (int)(blockIdx.x % P.k);
+    const SignWork &wk = A.work[item];
+    const uint8_t *sk = A.sk.row(item);
+    KeyRegs<N> key;
+    key_from_work<HF>(key, sk, sk + 2 * N, wk);
+    const uint32_t idx = fors_index(wk.mhash, P.a, t);
+    const uint32_t off = (uint32_t)t << P.a;
+    uint8_t *auth = A.sig + (uint64_t)item * P.sig_bytes + 2 * N + (uint64_t)t * (P.a + 1) * N;
+    const uint8_t *src = A.fors_nodes + ((uint64_t)blockIdx.x << g) * N;
+    for (uint32_t q = threadIdx.x; q < 1u << g; q += blockDim.x) {
+        uint32_t v[W];
+        HF::load(v, src + (uint64_t)q * N);
+#pragma unroll
+        for (int x = 0; x < W; x++) nodes[q * W + x] = v[x];
+    }
+    __syncthreads();
+    Adrs ad;
+    fors_adrs(ad, wk);
+    for (int hgt = P.a - g; hgt < P.a; hgt++) {
+        const uint32_t half = 1u << (P.a - hgt - 1);   // nodes of the next level
+        if (threadIdx.x == 0) {
+            uint32_t v[W];
+            const uint32_t sib = (idx >> hgt) ^ 1u;
+#pragma unroll
+            for (int x = 0; x < W; x++) v[x] = nodes[sib * W + x];
+            HF::store(auth + (uint64_t)hgt * N, v);
+        }
+        // each pass takes the next blockDim.x nodes of the level; writing node
+        // q never disturbs a later pass, which reads children 2q and up
+        for (uint32_t q0 = 0; q0 < half; q0 += blockDim.x) {
+            const uint32_t q = q0 + threadIdx.x;
+            uint32_t l[W], r[W];
+            if (q < half) {
+#pragma unroll
+                for (int x = 0; x < W; x++) {
+                    l[x] = nodes[2 * q * W + x];
+                    r[x] = nodes[(2 * q + 1) * W + x];
+                }
+                adrs_height(ad, hgt + 1);
+                adrs_index(ad, q + (off >> (hgt + 1)));
+                HF::H(l, l, r, ad, key);
+            }
+            __syncthreads();
+            if (q < half) {
+#pragma unroll
+                for (int x = 0; x < W; x++) nodes[q * W + x] = l[x];
+            }
+            __syncthreads();
+        }
+    }
+    if (threadIdx.x == 0) {
+        uint32_t v[W];
+#pragma unroll
+        for (int x = 0; x < W; x++) v[x] = nodes[x];
+        HF::store(A.fors_roots + (uint64_t)blockIdx.x * N, v);
+    }
 }
 
 // ===========================================================================
@@ -973,8 +1029,13 @@ SPX_DEV void compute_root(uint32_t root[HF::W], const uint32_t leaf[HF::W], uint
         idx_offset >>= 1;
         adrs_height(ad, i + 1);
         adrs_index(ad, leaf_idx + idx_offset);
-        if (right) HF::H(cur, sib, cur, ad, key);
-        else HF::H(cur, cur, sib, ad, key);
+        uint32_t l[W];
+#pragma unroll
+        for (int x = 0; x < W; x++) {
+            l[x] = right ? sib[x] : cur[x];
+            sib[x] = right ? cur[x] : sib[x];
+        }
+        HF::H(cur, l, sib, ad, key);
     }
 #pragma unroll
     for (int x = 0; x < W; x++) root[x] = cur[x];

@@ -161,7 +161,7 @@ struct Family {
         // queued request of its class).
         cudaFuncAttributes fa;
         const void *rest[] = {(const void *)k_sign_msg<HF>, (const void *)k_leaf_chains<HF>, (const void *)k_leaf_tstream<HF>,
-                              (const void *)k_trees_lane<HF>, (const void *)k_sign_finish<HF>,
+                              (const void *)k_trees_lane<HF>, (const void *)k_fors_top<HF>,
                               (const void *)k_verify_msg<HF>, (const void *)k_verify_fors<HF>,
                               (const void *)k_verify_chains<HF>, (const void *)k_vsort_chains<HF>,
                               (const void *)k_vspec_cand<HF>,
@@ -261,6 +261,21 @@ struct Family {
         }
     }
 
+    // log2 of the lanes per FORS tree: tu.fors_lanes_log2, more where the trees
+    // would leave SMs idle.  Within a warp, until the launch has 4 warps a
+    // scheduler (beyond, the shuffle levels' idle lanes cost more than the
+    // occupancy gives); with node scratch, tall trees over more lanes until it
+    // has 16, several rounds of blocks, since a lane of a tall tree runs for
+    // milliseconds and a part-empty last round is lost.
+    static int fors_lanes(const SetParams &P, uint64_t trees, const Tuning &tu, uint64_t nodes) {
+        const uint64_t sm = (uint64_t)device_sms();
+        int g = tu.fors_lanes_log2 < P.a ? tu.fors_lanes_log2 : P.a;
+        while (g < kForsWarpLanes && g < P.a && (trees << g) < sm * 512) g++;
+        if (g == kForsWarpLanes)
+            while (g < kForsMaxLanes && g < P.a && (trees << g) < sm * 2048 && (trees << (g + 1)) <= nodes) g++;
+        return g;
+    }
+
     static void sign(const SetParams &P, const SignArgs &A, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
                      uint64_t long_msg, const StreamFork *fk) {
         if (A.count == 0) return;
@@ -283,14 +298,15 @@ struct Family {
         }
         {
             const int b = tu.fors_block;
-            // small batches: spread each tree over more lanes until the launch
-            // has about one full wave of threads (SMs x 128), for latency
-            const uint64_t wave = (uint64_t)device_sms() * 128;
-            int g = tu.fors_lanes_log2 < P.a ? tu.fors_lanes_log2 : P.a;
-            while (g < 5 && g < P.a && (((uint64_t)A.count * P.k) << g) < wave) g++;
-            const uint64_t threads = (((uint64_t)A.count * P.k) << g);
-            k_fors_sign<HF><<<ceil_div(threads, b), b, (size_t)b * (P.a - g + 1) * W * 4, sf>>>(P, A, g);
+            const uint64_t trees = (uint64_t)A.count * P.k;
+            const int g = fors_lanes(P, trees, tu, A.fors_nodes ? A.fors_lanes : 0);
+            k_fors_sign<HF><<<ceil_div(trees << g, b), b, (size_t)b * (P.a - g + 1) * W * 4, sf>>>(P, A, g);
             CUSPX_MARK(pt, "k_fors_sign", s);
+            if (g > kForsWarpLanes) {
+                const unsigned tb = g > 8 ? 256u : 1u << (g - 1);
+                k_fors_top<HF><<<(unsigned)trees, tb, (size_t)W * 4 << g, sf>>>(P, A, g);
+                CUSPX_MARK(pt, "k_fors_top", s);
+            }
         }
         if (split) cudaEventRecord(fk->join, sf);
         {

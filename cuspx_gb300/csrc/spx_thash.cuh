@@ -103,11 +103,29 @@ struct Sha2 {
         sha256_compress<kFmaA>(k.mid, w);
     }
 
-    // SHA256(midstate; ADRS_c || in[L words]), truncated (thash_sha256.cu:16-34)
+    // ---- thash as a sequence of compressions --------------------------------
+    // thash over L words is kUnits<L> compressions: robust sets first draw
+    // each bitmask block (kMaskUnits of them per 8 input words), then the
+    // message's blocks follow.  They run through one compression call site
+    // with a loop around it: a site is 20 KB of unrolled rounds, and a kernel
+    // with several on its hot path waits for instructions: FORS trees with
+    // PRF, F and H each on their own kept the ALU pipe 74% (128f), 54% (192f)
+    // and 57% (256f-robust) busy, with 4.6 to 6.7 cycles of `no_instruction`
+    // an issue; 1024 signatures of 192f took 3.00 ms there, through one site
+    // 2.10 ms, 100 of 256s-robust 34 and 22 ms.  (Rolling the rounds instead
+    // is slower: 16.2 against 16.7 G compressions/s.)
     template <int L>
-    SPX_DEV static void core(uint32_t out[W], const uint32_t mid[8], const Adrs &a, const uint32_t in[L]) {
-        constexpr int TOT = 22 + 4 * L;
-        constexpr int NB = (TOT + 9 + 63) / 64;
+    static constexpr int kBlocks = (22 + 4 * L + 9 + 63) / 64;
+    static constexpr int kMaskUnits = (N + 26 + 9 + 63) / 64;
+    template <int L>
+    static constexpr int kMaskAll = ROBUST ? (L + 7) / 8 * kMaskUnits : 0;
+    template <int L>
+    static constexpr int kUnits = kMaskAll<L> + kBlocks<L>;
+
+    // block b of SHA256(midstate; ADRS_c || in[L words]) (thash_sha256.cu:16-34)
+    template <int L>
+    SPX_DEV static void core_block(uint32_t w[16], const Adrs &a, const uint32_t in[L], int b) {
+        constexpr int NB = kBlocks<L>;
         uint32_t m[16 * NB];
 #pragma unroll
         for (int i = 0; i < 5; i++) m[i] = a.w[i];
@@ -117,48 +135,84 @@ struct Sha2 {
         m[5 + L] = (in[L - 1] << 16) | 0x8000u;
 #pragma unroll
         for (int i = 6 + L; i < 16 * NB; i++) m[i] = 0;
-        m[16 * NB - 1] = (64 + TOT) * 8;
-        uint32_t s[8];
+        m[16 * NB - 1] = (64 + 22 + 4 * L) * 8;
 #pragma unroll
-        for (int i = 0; i < 8; i++) s[i] = mid[i];
-        sha256_compress<kFmaA>(s, m);
-        if (NB == 2) sha256_compress<kFmaA>(s, m + 16);
-#pragma unroll
-        for (int i = 0; i < W; i++) out[i] = s[i];
+        for (int i = 0; i < 16; i++) w[i] = NB == 1 || b == 0 ? m[i] : m[16 * (NB - 1) + i];
     }
-
-    // MGF1-SHA256(PUB_SEED || ADRS_c, .) block `ctr` (sha256.cu:362-383)
-    SPX_DEV static void mask_block(uint32_t out[8], const uint32_t pub[W], const Adrs &a, uint32_t ctr) {
+    // compression `part` of MGF1-SHA256(PUB_SEED || ADRS_c, .) block `ctr`
+    // (sha256.cu:362-383), from the IV
+    SPX_DEV static void mask_words(uint32_t w[16], const uint32_t pub[W], const Adrs &a, uint32_t ctr, int part) {
         constexpr int TOT = N + 26;
-        constexpr int NB = (TOT + 9 + 63) / 64;
-        uint32_t m[16 * NB];
+        if (kMaskUnits == 1 || part == 0) {
 #pragma unroll
-        for (int i = 0; i < W; i++) m[i] = pub[i];
+            for (int i = 0; i < W; i++) w[i] = pub[i];
 #pragma unroll
-        for (int i = 0; i < 5; i++) m[W + i] = a.w[i];
-        m[W + 5] = (a.w[5] & 0xffff0000u) | (ctr >> 16);
-        m[W + 6] = (ctr << 16) | 0x8000u;
+            for (int i = 0; i < 5; i++) w[W + i] = a.w[i];
+            w[W + 5] = (a.w[5] & 0xffff0000u) | (ctr >> 16);
+            w[W + 6] = (ctr << 16) | 0x8000u;
 #pragma unroll
-        for (int i = W + 7; i < 16 * NB; i++) m[i] = 0;
-        m[16 * NB - 1] = TOT * 8;
-        sha256_iv(out);
-        sha256_compress<kFmaA>(out, m);
-        if (NB == 2) sha256_compress<kFmaA>(out, m + 16);
+            for (int i = W + 7; i < 16; i++) w[i] = 0;
+            if (kMaskUnits == 1) w[15] = TOT * 8;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 15; i++) w[i] = 0;
+            w[15] = TOT * 8;
+        }
     }
-
+    SPX_DEV static void mask_block(uint32_t out[8], const uint32_t pub[W], const Adrs &a, uint32_t ctr) {
+        sha256_iv(out);
+#pragma unroll 1
+        for (int part = 0; part < kMaskUnits; part++) {
+            uint32_t w[16];
+            mask_words(w, pub, a, ctr, part);
+            sha256_compress<kFmaA>(out, w);
+        }
+    }
+    // block words w and start state st of unit u of thash over in (st holds
+    // the unit before's result where the unit continues it), ...
+    template <int L>
+    SPX_DEV static void unit_block(uint32_t w[16], uint32_t st[8], const KeyRegs<N> &k, const Adrs &a,
+                                   const uint32_t in[L], int u) {
+        constexpr int MU = kMaskAll<L>;
+        if (ROBUST && u < MU) {
+            const int part = u % kMaskUnits;
+            if (part == 0) sha256_iv(st);
+            mask_words(w, k.pub, a, (uint32_t)(u / kMaskUnits), part);
+        } else {
+            if (u == MU) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) st[i] = k.mid[i];
+            }
+            core_block<L>(w, a, in, u - MU);
+        }
+    }
+    // ... and what follows its compression: a finished bitmask block goes into in
+    template <int L>
+    SPX_DEV static void unit_done(const uint32_t st[8], uint32_t in[L], int u) {
+        if (ROBUST && u < kMaskAll<L> && u % kMaskUnits == kMaskUnits - 1) {
+#pragma unroll
+            for (int b = 0; b < (L + 7) / 8; b++)
+                if (b == u / kMaskUnits) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (8 * b + i < L) in[8 * b + i] ^= st[i];
+                }
+        }
+    }
     template <int L>
     SPX_DEV static void thash(uint32_t out[W], const KeyRegs<N> &k, const Adrs &a, uint32_t in[L]) {
-        if (ROBUST) {
+        uint32_t st[8];
 #pragma unroll
-            for (int b = 0; b < (L + 7) / 8; b++) {
-                uint32_t mk[8];
-                mask_block(mk, k.pub, a, b);
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                    if (8 * b + i < L) in[8 * b + i] ^= mk[i];
-            }
+        for (int i = 0; i < 8; i++) st[i] = k.mid[i];
+#pragma unroll 1
+        for (int u = 0; u < kUnits<L>; u++) {
+            uint32_t w[16];
+            unit_block<L>(w, st, k, a, in, u);
+            sha256_compress<kFmaA>(st, w);
+            unit_done<L>(st, in, u);
         }
-        core<L>(out, k.mid, a, in);
+#pragma unroll
+        for (int i = 0; i < W; i++) out[i] = st[i];
     }
 
     SPX_DEV static void F(uint32_t out[W], const uint32_t in[W], const Adrs &a, const KeyRegs<N> &k) {
@@ -255,8 +309,7 @@ struct Sha2 {
     }
 
     // PRF = SHA256(SK_SEED || ADRS_c), no midstate (hash_sha256.cu:65-77)
-    SPX_DEV static void PRF(uint32_t out[W], const Adrs &a, const KeyRegs<N> &k) {
-        uint32_t m[16];
+    SPX_DEV static void prf_words(uint32_t m[16], const Adrs &a, const KeyRegs<N> &k) {
 #pragma unroll
         for (int i = 0; i < W; i++) m[i] = k.skseed[i];
 #pragma unroll
@@ -265,11 +318,79 @@ struct Sha2 {
 #pragma unroll
         for (int i = W + 6; i < 16; i++) m[i] = 0;
         m[15] = (N + 22) * 8;
-        uint32_t s[8];
+    }
+    SPX_DEV static void PRF(uint32_t out[W], const Adrs &a, const KeyRegs<N> &k) {
+        uint32_t m[16], s[8];
+        prf_words(m, a, k);
         sha256_iv(s);
         sha256_compress<kFmaA>(s, m);
 #pragma unroll
         for (int i = 0; i < W; i++) out[i] = s[i];
+    }
+
+    // Root v of a FORS subtree of 2^sub leaves from leaf j0 (of the tree at
+    // leaf offset off), by one thread with a stack of sub + 1 values
+    // (treehash, utils.cu:189-241): a leaf's PRF and F and the merges it
+    // completes, every compression of them through one call site (see thash).
+    // sec(j, x) sees each leaf's secret, node(h, i, x) each node i of height h.
+    template <class S, class T>
+    SPX_DEV static void fors_subtree(uint32_t v[W], Adrs &ad, const KeyRegs<N> &k, uint32_t j0, int sub, uint32_t off,
+                                     uint32_t *stk, S sec, T node) {
+        uint32_t jj = 0, x[2 * W], st[8];
+        int hgt = -1, u = 0;   // hgt: height of the node in the making, -1 a leaf's secret
+#pragma unroll
+        for (int i = 0; i < 2 * W; i++) x[i] = 0;
+        adrs_height(ad, 0);
+        adrs_index(ad, off + j0);
+#pragma unroll 1
+        for (;;) {
+            uint32_t w[16];
+            if (hgt < 0) {
+                prf_words(w, ad, k);
+                sha256_iv(st);
+            } else if (hgt == 0) {
+                unit_block<W>(w, st, k, ad, x, u);
+            } else {
+                unit_block<2 * W>(w, st, k, ad, x, u);
+            }
+            sha256_compress<kFmaA>(st, w);
+            if (hgt < 0) {
+#pragma unroll
+                for (int i = 0; i < W; i++) x[i] = st[i];
+                sec(j0 + jj, x);
+                hgt = u = 0;
+                continue;
+            }
+            if (hgt == 0) unit_done<W>(st, x, u);
+            else unit_done<2 * W>(st, x, u);
+            if (++u < (hgt == 0 ? kUnits<W> : kUnits<2 * W>)) continue;
+            u = 0;
+            // st: node (j0 + jj) >> hgt of height hgt
+            node(hgt, (j0 + jj) >> hgt, st);
+            if ((jj >> hgt) & 1u) {   // a right child: merge with the stack's top
+                const uint32_t *top = stk + (__popc(jj >> hgt) - 1) * W;
+#pragma unroll
+                for (int i = 0; i < W; i++) {
+                    x[i] = top[i];
+                    x[W + i] = st[i];
+                }
+                hgt++;
+                adrs_height(ad, hgt);
+                adrs_index(ad, ((j0 + jj) >> hgt) + (off >> hgt));
+                continue;
+            }
+            if (jj + 1 == 1u << sub) break;
+            // a left child waits on the stack, above an entry per set bit
+            uint32_t *top = stk + __popc(jj >> hgt) * W;
+#pragma unroll
+            for (int i = 0; i < W; i++) top[i] = st[i];
+            jj++;
+            hgt = -1;
+            adrs_height(ad, 0);
+            adrs_index(ad, off + j0 + jj);
+        }
+#pragma unroll
+        for (int i = 0; i < W; i++) v[i] = st[i];
     }
 
     // T_l streaming: midstate; ADRS_c || v_0 || v_1 ... Every value lands at a
@@ -370,9 +491,17 @@ struct Sha2 {
             }
             if constexpr (ROBUST) {
                 // mk: mask blocks 2j - 1 (kept from the last block), 2j, 2j + 1
+#pragma unroll 1
+                for (int h = 0; h < 2; h++) {
+                    uint32_t x[8];
+                    mask_block(x, k.pub, a, 2 * j + h);
 #pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (2 * j + h < MB) mask_block(mk + 8 + 8 * h, k.pub, a, 2 * j + h);
+                    for (int i = 0; i < 8; i++) {
+                        if (h == 0) mk[8 + i] = x[i];
+                        else mk[16 + i] = x[i];
+                    }
+                    if (2 * j + 1 >= MB) break;
+                }
 #pragma unroll
                 for (int i = 0; i < 18; i++) {
                     const int x = 16 * j - 6 + i;
@@ -767,6 +896,37 @@ struct Shake {
         short_hash<0, NL>(o, k.skseed, a, dummy);
 #pragma unroll
         for (int i = 0; i < NL; i++) { out[2 * i] = (uint32_t)o[i]; out[2 * i + 1] = (uint32_t)(o[i] >> 32); }
+    }
+
+    // Root of a FORS subtree (see Sha2::fors_subtree)
+    template <class S, class T>
+    SPX_DEV static void fors_subtree(uint32_t v[W], Adrs &ad, const KeyRegs<N> &k, uint32_t j0, int sub, uint32_t off,
+                                     uint32_t *stk, S sec, T node) {
+        int sp = 0;
+        for (uint32_t jj = 0; jj < 1u << sub; jj++) {
+            const uint32_t j = j0 + jj;
+            adrs_height(ad, 0);
+            adrs_index(ad, off + j);
+            uint32_t x[W];
+            PRF(x, ad, k);
+            sec(j, x);
+            F(v, x, ad, k);
+            node(0, j, v);
+            int hgt = 0;
+            while ((jj >> hgt) & 1u) {   // merge equal-height nodes on the stack
+                sp--;
+#pragma unroll
+                for (int q = 0; q < W; q++) x[q] = stk[sp * W + q];
+                hgt++;
+                adrs_height(ad, hgt);
+                adrs_index(ad, (j >> hgt) + (off >> hgt));
+                H(v, x, v, ad, k);
+                node(hgt, j >> hgt, v);
+            }
+#pragma unroll
+            for (int q = 0; q < W; q++) stk[sp * W + q] = v[q];
+            sp++;
+        }
     }
 
     // T_l streaming: PUB_SEED || ADRS || v_0 || v_1 ...  (lanes, rate 17)

@@ -1,6 +1,6 @@
 """Sign batches through each way their work is laid out: chain lanes with the
-streaming T_len (batches above chain_mode_max) in one or more chunks of trees.
-They are byte-identical to the small-batch path, which
+streaming T_len (batches above chain_mode_max) in one or more chunks of trees,
+and FORS trees spread over more lanes than a warp.  All of them are byte-identical to the small-batch path, which
 test_gpu_parity.py pins to the oracle, and to the oracle itself.
 """
 import random
@@ -66,3 +66,17 @@ def test_leaf_chunks(engine, setname, count):
     sigs, st = engine.sign_batch(sid, sks, msgs)
     assert not any(st)
     assert sigs == _in_pieces(engine, sid, sks, msgs, 30)
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-192f-simple", 1), ("sha256-192f-robust", 20),
+                                           ("shake256-256f-simple", 1), ("sha256-128s-robust", 1),
+                                           ("shake256-128s-simple", 2), ("sha256-256s-simple", 30),
+                                           ("sha256-192s-simple", 150), ("sha256-192s-simple", 300)])
+def test_fors_lane_spread(engine, setname, count):
+    """2^8 (a whole tree of 192f), 2^9, 2^10 and down to 2^6 lanes per tree"""
+    sid = engine.set_id(setname)
+    pks, sks, msgs = _requests(engine, sid, count, count, 9)
+    sigs, st = engine.sign_batch(sid, sks, msgs)
+    assert not any(st)
+    assert sigs[count - 1] == _oracle(setname).sign(msgs[count - 1], sks[count - 1])
+    assert not any(engine.verify_batch(sid, pks, msgs, sigs))
