@@ -17,8 +17,9 @@
 //                                        batches; k_leaves: both per leaf, without scratch)
 //   k_trees         warp / XMSS tree     level-by-level reduction in shared memory,
 //                                        auth path, root (k_trees_lane: lane / tree)
-//   k_sign_finish   block / signature    FORS pk (T_k), WOTS signatures gathered
-//                                        from the recorded chains
+//   k_fors_pk       thread / signature   FORS pk (T_k)
+//   k_sign_finish   block / signature    WOTS signatures gathered from the recorded
+//                                        chains
 //
 // Verify: k_verify_msg (+ k_verify_msg_pair / _wide) -> k_verify_fors -> the
 // hypertree: for tiny batches every chain run from all 16 start steps, then a
@@ -551,14 +552,11 @@ __global__ void __launch_bounds__(256, HF::kLeafMinBlocks) k_leaves(SetParams P,
 // the len ends with T_len.
 //
 // k_leaf_chains is bound by the ALU pipe.  A chain's state is its context and
-// value alone (64 registers at 128f against 117 with the T stream of
-// k_leaves), so 8 warps instead of 4 share a scheduler, and a batch is
-// millions of equal threads, so no wave is left part empty: 19.2 G
-// compressions/s at 1024 signatures of 128f, against 17.1 in k_leaves (5.25 +
-// 0.13 ms for T_len, against 5.99); 256s-robust, 100 signatures, 43.8 against
-// 45.9 ms; SHAKE-256f, 1024, 63.4 against 66.2 ms.  The ends cross memory
-// once (99 KB a signature at 128f, 0.4% of the time at HBM rate).  Launched in
-// chunks of whole trees that the ends scratch holds.
+// value alone (71 registers at 128f against 122 with the T stream of
+// k_leaves), so 7 warps instead of 4 share a scheduler, and a batch is
+// millions of equal threads, so no wave is left part empty.  The ends cross
+// memory once (99 KB a signature at 128f, 0.4% of the time at HBM rate).
+// Launched in chunks of whole trees that the ends scratch holds.
 // ===========================================================================
 // the tree (item and layer) and leaf of the launch's leaf x
 SPX_DEV void leaf_pos(const SetParams &P, const LeafArgs &A, uint32_t x, uint32_t &item, int &L, uint32_t &j) {
@@ -675,8 +673,8 @@ __global__ void k_leaf_tlen(SetParams P, LeafArgs A, uint32_t slot_words) {
 
 // thread per leaf, large batches: T_len over the interleaved ends, block by
 // block in registers (HF::t_values).  A warp's 32 leaves read value c as one
-// run of 32 n bytes.  4096 keys at 128f: 0.036 ms, against 0.058 ms through
-// the T stream's shared buffer and a leaf's own 560 bytes.
+// run of 32 n bytes.  4096 keys at 128f: 0.058 ms through the T stream's
+// shared buffer and a leaf's own 560 bytes.
 template <class HF>
 __global__ void __launch_bounds__(128) k_leaf_tstream(SetParams P, LeafArgs A) {
     constexpr int W = HF::W, N = 4 * W, NW = N / 8, LEN = 2 * N + 3;
@@ -847,54 +845,59 @@ __global__ void k_trees(SetParams P, TreeArgs A) {
 }
 
 // ===========================================================================
-// sign finish: block per signature.  Thread 0 computes the FORS public key
-// T_k(roots) (fors.cu:141-142); then all threads gather each layer's WOTS
+// FORS public key: thread per signature, T_k over its FORS roots (fors.cu:
+// 141-142) through a verify slot (slot_tl), in place of the first root.  Runs
+// behind k_fors_sign, beside the hypertree: one signature at 128f spends
+// ~20 us here that k_sign_finish added behind the trees before.
+// ===========================================================================
+template <class HF>
+__global__ void __launch_bounds__(32) k_fors_pk(SetParams P, SignArgs A, uint32_t slot_words) {
+    constexpr int W = HF::W, N = 4 * W;
+    extern __shared__ uint32_t smem[];
+    const uint32_t item = blockIdx.x * blockDim.x + threadIdx.x;
+    if (item >= A.count) return;
+    const SignWork &wk = A.work[item];
+    const uint8_t *sk = A.sk.row(item);
+    KeyRegs<N> key;
+    key_from_work<HF>(key, sk, sk + 2 * N, wk);
+    Adrs pa;
+    adrs_zero(pa);
+    adrs_tree(pa, wk.tree);
+    adrs_keypair(pa, wk.idx_leaf);
+    adrs_type(pa, ADDR_FORSPK);
+    uint32_t o[W];
+    uint8_t *roots = A.fors_roots + (uint64_t)item * P.k * N;
+    slot_tl<HF>(smem + threadIdx.x * slot_words, key, sk + 2 * N, pa, roots, P.k, o);
+    HF::store(roots, o);
+}
+
+// ===========================================================================
+// sign finish: block per signature.  All threads gather each layer's WOTS+
 // signature from the recorded chain values: layer 0 signs the FORS key,
 // layer L signs the root of layer L-1.
 // ===========================================================================
 template <class HF>
 __global__ void k_sign_finish(SetParams P, SignArgs A) {
     constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
-    extern __shared__ uint32_t smem[];
     const uint32_t item = blockIdx.x;
     if (item >= A.count) return;
-    uint32_t *forspk = smem;                   // W words
-    uint32_t *slot = smem + 8;                 // slot_tl scratch
-    const SignWork wk = A.work[item];
-    const uint8_t *sk = A.sk.row(item);
     if (threadIdx.x == 0) {
-        KeyRegs<N> key;
-        key_from_work<HF>(key, sk, sk + 2 * N, wk);
-        Adrs pa;
-        adrs_zero(pa);
-        adrs_tree(pa, wk.tree);
-        adrs_keypair(pa, wk.idx_leaf);
-        adrs_type(pa, ADDR_FORSPK);
-        uint32_t o[W];
-        slot_tl<HF>(slot, key, sk + 2 * N, pa, A.fors_roots + (uint64_t)item * P.k * N, P.k, o);
-#pragma unroll
-        for (int x = 0; x < W; x++) forspk[x] = o[x];
         // the top layer root must equal the key's root; otherwise the key row
         // is inconsistent (sk root does not match its seeds)
         uint32_t top[W], skroot[W];
         HF::load(top, A.roots + ((uint64_t)item * P.d + (P.d - 1)) * N);
-        HF::load(skroot, sk + 3 * N);
+        HF::load(skroot, A.sk.row(item) + 3 * N);
         bool ok = true;
 #pragma unroll
         for (int x = 0; x < W; x++) ok &= top[x] == skroot[x];
         if (A.status) A.status[item] = ok ? 0 : -2;
     }
-    __syncthreads();
     uint8_t *sig = A.sig + (uint64_t)item * P.sig_bytes;
     for (int e = threadIdx.x; e < P.d * LEN; e += blockDim.x) {
         const int L = e / LEN, c = e % LEN;
         uint32_t msg[W];
-        if (L == 0) {
-#pragma unroll
-            for (int x = 0; x < W; x++) msg[x] = forspk[x];
-        } else {
-            HF::load(msg, A.roots + ((uint64_t)item * P.d + (L - 1)) * N);
-        }
+        HF::load(msg, L == 0 ? A.fors_roots + (uint64_t)item * P.k * N
+                             : A.roots + ((uint64_t)item * P.d + (L - 1)) * N);
         const uint32_t ln = chain_len<HF>(P, msg, c);
         const uint8_t *src = A.chains + ((((uint64_t)item * P.d + L) * LEN + c) * 16 + ln) * N;
         uint32_t v[W];

@@ -154,7 +154,7 @@ struct Family {
         if ((e = cudaFuncSetAttribute(k_verify_item<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         if ((e = cudaFuncSetAttribute(k_vsort_layer<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         if ((e = cudaFuncSetAttribute(k_vspec_walk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
-        if ((e = cudaFuncSetAttribute(k_sign_finish<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
+        if ((e = cudaFuncSetAttribute(k_fors_pk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         // Load every other kernel of the family now: with lazy module loading
         // a kernel's first launch loads it, and in a server that first launch
         // is a request's (one took ~50 ms of host time and held back every
@@ -307,6 +307,9 @@ struct Family {
                 k_fors_top<HF><<<(unsigned)trees, tb, (size_t)W * 4 << g, sf>>>(P, A, g);
                 CUSPX_MARK(pt, "k_fors_top", s);
             }
+            const uint32_t sw = VsortSmem<HF>::slot_stride(0);
+            k_fors_pk<HF><<<ceil_div(A.count, 32), 32, (size_t)32 * sw * 4, sf>>>(P, A, sw);
+            CUSPX_MARK(pt, "k_fors_pk", s);
         }
         if (split) cudaEventRecord(fk->join, sf);
         {
@@ -320,7 +323,7 @@ struct Family {
             CUSPX_MARK(pt, "k_trees", s);
         }
         if (split) cudaStreamWaitEvent(s, fk->join, 0);
-        k_sign_finish<HF><<<A.count, 128, (8 + VsortSmem<HF>::slot_stride(0)) * 4, s>>>(P, A);
+        k_sign_finish<HF><<<A.count, 128, 0, s>>>(P, A);
         CUSPX_MARK(pt, "k_sign_finish", s);
     }
 
