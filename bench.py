@@ -334,7 +334,8 @@ def main():
     # the chain kernel runs in chunks of trees: its time is all launches of a step
     leaves = sum(m for name, m, _ in kern if name == "k_leaf_chains") / 3
     P = dict(n=16, d=22, hp=3)
-    leaf_ops = BATCH * P["d"] * (1 << P["hp"]) * chain_units(SET) * OPS_PER_CMP
+    trees = distinct_trees(BATCH, P["d"], P["hp"])   # the batch has one key
+    leaf_ops = trees * (1 << P["hp"]) * chain_units(SET) * OPS_PER_CMP
     achieved = leaf_ops / (leaves * 1e-3) / 1e12
     traffic = None
     tfile = os.path.join(ROOT, "profiles", "k_leaf_chains_sha256-128f_traffic.json")
@@ -371,13 +372,16 @@ def main():
     # ---- what the kernels execute, beside the model ----
     # The model counts the reference's structure at 1384 INT ops per
     # compression.  This engine skips two of its parts (the FORS secret PRF
-    # and wots_sign's chain recomputation: ~6.5k of 113k compressions), and
+    # and wots_sign's chain recomputation: ~6.5k of 113k compressions),
+    # computes a tree that several signatures of the batch go through once
+    # (one key: ~17.7 of 22 layers a signature), and
     # the compiler issues fewer ALU instructions per compression than the
     # model's ops (ncu: ALU instructions of a k_leaf_chains launch / its
     # compressions, profiles/k_leaf_chains_sha256-128f_pipe.json).
     m128 = unit_model(SET)
-    executed = {"sign_compressions": m128["executed_sign"] + MSG_CMP_64B_SIGN,
-                "step_frac_of_mix_peak": value * (m128["executed_sign"] + MSG_CMP_64B_SIGN) * OPS_PER_CMP / peak_ops}
+    ex_cmp = m128["executed_sign"] + MSG_CMP_64B_SIGN - \
+        (P["d"] - trees / BATCH) * (1 << P["hp"]) * leaf_units(SET)
+    executed = {"sign_compressions": ex_cmp, "step_frac_of_mix_peak": value * ex_cmp * OPS_PER_CMP / peak_ops}
     pfile = os.path.join(ROOT, "profiles", "k_leaf_chains_sha256-128f_pipe.json")
     if os.path.exists(pfile):
         with open(pfile) as f:
@@ -495,7 +499,7 @@ def main():
                          "peak": peak_ops / 1e12, "unit": "Tops/s", "frac": achieved / (peak_ops / 1e12),
                          "traffic": traffic,
                          "work": "%d compressions x %d INT ops per step" %
-                                 (BATCH * 176 * chain_units(SET), OPS_PER_CMP),
+                                 (leaf_ops / OPS_PER_CMP, OPS_PER_CMP),
                          "peak_source": "measured in this run on all SMs: SHA-256 round mix, 7 ALU ops "
                                         "(SHF/LOP3/IADD3) to 1 IMAD on the FMA pipe (cuspx_int_peak_mix 1)",
                          "peak_alu_only": peak_alu / 1e12,
@@ -758,6 +762,18 @@ def leaf_units(name):
     return ln * 16 + t
 
 
+def distinct_trees(count, d, hp):
+    """Expected number of different hypertree trees that `count` random
+    signatures of one key go through (a tree that several need is computed
+    once)."""
+    import math
+    out = 0.0
+    for layer in range(d):
+        there = 2.0 ** (hp * (d - 1 - layer))
+        out += there * -math.expm1(count * math.log1p(-1.0 / there)) if there > 1 else 1.0
+    return out
+
+
 def chain_units(name):
     """Hash units of the WOTS+ chains of one XMSS leaf (leaf_units without T_len)."""
     n = {"128": 16, "192": 24, "256": 32}[name.split("-")[1][:3]]
@@ -803,7 +819,7 @@ def sign_sets(c, eng, peak_alu, peak_mix, count=1024, mlen=256):
         sb.profile(False)
         sb.close()
         h, d = hypertree[name.split("-")[1]]
-        units = count * d * (1 << (h // d)) * chain_units(name)
+        units = distinct_trees(count, d, h // d) * (1 << (h // d)) * chain_units(name)
         shake = name.startswith("shake")
         ops = units * (4560 if shake else OPS_PER_CMP)
         leaves = km.get("k_leaf_chains")

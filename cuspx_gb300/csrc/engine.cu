@@ -169,6 +169,7 @@ struct cuspx_batch {
     uint32_t ends_trees = 0;
     uint8_t *fors_nodes = nullptr;
     uint64_t fors_lanes = 0;
+    ShareArgs share;
     size_t count = 0;
     bool use_keyrow = false, use_aux = false, use_siglen = false;
     const uint8_t *bound_keys = nullptr;   // external device key table (not owned)
@@ -699,6 +700,17 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
             A((void **)&b->roots, cap * P.d * n);
             A((void **)&b->chains, cap * P.d * P.len * 16 * n);
             ends(cap * P.d);
+            // trees that items have in common (ShareArgs), for the deepest
+            // layer that a full batch looks at
+            const size_t sh = P.d - shared_layer0(P, cap);
+            const size_t tab = (sh + 1) * (size_t)share_table(cap);
+            A((void **)&b->share.cnt, (4 + tab + (sh + 1) * cap + sh * cap + (sh * cap << P.hp)) * sizeof(uint32_t));
+            if (b->share.cnt) {
+                b->share.tab = b->share.cnt + 4;
+                b->share.rep = b->share.tab + tab;
+                b->share.list = b->share.rep + (sh + 1) * cap;
+                b->share.recs = b->share.list + sh * cap;
+            }
             // FORS subtree roots of trees spread over more than a warp
             // (fors_lanes stops below twice 2048 lanes an SM)
             b->fors_lanes = std::min<uint64_t>((uint64_t)cap * P.k << std::min(P.a, kForsMaxLanes),
@@ -837,6 +849,7 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.ends_trees = b->ends_trees;
         A.fors_nodes = b->fors_nodes;
         A.fors_lanes = b->fors_lanes;
+        A.share = b->share;
         ops.sign(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0,
                  (CUSPX_SIGN_FORK && b->fork.side) ? &b->fork : nullptr);
     } else if (b->op == CUSPX_OP_VERIFY) {

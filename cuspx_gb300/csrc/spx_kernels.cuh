@@ -9,6 +9,7 @@
 //   k_sign_msg_wide warp / signature     the same for messages of >= 2 KiB (SHAKE)
 //   k_sign_msg_pair 2 warps / 32 sigs    the same for messages of >= 2 KiB (SHA-256):
 //                                        schedule warp + rounds warp per message
+//   k_share         thread / (item, upper layer)  trees that items of one key share
 //   k_fors_sign     2^g lanes / FORS tree leaves (PRF+F), per-lane subtree stack,
 //                                        g shuffle levels, auth path, root
 //   k_fors_top      block / FORS tree    the levels above 2^g > 32 lanes
@@ -85,6 +86,31 @@ struct MsgRef {
     const uint64_t *len;       // per-item length
 };
 
+// Hypertree trees that several items of a sign batch have in common.  Items
+// of one key meet in the same subtrees towards the top (layer d-1 is one tree
+// for all of them, layer d-2 2^h' trees, ...), and a shared tree's leaves and
+// WOTS+ signatures are the same bytes for each.  For the layers layer0 .. d-1
+// k_share finds for every item a representative among those in the same tree
+// under the same key; only representatives' trees are computed.  Layer
+// layer0 - 1 has a table too: its trees are the leaves of layer layer0.
+// 4096 signatures of 128f under one key run 17.7 of 22 layers' trees each:
+// 23.8 -> 19.8 ms; 1024 of SHAKE-256f 14 of 17, 75.6 -> 64.9 ms.  With a key
+// each nothing is shared and the search costs 0.7% (1024 of 128f, 5.91 ->
+// 5.95 ms).
+struct ShareArgs {
+    int layer0 = 0;             // first shared layer (>= 1); 0: nothing is shared
+    uint32_t mask = 0;          // table size - 1 (a power of two >= 2 x count)
+    uint32_t *cnt = nullptr;    // entries of list; zeroed, like tab, before k_share
+    uint32_t *tab = nullptr;    // [layer - layer0 + 1][mask + 1] item + 1, open addressing; 0 empty
+    uint32_t *rep = nullptr;    // [layer - layer0 + 1][count] representative item
+    uint32_t *list = nullptr;   // item * d + layer of the representatives' trees, layers >= layer0
+    uint32_t *recs = nullptr;   // [layer - layer0][representative][leaf] item + 1 whose chain record
+                                // the leaf fills, 0: no item signs with it; zeroed
+    SPX_DEV uint32_t of(int L, uint32_t item, uint32_t count) const {
+        return layer0 && L + 1 >= layer0 ? rep[(uint64_t)(L + 1 - layer0) * count + item] : item;
+    }
+};
+
 struct SignArgs {
     uint32_t count;
     KeyRef sk;
@@ -101,6 +127,7 @@ struct SignArgs {
     uint32_t ends_trees = 0;
     uint8_t *fors_nodes = nullptr;   // FORS subtree roots: fors_lanes x n, or null
     uint64_t fors_lanes = 0;
+    ShareArgs share;
 };
 
 // tree/leaf indices of hypertree layer L (sign.cu:1987-1988)
@@ -115,6 +142,39 @@ SPX_DEV void layer_index(const SetParams &P, uint64_t tree, uint32_t idx_leaf, i
         idx_L = (uint32_t)(t & mask);
         tree_L = P.hp >= 64 ? 0 : (t >> P.hp);
     }
+}
+
+// whether items i and r sign under the same key (the seeds decide every tree)
+template <int N>
+SPX_DEV bool same_key(const KeyRef &sk, uint32_t i, uint32_t r) {
+    const uint64_t *x = reinterpret_cast<const uint64_t *>(sk.row(i));
+    const uint64_t *y = reinterpret_cast<const uint64_t *>(sk.row(r));
+    bool eq = true;
+    if (x != y) {
+#pragma unroll
+        for (int j = 0; j < N / 8; j++) eq &= x[j] == y[j] && x[2 * N / 8 + j] == y[2 * N / 8 + j];
+    }
+    return eq;
+}
+// The item that item i's tree of `layer` is kept under: the first to come into
+// the layer's table with that tree and key.  The table is at most half full,
+// so a probe ends.
+template <int N>
+SPX_DEV uint32_t share_insert(const SetParams &P, const ShareArgs &S, const KeyRef &sk, const SignWork *work,
+                              int layer, uint64_t tree, uint32_t i) {
+    uint32_t *tab = S.tab + (uint64_t)(layer + 1 - S.layer0) * (S.mask + 1);
+    const uint32_t k = *reinterpret_cast<const uint32_t *>(sk.row(i));
+    uint32_t h = ((uint32_t)tree ^ (uint32_t)(tree >> 32) * 0x85ebca6bu ^ k) * 0x9e3779b1u;
+    h ^= h >> 15;
+    for (uint32_t n = 0; n <= S.mask; n++, h++) {
+        const uint32_t e = atomicCAS(tab + (h & S.mask), 0u, i + 1);
+        if (e == 0) break;
+        uint64_t t;
+        uint32_t idx;
+        layer_index(P, work[e - 1].tree, work[e - 1].idx_leaf, layer, t, idx);
+        if (t == tree && same_key<N>(sk, i, e - 1)) return e - 1;
+    }
+    return i;
 }
 
 // LSB-first FORS index of tree t (message_to_indices, fors.cu:77-88)
@@ -324,6 +384,36 @@ __global__ void __launch_bounds__(128) k_sign_msg_wide(SetParams P, SignArgs A, 
     if (lane == 0) A.work[i] = work_from_digest<HF>(P, reinterpret_cast<const uint8_t *>(dgs[wib]), sk + 2 * N);
 }
 
+// thread per (item, layer >= share.layer0 - 1), after the message phase
+template <class HF>
+__global__ void k_share(SetParams P, SignArgs A) {
+    const ShareArgs &S = A.share;
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t q = x / A.count, item = x - q * A.count;
+    const int L = S.layer0 - 1 + (int)q;
+    if (L >= P.d) return;
+    uint64_t tree_L;
+    uint32_t idx_L;
+    layer_index(P, A.work[item].tree, A.work[item].idx_leaf, L, tree_L, idx_L);
+    const uint32_t r = share_insert<4 * HF::W>(P, S, A.sk, A.work, L, tree_L, item);
+    S.rep[(uint64_t)q * A.count + item] = r;
+    if (q > 0 && r == item) S.list[atomicAdd(S.cnt, 1u)] = item * (uint32_t)P.d + (uint32_t)L;
+}
+// thread per (item, layer >= share.layer0), after k_share: who signs with
+// which leaf of the shared trees
+template <class HF>
+__global__ void k_share_leaves(SetParams P, SignArgs A) {
+    const ShareArgs &S = A.share;
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t q = x / A.count, item = x - q * A.count;
+    const int L = S.layer0 + (int)q;
+    if (L >= P.d || S.of(L - 1, item, A.count) != item) return;
+    uint64_t tree_L;
+    uint32_t idx_L;
+    layer_index(P, A.work[item].tree, A.work[item].idx_leaf, L, tree_L, idx_L);
+    S.recs[(((uint64_t)q * A.count + S.of(L, item, A.count)) << P.hp) + idx_L] = item + 1;
+}
+
 // ===========================================================================
 // FORS sign: G = 2^g lanes per (signature, tree), g in 0..min(a, 10).  Lane l
 // owns the contiguous subtree of 2^(a-g) leaves starting at l*2^(a-g) and
@@ -488,6 +578,9 @@ struct LeafArgs {
     uint8_t *ends;       // the launch's chain ends (chain_end), n bytes each
     uint32_t tree0, trees;
     bool interleaved;
+    // signing: of a batch's trees the first count * (share.layer0 - layer0)
+    // are the items' own, layer by layer as above, and the rest share.list's
+    ShareArgs share;
 };
 
 template <class HF>
@@ -552,18 +645,44 @@ __global__ void __launch_bounds__(256, HF::kLeafMinBlocks) k_leaves(SetParams P,
 // the len ends with T_len.
 //
 // k_leaf_chains is bound by the ALU pipe.  A chain's state is its context and
-// value alone (71 registers at 128f against 122 with the T stream of
-// k_leaves), so 7 warps instead of 4 share a scheduler, and a batch is
-// millions of equal threads, so no wave is left part empty.  The ends cross
-// memory once (99 KB a signature at 128f, 0.4% of the time at HBM rate).
-// Launched in chunks of whole trees that the ends scratch holds.
+// value alone (64 registers at 128f against 117 with the T stream of
+// k_leaves), so 8 warps instead of 4 share a scheduler, and a batch is
+// millions of equal threads, so no wave is left part empty: 19.2 G
+// compressions/s at 1024 signatures of 128f, against 17.1 in k_leaves (5.25 +
+// 0.13 ms for T_len, against 5.99); 256s-robust, 100 signatures, 43.8 against
+// 45.9 ms; SHAKE-256f, 1024, 63.4 against 66.2 ms.  The ends cross memory
+// once (99 KB a signature at 128f, 0.4% of the time at HBM rate).  Launched in
+// chunks of whole trees that the ends scratch holds.
 // ===========================================================================
-// the tree (item and layer) and leaf of the launch's leaf x
-SPX_DEV void leaf_pos(const SetParams &P, const LeafArgs &A, uint32_t x, uint32_t &item, int &L, uint32_t &j) {
-    const uint32_t t = A.tree0 + (x >> P.hp);
+// the tree (item and layer) and leaf of the launch's leaf x, if there is one
+SPX_DEV bool leaf_pos(const SetParams &P, const LeafArgs &A, uint32_t x, uint32_t &item, int &L, uint32_t &j) {
+    if (x >> P.hp >= A.trees) return false;
+    uint32_t t = A.tree0 + (x >> P.hp);
     j = x & ((1u << P.hp) - 1u);
+    if (A.share.layer0) {
+        const uint32_t per = (uint32_t)A.share.layer0, own = A.count * per;
+        if (t >= own) {
+            if (t - own >= *A.share.cnt) return false;
+            t = A.share.list[t - own];
+            item = t / (uint32_t)P.d;
+            L = (int)(t - item * (uint32_t)P.d);
+        } else {
+            item = t / per;
+            L = (int)(t - item * per);
+        }
+        return true;
+    }
     item = t / (uint32_t)A.nlayers;
     L = A.layer0 + (int)(t - item * (uint32_t)A.nlayers);
+    return true;
+}
+
+// the item whose chain record leaf j of layer L's tree fills, or -1 if no
+// item signs with that leaf
+SPX_DEV int leaf_record(const SetParams &P, const LeafArgs &A, uint32_t item, int L, uint32_t idx_L, uint32_t j) {
+    if (!A.chains) return -1;
+    if (!A.share.layer0 || L < A.share.layer0) return j == idx_L ? (int)item : -1;
+    return (int)A.share.recs[(((uint64_t)(L - A.share.layer0) * A.count + item) << P.hp) + j] - 1;
 }
 
 // where chain c's end of the launch's leaf x goes: the chains of a leaf in
@@ -582,10 +701,9 @@ __global__ void __launch_bounds__(128) k_leaf_chains(SetParams P, LeafArgs A) {
     constexpr uint32_t LEN = 2 * N + 3;
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t x = gid / LEN, c = gid - x * LEN;
-    if (x >> P.hp >= A.trees) return;
     uint32_t item, j;
     int L;
-    leaf_pos(P, A, x, item, L, j);
+    if (!leaf_pos(P, A, x, item, L, j)) return;
     const uint8_t *sk = A.sk.row(item);
     KeyRegs<N> key;
     uint64_t tree_L = 0;
@@ -597,8 +715,9 @@ __global__ void __launch_bounds__(128) k_leaf_chains(SetParams P, LeafArgs A) {
     } else {
         HF::key_init(key, sk, sk + 2 * N);
     }
-    const bool rec = A.chains && (j == idx_L);
-    uint8_t *chain = rec ? A.chains + ((((uint64_t)item * P.d + L) * LEN + c) * 16) * N : nullptr;
+    const int to = leaf_record(P, A, item, L, idx_L, j);
+    const bool rec = to >= 0;
+    uint8_t *chain = rec ? A.chains + ((((uint64_t)to * P.d + L) * LEN + c) * 16) * N : nullptr;
     Adrs wa;
     adrs_zero(wa);
     adrs_layer(wa, L);
@@ -628,13 +747,14 @@ SPX_DEV void slot_tl(uint32_t *S, const KeyRegs<4 * HF::W> &key, const uint8_t *
                      const uint8_t *vals, int m, uint32_t out[HF::W]);
 
 // key, address and output of a T_len thread: the launch's leaf x
+// (null: there is none)
 template <class HF>
 SPX_DEV const uint8_t *tlen_pos(const SetParams &P, const LeafArgs &A, uint32_t x, KeyRegs<4 * HF::W> &key, Adrs &pa,
                                 uint8_t *&leaf) {
     constexpr int N = 4 * HF::W;
     uint32_t item, j;
     int L;
-    leaf_pos(P, A, x, item, L, j);
+    if (!leaf_pos(P, A, x, item, L, j)) return nullptr;
     const uint8_t *sk = A.sk.row(item);
     uint64_t tree_L = 0;
     uint32_t idx_L = 0;
@@ -661,11 +781,11 @@ __global__ void k_leaf_tlen(SetParams P, LeafArgs A, uint32_t slot_words) {
     constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
     extern __shared__ uint32_t smem[];
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >> P.hp >= A.trees) return;
     KeyRegs<N> key;
     Adrs pa;
     uint8_t *to;
     const uint8_t *sk = tlen_pos<HF>(P, A, x, key, pa, to);
+    if (!sk) return;
     uint32_t leaf[W];
     slot_tl<HF>(smem + threadIdx.x * slot_words, key, sk + 2 * N, pa, chain_end<N>(A, x, 0), LEN, leaf);
     HF::store(to, leaf);
@@ -673,17 +793,16 @@ __global__ void k_leaf_tlen(SetParams P, LeafArgs A, uint32_t slot_words) {
 
 // thread per leaf, large batches: T_len over the interleaved ends, block by
 // block in registers (HF::t_values).  A warp's 32 leaves read value c as one
-// run of 32 n bytes.  4096 keys at 128f: 0.058 ms through the T stream's
-// shared buffer and a leaf's own 560 bytes.
+// run of 32 n bytes.  4096 keys at 128f: 0.036 ms, against 0.058 ms through
+// the T stream's shared buffer and a leaf's own 560 bytes.
 template <class HF>
 __global__ void __launch_bounds__(128) k_leaf_tstream(SetParams P, LeafArgs A) {
     constexpr int W = HF::W, N = 4 * W, NW = N / 8, LEN = 2 * N + 3;
     const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >> P.hp >= A.trees) return;
     KeyRegs<N> key;
     Adrs pa;
     uint8_t *to;
-    tlen_pos<HF>(P, A, x, key, pa, to);
+    if (!tlen_pos<HF>(P, A, x, key, pa, to)) return;
     const uint2 *e = reinterpret_cast<const uint2 *>(chain_end<N>(A, x, 0));
     uint32_t leaf[W];
     HF::template t_values<LEN>(leaf, key, pa, [&](uint32_t q) { return e[(q / NW) * (32 * NW) + q % NW]; });
@@ -704,7 +823,17 @@ struct TreeArgs {
     const uint8_t *leaves;
     uint8_t *roots;         // [item][layer-layer0] n bytes
     uint8_t *sig;           // auth paths are written here when work != null
+    ShareArgs share;
 };
+
+// leaves of an item's tree at layer L: its own or its representative's (the
+// reduction itself, 2^h' - 1 of a tree's hashes, is repeated for each item,
+// whose auth path it writes)
+template <int N>
+SPX_DEV const uint8_t *tree_leaves(const SetParams &P, const TreeArgs &A, uint32_t item, int L) {
+    const uint32_t r = A.share.layer0 && L >= A.share.layer0 ? A.share.of(L, item, A.count) : item;
+    return A.leaves + ((((uint64_t)r * A.nlayers + (L - A.layer0)) << P.hp)) * N;
+}
 
 // Lane-per-tree variant for short subtrees: a thread reduces one whole
 // (item, layer) tree with a stack of hp+1 nodes; no shared memory, no idle
@@ -728,7 +857,7 @@ __global__ void k_trees_lane(SetParams P, TreeArgs A) {
     } else {
         HF::key_init(key, sk, sk + 2 * N);
     }
-    const uint8_t *lv = A.leaves + (((uint64_t)item * A.nlayers + (L - A.layer0)) * nleaf) * N;
+    const uint8_t *lv = tree_leaves<N>(P, A, item, L);
     uint8_t *auth = nullptr;
     if (A.work)
         auth = A.sig + (uint64_t)item * P.sig_bytes + N + P.fors_bytes +
@@ -792,7 +921,7 @@ __global__ void k_trees(SetParams P, TreeArgs A) {
     } else {
         HF::key_init(key, sk, sk + 2 * N);
     }
-    const uint8_t *lv = A.leaves + (((uint64_t)item * A.nlayers + (L - A.layer0)) * nleaf) * N;
+    const uint8_t *lv = tree_leaves<N>(P, A, item, L);
     for (uint32_t q = lane; q < nleaf; q += 32) {
         uint32_t v[W];
         HF::load(v, lv + (uint64_t)q * N);
@@ -899,7 +1028,10 @@ __global__ void k_sign_finish(SetParams P, SignArgs A) {
         HF::load(msg, L == 0 ? A.fors_roots + (uint64_t)item * P.k * N
                              : A.roots + ((uint64_t)item * P.d + (L - 1)) * N);
         const uint32_t ln = chain_len<HF>(P, msg, c);
-        const uint8_t *src = A.chains + ((((uint64_t)item * P.d + L) * LEN + c) * 16 + ln) * N;
+        // layer L's WOTS+ signature is that of its tree's leaf, shared with the
+        // items in the same tree of layer L - 1
+        const uint32_t r = A.share.layer0 && L >= A.share.layer0 ? A.share.of(L - 1, item, A.count) : item;
+        const uint8_t *src = A.chains + ((((uint64_t)r * P.d + L) * LEN + c) * 16 + ln) * N;
         uint32_t v[W];
         load_bytes_le<N>(v, src);
         store_bytes_le<N>(sig + N + P.fors_bytes + (uint64_t)L * (P.wots_bytes + P.hp * N) + (uint64_t)c * N, v);

@@ -89,7 +89,7 @@ struct FamilyOps {
     // long_msg: messages of at least this many bytes are hashed two warps per
     // 32 messages (SHA-256 sets; 0 or a SHAKE set: one thread each).
     // fk: optional side stream (ignored while per-kernel timing is on).
-    void (*sign)(const SetParams &, const SignArgs &, const Tuning &, cudaStream_t, PhaseTimer *, uint64_t long_msg,
+    void (*sign)(const SetParams &, SignArgs, const Tuning &, cudaStream_t, PhaseTimer *, uint64_t long_msg,
                  const StreamFork *fk);
     // vl / vf: bucket lists and streams of verify_mode 3 (null: that mode
     // runs as verify_mode 2)
@@ -101,6 +101,19 @@ struct FamilyOps {
 
 // registry: [hash][n index 0..2][robust]
 extern FamilyOps g_family[2][3][2];
+
+// Shared trees of a sign batch (ShareArgs): the first layer with at most 8
+// trees per item, and the entries of one layer's table.
+inline int shared_layer0(const SetParams &P, uint64_t count) {
+    int L = P.d - 1;
+    while (L > 1 && (P.d - L) * P.hp < 40 && (1ull << ((P.d - L) * P.hp)) <= 8 * count) L--;
+    return L;
+}
+inline uint32_t share_table(uint64_t count) {
+    uint32_t n = 64;
+    while (n < 2 * count) n *= 2;
+    return n;
+}
 
 inline unsigned ceil_div(uint64_t a, uint64_t b) { return (unsigned)((a + b - 1) / b); }
 
@@ -161,7 +174,7 @@ struct Family {
         // queued request of its class).
         cudaFuncAttributes fa;
         const void *rest[] = {(const void *)k_sign_msg<HF>, (const void *)k_leaf_chains<HF>, (const void *)k_leaf_tstream<HF>,
-                              (const void *)k_trees_lane<HF>, (const void *)k_fors_top<HF>,
+                              (const void *)k_trees_lane<HF>, (const void *)k_fors_top<HF>, (const void *)k_share<HF>, (const void *)k_share_leaves<HF>,
                               (const void *)k_verify_msg<HF>, (const void *)k_verify_fors<HF>,
                               (const void *)k_verify_chains<HF>, (const void *)k_vsort_chains<HF>,
                               (const void *)k_vspec_cand<HF>,
@@ -276,7 +289,16 @@ struct Family {
         return g;
     }
 
-    static void sign(const SetParams &P, const SignArgs &A, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
+    // First layer whose trees are looked for among the items (0: none).  A
+    // layer of 8 trees per item still saves about 6% of its work if all items
+    // have one key; k_share and the two memsets take ~10 us (1 us a thousand
+    // items), so batches of the latency mapping go without.
+    static int share_layer(const SetParams &P, uint32_t count, const Tuning &tu, const ShareArgs &S) {
+        if (!S.tab || count <= 64 || count <= (uint32_t)tu.chain_mode_max) return 0;
+        return shared_layer0(P, count);
+    }
+
+    static void sign(const SetParams &P, SignArgs A, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
                      uint64_t long_msg, const StreamFork *fk) {
         if (A.count == 0) return;
         k_sign_msg<HF><<<ceil_div(A.count, 128), 128, 0, s>>>(P, A, long_msg);
@@ -289,6 +311,18 @@ struct Family {
                 k_sign_msg_wide<HF><<<ceil_div(A.count, 4), 128, 0, s>>>(P, A, long_msg);
                 CUSPX_MARK(pt, "k_sign_msg_wide", s);
             }
+        }
+        // (k_leaves, without chain-end scratch, computes every item's trees)
+        A.share.layer0 = A.ends_trees && tu.chain_mode_max > 0 ? share_layer(P, A.count, tu, A.share) : 0;
+        if (A.share.layer0) {
+            const int tabs = P.d - A.share.layer0 + 1;
+            A.share.mask = share_table(A.count) - 1;
+            cudaMemsetAsync(A.share.cnt, 0, 16, s);
+            cudaMemsetAsync(A.share.tab, 0, (size_t)tabs * (A.share.mask + 1) * 4, s);
+            cudaMemsetAsync(A.share.recs, 0, ((size_t)(tabs - 1) * A.count << P.hp) * 4, s);
+            k_share<HF><<<ceil_div((uint64_t)tabs * A.count, 128), 128, 0, s>>>(P, A);
+            k_share_leaves<HF><<<ceil_div((uint64_t)(tabs - 1) * A.count, 128), 128, 0, s>>>(P, A);
+            CUSPX_MARK(pt, "k_share", s);
         }
         const bool split = fk && !pt;
         cudaStream_t sf = split ? fk->side : s;
@@ -313,12 +347,12 @@ struct Family {
         }
         if (split) cudaEventRecord(fk->join, sf);
         {
-            LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false};
+            LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false, A.share};
             leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? A.ends_trees : 0,
                    A.count <= (uint32_t)tu.chain_mode_max && A.count <= 256);
         }
         {
-            TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig};
+            TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig, A.share};
             trees(P, T, tu, s);
             CUSPX_MARK(pt, "k_trees", s);
         }
@@ -468,9 +502,9 @@ struct Family {
     static void keygen(const SetParams &P, const KeygenArgs &K, const Tuning &tu, cudaStream_t s, PhaseTimer *pt) {
         if (K.count == 0) return;
         KeyRef kr{K.sk, nullptr, (uint32_t)(4 * N)};
-        LeafArgs L{K.count, P.d - 1, 1, kr, nullptr, K.leaves, nullptr, K.ends, 0, 0, false};
+        LeafArgs L{K.count, P.d - 1, 1, kr, nullptr, K.leaves, nullptr, K.ends, 0, 0, false, {}};
         leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? K.ends_trees : 0, false);
-        TreeArgs T{K.count, P.d - 1, 1, kr, nullptr, K.leaves, K.roots, nullptr};
+        TreeArgs T{K.count, P.d - 1, 1, kr, nullptr, K.leaves, K.roots, nullptr, {}};
         trees(P, T, tu, s);
         CUSPX_MARK(pt, "k_trees", s);
         k_keygen_finish<N><<<ceil_div(K.count, 128), 128, 0, s>>>(K);

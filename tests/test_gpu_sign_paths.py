@@ -1,6 +1,7 @@
 """Sign batches through each way their work is laid out: chain lanes with the
 streaming T_len (batches above chain_mode_max) in one or more chunks of trees,
-and FORS trees spread over more lanes than a warp.  All of them are byte-identical to the small-batch path, which
+trees that items share computed once, and FORS trees spread over more lanes
+than a warp.  All of them are byte-identical to the small-batch path, which
 test_gpu_parity.py pins to the oracle, and to the oracle itself.
 """
 import random
@@ -66,6 +67,51 @@ def test_leaf_chunks(engine, setname, count):
     sigs, st = engine.sign_batch(sid, sks, msgs)
     assert not any(st)
     assert sigs == _in_pieces(engine, sid, sks, msgs, 30)
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-128f-simple", 65), ("sha256-128f-simple", 1000),
+                                           ("sha256-192f-robust", 130), ("shake256-256f-simple", 130),
+                                           ("sha256-128s-simple", 100)])
+@pytest.mark.parametrize("keys", [1, 3, 0])
+def test_shared_trees(engine, setname, count, keys):
+    """one key, a few, and a key per item; some messages twice, so that items
+    share even their lowest leaf"""
+    sid = engine.set_id(setname)
+    pks, sks, msgs = _requests(engine, sid, count, keys or count, 7)
+    for i in range(5):
+        sks[count - 1 - i], pks[count - 1 - i], msgs[count - 1 - i] = sks[i], pks[i], msgs[i]
+    sigs, st = engine.sign_batch(sid, sks, msgs)
+    assert not any(st)
+    assert sigs == _in_pieces(engine, sid, sks, msgs)
+    assert sigs[count // 2] == _oracle(setname).sign(msgs[count // 2], sks[count // 2])
+    assert not any(engine.verify_batch(sid, pks, msgs, sigs))
+
+
+def test_shared_trees_by_key_index_and_wrong_root(engine):
+    """rows of a key table picked by index; a row whose ROOT is not its own is
+    reported for its items alone, whose seeds they share with a good row"""
+    import numpy as np
+    import cuspx_gb300 as c
+    sid = engine.set_id("sha256-128f-simple")
+    z = c.set_sizes(sid)
+    pks, sks, msgs = _requests(engine, sid, 200, 1, 8)
+    bad = bytearray(sks[0])
+    bad[-1] ^= 1
+    table = np.frombuffer(sks[0] + bytes(bad), np.uint8)
+    idx = np.array([i % 7 == 3 for i in range(200)], np.uint32)
+    slab, offs, lens = c.pack_messages(msgs)
+    b = engine.batch(c.OP_SIGN, sid, 200, len(slab), 2)
+    out, st = np.zeros(200 * z["sig"], np.uint8), np.zeros(200, np.int32)
+    for _ in range(3):   # direct launch, capture, replay
+        b.upload(200, table, 2, idx, slab, len(slab), offs, lens)
+        b.run()
+        b.download(out, None, st)
+        assert list(st) == [-2 if x else 0 for x in idx]
+        want = _in_pieces(engine, sid, [sks[0]] * 60, msgs[:60])
+        for i in range(60):
+            if not idx[i]:
+                assert out[i * z["sig"]:(i + 1) * z["sig"]].tobytes() == want[i]
+    b.close()
 
 
 @pytest.mark.parametrize("setname,count", [("sha256-192f-simple", 1), ("sha256-192f-robust", 20),
