@@ -177,6 +177,52 @@ SPX_DEV void sha256_rounds(uint32_t st[8], uint32_t w[16]) {
     st[0] = a; st[1] = b; st[2] = c; st[3] = d; st[4] = e; st[5] = f; st[6] = g; st[7] = h;
 }
 
+// K_t + W_t of a block of 15 zero words and the last word `len`: the block
+// behind a message whose length field alone does not fit its last block.
+struct Sha256PadKw {
+    uint32_t v[64];
+};
+__host__ __device__ constexpr Sha256PadKw sha256_pad_kw(uint32_t len) {
+    Sha256PadKw kw{};
+    uint32_t w[64] = {};
+    w[15] = len;
+    for (int t = 0; t < 64; t++) {
+        if (t >= 16) {
+            const uint32_t x = w[t - 15], y = w[t - 2];
+            w[t] = w[t - 16] + ((x >> 7 | x << 25) ^ (x >> 18 | x << 14) ^ x >> 3) + w[t - 7] +
+                   ((y >> 17 | y << 15) ^ (y >> 19 | y << 13) ^ y >> 10);
+        }
+        kw.v[t] = w[t] + sha256_k(t);
+    }
+    return kw;
+}
+// The 64 rounds over such a block, sixteen at a time: they need no schedule,
+// and 4 KB of code instead of 15 KB leaves a loop that runs them beside other
+// compressions within the instruction cache.
+template <bool AF>
+SPX_DEV void sha256_rounds_pad(uint32_t st[8], const Sha256PadKw &kw) {
+#pragma unroll 1
+    for (int r = 0; r < 64; r += 16) {
+        uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6], h = st[7];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
+            const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
+            const uint32_t t1 = h + kw.v[r + i] + S1 + ch;
+            const uint32_t na = AF ? add_fma(add_fma(S0, mj), t1) : t1 + (S0 + mj);
+            h = g;
+            g = f;
+            f = e;
+            e = add_fma(d, t1);
+            d = c;
+            c = b;
+            b = a;
+            a = na;
+        }
+        st[0] = a; st[1] = b; st[2] = c; st[3] = d; st[4] = e; st[5] = f; st[6] = g; st[7] = h;
+    }
+}
+
 // Message schedule with the round constants added: kw[t * S] = W_t + K_t
 // for t = 0..63 from the 16 block words w (consumed); S interleaves the
 // buffers of several threads in shared memory.

@@ -68,6 +68,9 @@ SPX_DEV void store_bytes_le(uint8_t *p, const uint32_t v[N / 4]) {
 // ===========================================================================
 // SHA-256 family
 // ===========================================================================
+// second block of a robust n = 32 bitmask (PUB_SEED || ADRS_c || ctr, 58 bytes)
+static __constant__ Sha256PadKw c_mask_pad = sha256_pad_kw(58 * 8);
+
 template <int N, bool ROBUST>
 struct Sha2 {
     static constexpr int W = N / 4;
@@ -285,7 +288,13 @@ struct Sha2 {
             sha256_rounds<W + 5, 64, kFmaA>(t, mw);
 #pragma unroll
             for (int i = 0; i < 8; i++) ms[i] = t[i] + sha256_iv_word(i);
-            if (NB == 2) sha256_compress<kFmaA>(ms, mw + 16);
+            if (NB == 2) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) t[i] = ms[i];
+                sha256_rounds_pad<kFmaA>(t, c_mask_pad);
+#pragma unroll
+                for (int i = 0; i < 8; i++) ms[i] += t[i];
+            }
 #pragma unroll
             for (int i = 0; i < W; i++) x[i] ^= ms[i];
         }
