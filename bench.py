@@ -492,7 +492,7 @@ def main():
                     "serial": {"value": world * BATCH * args.steps / (serial_total / 1e3),
                                "ms_per_step": serial_total / args.steps,
                                "mode": "one call at a time: upload, run, download per step"}},
-            "gpu_launches": (5 + 3) * args.steps,
+            "gpu_launches": round(sum(n for _, _, n in kern) / 3 + sum(n for _, _, n in vkern)) * args.steps,
             "kernels_ms": {name: round(m / n, 4) for name, m, n in kern},
             "verify_kernels_ms": {name: round(m / n, 4) for name, m, n in vkern},
             "roofline": {"bound": "int_alu", "kernel": "k_leaf_chains", "achieved": achieved,

@@ -1056,6 +1056,7 @@ void batch_direct_launch(cuspx_batch *b, bool on) {
     // (a three-set stream at 20k req/s: sign p99 6.6 -> 138 ms).
     if (on) {
         b->no_spec = true;
+        b->vlists.direct = true;
         for (int g = 0; g + 1 < VerifyFork::kMaxGroups; g++) {
             if (b->vfork.side[g]) {
                 cudaStreamSynchronize(b->vfork.side[g]);

@@ -24,10 +24,10 @@
 //
 // Verify: k_verify_msg (+ k_verify_msg_pair / _wide) -> k_verify_fors -> the
 // hypertree: for tiny batches every chain run from all 16 start steps, then a
-// serial walk (k_vspec_cand + k_vspec_walk, spx_vsort.cuh), one block per
-// item for small batches (k_verify_item, spx_verify.cuh), one persistent
-// launch for mid-size ones (k_verify_hyper),
-// per-layer kernels over length-sorted chains for large ones
+// serial walk (k_vspec_cand + k_vspec_walk, spx_vsort.cuh); up to about 4
+// items an SM one launch of blocks that keep 2 to 8 items (k_verify_block,
+// spx_vblock.cuh; SHAKE: k_verify_item and k_verify_hyper, spx_verify.cuh);
+// per-layer kernels over length-sorted chains for larger ones
 // (k_vsort_chains + k_vsort_layer, spx_vsort.cuh); or per-layer
 // k_verify_chains + k_verify_root, or k_verify_ht (one thread per item over
 // all layers).

@@ -10,6 +10,7 @@
 
 #include "spx_kernels.cuh"
 #include "spx_verify.cuh"
+#include "spx_vblock.cuh"
 #include "spx_vsort.cuh"
 
 namespace cuspx {
@@ -164,9 +165,22 @@ struct Family {
         if constexpr (kPersistVerify)
             if ((e = cudaFuncSetAttribute(k_verify_hyper<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
                 return e;
-        if ((e = cudaFuncSetAttribute(k_verify_item<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
+        if constexpr (HF::kShake)
+            if ((e = cudaFuncSetAttribute(k_verify_item<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
+                return e;
         if ((e = cudaFuncSetAttribute(k_vsort_layer<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
-        if ((e = cudaFuncSetAttribute(k_vspec_walk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
+        if constexpr (!HF::kShake) {
+            const void *blocks[] = {(const void *)k_verify_block<HF, 2>, (const void *)k_verify_block<HF, 4>,
+                                    (const void *)k_verify_block<HF, 8>};
+            for (const void *f : blocks)
+                if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
+            if ((e = cudaFuncSetAttribute(k_vsort_layer_group<HF, kGroupLanes>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
+                return e;
+        }
+        if constexpr (HF::kShake)
+            if ((e = cudaFuncSetAttribute(k_vspec_walk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
+                return e;
         if ((e = cudaFuncSetAttribute(k_fors_pk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         // Load every other kernel of the family now: with lazy module loading
         // a kernel's first launch loads it, and in a server that first launch
@@ -182,6 +196,7 @@ struct Family {
         for (const void *f : rest)
             if ((e = cudaFuncGetAttributes(&fa, f))) return e;
         if constexpr (!HF::kShake) {
+            if ((e = cudaFuncGetAttributes(&fa, (const void *)k_vspec_walk_group<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_sign_msg_pair<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_verify_msg_pair<HF>))) return e;
         } else {
@@ -191,10 +206,31 @@ struct Family {
         return cudaSuccess;
     }
 
-    // the persistent verify kernel covers every set (the robust SHA-256
-    // policy lays its slot out for subtrees of height <= 9, the tallest of
-    // any set)
-    static constexpr bool kPersistVerify = true;
+    // SHA-256: the whole hypertree in one launch of blocks of I items
+    // (spx_vblock.cuh).  More items a block fill its chain warps better but
+    // leave its one T warp fewer lanes an item; few blocks an SM are bound by
+    // a block's serial path, many by the SM.  Measured (ms, I = 2 / 4 / 8):
+    // 128f, 301 items 0.92 / 0.85 / 1.08, 1024 items 1.39 / 1.23 / 1.11; 192f
+    // 1.13 / 1.30 / 1.66, 2.27 / 1.96 / 1.76; 256f-robust 2.59 / 2.77 / 3.66,
+    // 7.5 / 4.9 / 4.0.  (One block an item with its T lane behind the chains,
+    // and warps that claim chains for up to 4 items, took 1.77 and 1.42 ms at
+    // 301 items of 128f, 7.8 and 9.2 ms of 256f-robust.)
+    static void verify_block(const SetParams &P, const VerifyArgs &A, cudaStream_t s) {
+        if constexpr (!HF::kShake) {
+            const uint64_t sms = (uint64_t)device_sms();
+            if (A.count > 4 * sms) block_launch<8>(P, A, s);
+            else if (N == 16 || A.count > 2 * sms) block_launch<4>(P, A, s);
+            else block_launch<2>(P, A, s);
+        }
+    }
+    template <int I>
+    static void block_launch(const SetParams &P, const VerifyArgs &A, cudaStream_t s) {
+        using VB = VerifyBlock<HF, I>;
+        k_verify_block<HF, I><<<ceil_div(A.count, I), VB::kThreads, VB::words(P.hp) * 4, s>>>(P, A);
+    }
+
+    // SHAKE-256: the persistent verify kernel
+    static constexpr bool kPersistVerify = HF::kShake;
 
     // one launch over the batch's whole hypertree: as many blocks as are
     // resident at once (or fewer for small batches); warps take items from
@@ -363,6 +399,19 @@ struct Family {
 
     static constexpr uint32_t kLayerSmem = 200u * 1024u;   // the shared-memory limit configure() sets
 
+    // SHA-256: batches of up to kGroupItems items run the layer kernel with
+    // kGroupLanes lanes an item (spx_vgroup.cuh), one item group: the lanes
+    // shorten the serial path (128f, 301 items: 0.92 ms a batch, against 1.33
+    // with a thread an item), but all repeat its rounds, which costs a third
+    // more issue slots, so larger batches take a thread an item and hide its
+    // latency behind other item groups' chains (128f, lanes / thread: 2048
+    // items 1.48 / 1.59 ms, 4096 2.45 / 2.22 ms; 192f 2.25 / 2.40, 3.65 / 3.29;
+    // robust, whose H masks the lanes share out: 4096 items of 192f 6.6 / 8.0
+    // ms, of 256s 5.0 / 5.2 ms, 8192 of 256s 10.4 / 9.7 ms).  32, 4 or 2 lanes
+    // are slower than 8 from 301 to 2048 items but for 2 at 2048 (1.40 ms).
+    static constexpr int kGroupLanes = 8;
+    static constexpr uint32_t kGroupItems = HF::kRobust ? 4096 : 2048;
+
     // verify_mode 3: per group of items, T_k then per layer the sorted
     // chains and the layer roots (spx_vsort.cuh).  Groups run on their own
     // streams; a group's chain kernel of layer L starts after the previous
@@ -372,7 +421,8 @@ struct Family {
     static void verify_sorted(const SetParams &P, const VerifyArgs &A, const Tuning &tu, cudaStream_t s,
                               PhaseTimer *pt, const VerifyLists &V, const VerifyFork *vf) {
         constexpr int LEN = 2 * N + 3;
-        int G = tu.verify_groups < 1 ? 1 : tu.verify_groups;
+        const bool grouped = !HF::kShake && A.count <= kGroupItems;
+        int G = grouped || tu.verify_groups < 1 ? 1 : tu.verify_groups;
         const int gmax = pt || !vf ? 1 : vf->sides + 1;
         if (G > gmax) G = gmax;
         if ((uint32_t)G > A.count) G = (int)A.count;
@@ -383,7 +433,17 @@ struct Family {
         // every set: SHAKE-256f-robust needs 176 KiB)
         int b = tu.verify_block;
         while (b > 32 && VsortSmem<HF>::bytes(P, (uint32_t)b) > kLayerSmem) b /= 2;
-        const size_t smem = VsortSmem<HF>::bytes(P, (uint32_t)b);
+        auto layer = [&](int L, uint32_t first, uint32_t n, int g, cudaStream_t st) {
+            if constexpr (!HF::kShake) {
+                if (grouped) {
+                    constexpr int kItems = 64 / kGroupLanes;
+                    k_vsort_layer_group<HF, kGroupLanes>
+                        <<<ceil_div(n, kItems), 64, kItems * ShaGroup<HF>::kStride * 4, st>>>(P, A, V, L, first, n, g);
+                    return;
+                }
+            }
+            k_vsort_layer<HF><<<ceil_div(n, b), b, VsortSmem<HF>::bytes(P, (uint32_t)b), st>>>(P, A, V, L, first, n, g);
+        };
         cudaMemsetAsync(V.cnt, 0, (size_t)G * P.d * 16 * sizeof(uint32_t), s);
         cudaStream_t gs[VerifyFork::kMaxGroups];
         gs[0] = s;
@@ -397,7 +457,7 @@ struct Family {
         for (int g = 0; g < G; g++) {
             k_verify_fors<HF><<<ceil_div((uint64_t)items(g) * P.k, 128), 128, 0, gs[g]>>>(P, A, first(g), items(g));
             CUSPX_MARK(pt, "k_verify_fors", s);
-            k_vsort_layer<HF><<<ceil_div(items(g), b), b, smem, gs[g]>>>(P, A, V, -1, first(g), items(g), g);
+            layer(-1, first(g), items(g), g, gs[g]);
             CUSPX_MARK(pt, "k_vsort_layer", s);
         }
         for (int L = 0; L < P.d; L++) {
@@ -406,7 +466,7 @@ struct Family {
                 k_vsort_chains<HF><<<ceil_div((uint64_t)items(g) * LEN, 128), 128, 0, gs[g]>>>(P, A, V, L, first(g), g);
                 CUSPX_MARK(pt, "k_vsort_chains", s);
                 if (g + 1 < G) cudaEventRecord(vf->chain[g], gs[g]);
-                k_vsort_layer<HF><<<ceil_div(items(g), b), b, smem, gs[g]>>>(P, A, V, L, first(g), items(g), g);
+                layer(L, first(g), items(g), g, gs[g]);
                 CUSPX_MARK(pt, "k_vsort_layer", s);
             }
         }
@@ -430,18 +490,24 @@ struct Family {
                 CUSPX_MARK(pt, "k_verify_msg_wide", s);
             }
         }
-        const bool want_sorted =
-            tu.verify_mode == 3 || (tu.verify_sorted_min > 0 && A.count >= (uint32_t)tu.verify_sorted_min);
-        const bool sorted = want_sorted && vl && vl->tasks && vl->stride >= (uint64_t)A.count * (2 * N + 3) &&
-                            A.count < (1u << 25) && VsortSmem<HF>::bytes(P, 32) <= kLayerSmem && P.len1 == 2 * N &&
-                            P.len2 == 3 && !(tu.verify_item_max > 0 && A.count <= (uint32_t)tu.verify_item_max);
+        const bool spec = tu.verify_mode != 3 && tu.verify_spec_max > 0 && A.count <= (uint32_t)tu.verify_spec_max &&
+                          vl && vl->cand && A.count <= vl->cand_items &&
+                          32u * VsortSmem<HF>::slot_stride(P.hp) * 4u <= kLayerSmem && P.len1 == 2 * N && P.len2 == 3;
+        const bool by_size = tu.verify_sorted_min > 0 && A.count >= (uint32_t)tu.verify_sorted_min && !spec;
+        const bool item = tu.verify_item_max > 0 && A.count <= (uint32_t)tu.verify_item_max;
+        // a SHA-256 batch of more than 4 items an SM has the throughput of the
+        // layers' own launches (128f, 700 items: 0.97 ms, fused 1.09), unless
+        // each is a host launch (serving) or sorted_min is 0
+        const bool layers = !HF::kShake && tu.verify_sorted_min > 0 && tu.verify_mode >= 2 && vl && !vl->direct &&
+                            A.count > 4u * (uint32_t)device_sms();
+        const bool sorted = (tu.verify_mode == 3 || by_size || layers) && vl && vl->tasks &&
+                            vl->stride >= (uint64_t)A.count * (2 * N + 3) && A.count < (1u << 25) &&
+                            VsortSmem<HF>::bytes(P, 32) <= kLayerSmem && P.len1 == 2 * N && P.len2 == 3 && !item;
         if (sorted) {   // FORS per item group, beside the other groups' layers
             verify_sorted(P, A, tu, s, pt, *vl, vf);
             return;
         }
-        if (tu.verify_spec_max > 0 && A.count <= (uint32_t)tu.verify_spec_max && vl && vl->cand &&
-            A.count <= vl->cand_items && 32u * VsortSmem<HF>::slot_stride(P.hp) * 4u <= kLayerSmem &&
-            P.len1 == 2 * N && P.len2 == 3) {
+        if (spec) {
             // tiny batches: every chain run from every start step, then the
             // serial walk over T_len and the auth paths alone (spx_vsort.cuh)
             // (the chain runs beside the FORS roots, on a side stream)
@@ -460,14 +526,23 @@ struct Family {
                 cudaEventRecord(vf->join[0], cs);
                 cudaStreamWaitEvent(s, vf->join[0], 0);
             }
-            k_vspec_walk<HF><<<ceil_div(A.count, 32), 32, 32u * VsortSmem<HF>::slot_stride(P.hp) * 4u, s>>>(
-                P, A, vl->cand);
+            if constexpr (!HF::kShake)
+                k_vspec_walk_group<HF><<<A.count, 32, ShaGroup<HF>::kWords * 4, s>>>(P, A, vl->cand);
+            else
+                k_vspec_walk<HF><<<ceil_div(A.count, 32), 32, 32u * VsortSmem<HF>::slot_stride(P.hp) * 4u, s>>>(
+                    P, A, vl->cand);
             CUSPX_MARK(pt, "k_vspec_walk", s);
             return;
         }
         k_verify_fors<HF><<<ceil_div((uint64_t)A.count * P.k, 128), 128, 0, s>>>(P, A, 0, A.count);
         CUSPX_MARK(pt, "k_verify_fors", s);
-        if (tu.verify_item_max > 0 && A.count <= (uint32_t)tu.verify_item_max && P.hp <= 9) {
+        if constexpr (!HF::kShake) {
+            if ((item || (tu.verify_mode >= 2 && A.ctr)) && P.hp <= 9) {
+                verify_block(P, A, s);
+                CUSPX_MARK(pt, "k_verify_block", s);
+                return;
+            }
+        } else if (item && P.hp <= 9) {
             // small batches: one item per block (its serial path sets the time)
             constexpr int LEN = 2 * N + 3, CW = (LEN + 31) / 32;
             // one slot and the prefetched auth path of the next layer
@@ -475,12 +550,11 @@ struct Family {
             k_verify_item<HF><<<A.count, 32 * (CW + 1), smem, s>>>(P, A);
             CUSPX_MARK(pt, "k_verify_item", s);
             return;
-        }
-        const int b = tu.verify_block;
-        if (tu.verify_mode >= 2 && kPersistVerify && A.ctr && P.hp <= 9) {
+        } else if (tu.verify_mode >= 2 && A.ctr && P.hp <= 9) {
             verify_persistent(P, A, tu, s, pt);
             return;
         }
+        const int b = tu.verify_block;
         if (tu.verify_mode == 1) {
             k_verify_ht<HF><<<ceil_div(A.count, b), b, (size_t)b * HF::kSmemWords * 4, s>>>(P, A);
             CUSPX_MARK(pt, "k_verify_ht", s);

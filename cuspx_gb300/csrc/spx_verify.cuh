@@ -1,4 +1,4 @@
-// spx_verify.cuh -- persistent hypertree verify (every parameter set).
+// spx_verify.cuh -- verify units and slots; persistent hypertree verify (SHAKE).
 //
 // crypto_sign_verify (sign.cu:3048-3121) is serial over the d layers of an
 // item: layer L's WOTS+ chains (wots_pk_from_sig, wots.cu:777-804) need the

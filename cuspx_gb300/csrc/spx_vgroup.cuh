@@ -1,0 +1,238 @@
+// spx_vgroup.cuh -- SHA-256 T_l and auth paths by a group of lanes per item.
+//
+// What is serial in a verify layer is T_len over the len chain ends (10
+// compressions at n = 16, 35 at n = 32) and the auth path.  A compression's
+// chaining goes through its rounds alone: the message schedules of all of
+// T_len's blocks are independent.  Here the G lanes of an item compute them
+// side by side (lane g those of blocks g, g + G, ...) into shared memory,
+// W_t + K_t, and then all run the rounds, the same ones in every lane, from
+// broadcast reads.  A warp alone on its SM takes 31 cycles a round that way,
+// against ~46 with the schedule in between, and beside other warps the serial
+// path issues 15 instead of 24 instructions a round.  Robust sets' bitmasks
+// of the auth path (and of T_k) depend on addresses alone and are computed by
+// the lanes side by side too.
+#pragma once
+#include "spx_kernels.cuh"
+
+namespace cuspx {
+
+template <class HF>
+struct ShaGroup {
+    static constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3, LEN1 = 2 * N;
+    static constexpr int blocks(int m) { return (22 + m * N + 9 + 63) / 64; }
+    static constexpr int NB = blocks(LEN);        // no set's T_k is longer
+    static constexpr int NBP = NB | 1;            // row of kw: an odd stride spreads the lanes' stores over the banks
+    static constexpr int kMaskH = HF::kRobust ? (2 * W + 7) / 8 : 0;   // mask blocks of an H
+    static constexpr int kMaxHp = 9;              // tallest subtree of any set
+    // an item's shared words: kw[t * NBP + block], the H masks, the layer's message
+    static constexpr int S_HM = 64 * NBP, S_ROOT = S_HM + kMaxHp * kMaskH * 8, kWords = S_ROOT + 8;
+    // a stride of 4 mod 32 keeps the groups of a warp in different banks
+    static constexpr int kStride = kWords + (36 - kWords % 32) % 32;
+
+    // rounds of one block from kw (stride NBP): h + K + W is ready a round early
+    SPX_DEV static void rounds(uint32_t st[8], const uint32_t *kw) {
+        uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6], h = st[7];
+        uint32_t hk = add_fma(h, kw[0]);
+#pragma unroll 1
+        for (int r = 0; r < 64; r += 16) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const uint32_t nx = add_fma(g, kw[((r + i + 1) & 63) * NBP]);
+                const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
+                const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
+                const uint32_t t1 = hk + S1 + ch;
+                const uint32_t na = add_fma(add_fma(S0, mj), t1);
+                hk = nx;
+                h = g;
+                g = f;
+                f = e;
+                e = add_fma(d, t1);
+                d = c;
+                c = b;
+                b = a;
+                a = na;
+            }
+        }
+        st[0] += a; st[1] += b; st[2] += c; st[3] += d; st[4] += e; st[5] += f; st[6] += g; st[7] += h;
+    }
+
+    // s <- compress(s, w) with each round's h + K + W made a round early and
+    // the schedule a round ahead of its use: for a warp alone on its SM (the
+    // walk of one 128f item 0.445 -> 0.432 ms against sha256_compress)
+    SPX_DEV static void compress_ahead(uint32_t s[8], uint32_t w[16]) {
+        uint32_t a = s[0], b = s[1], c = s[2], d = s[3], e = s[4], f = s[5], g = s[6], h = s[7];
+        uint32_t hk = h + (w[0] + sha256_k(0));
+#pragma unroll
+        for (int i = 0; i < 64; i++) {
+            const int t = i + 1;
+            if (t >= 16 && t < 64)
+                w[t & 15] = add_fma(w[t & 15], sha_sigma0(w[(t - 15) & 15]) + w[(t - 7) & 15] +
+                                                   sha_sigma1(w[(t - 2) & 15]));
+            const uint32_t nx = t < 64 ? g + (w[t & 15] + sha256_k(t & 63)) : 0u;
+            const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
+            const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
+            const uint32_t t1 = hk + S1 + ch;
+            hk = nx;
+            h = g;
+            g = f;
+            f = e;
+            e = add_fma(d, t1);
+            d = c;
+            c = b;
+            b = a;
+            a = t1 + (S0 + mj);
+        }
+        s[0] += a; s[1] += b; s[2] += c; s[3] += d; s[4] += e; s[5] += f; s[6] += g; s[7] += h;
+    }
+
+    // T_l of m values under ADRS pa into out, in every lane of the group; g
+    // the lane's number in it.  ld(q): bytes 8q .. 8q + 7 of the values (memory
+    // order), already xored with a robust set's mask unless `mask`.  Every lane
+    // of the warp calls this, with the same m.
+    template <int G, class LD>
+    SPX_DEV static void tl(uint32_t out[W], uint32_t *S, uint32_t g, const KeyRegs<N> &key, const Adrs &pa, int m,
+                           bool mask, LD ld) {
+        const int nb = blocks(m), Q = m * N / 8;
+        for (int j = (int)g; j < nb; j += G) {
+            uint32_t v[18], w[16];   // v[i]: value word 16j - 6 + i (see Sha2::t_values)
+#pragma unroll
+            for (int i = 0; i < 9; i++) {
+                const int q = 8 * j - 3 + i;
+                uint2 x = make_uint2(0u, 0u);
+                if (q >= 0 && q < Q) x = ld((uint32_t)q);
+                v[2 * i] = bswap32(x.x);
+                v[2 * i + 1] = bswap32(x.y);
+            }
+            if (HF::kRobust && mask) {
+#pragma unroll 1
+                for (int b = 0; b < 3; b++) {   // mask blocks 2j - 1, 2j, 2j + 1
+                    uint32_t x[8];
+                    if (2 * j - 1 + b >= 0) HF::mask_block(x, key.pub, pa, (uint32_t)(2 * j - 1 + b));
+#pragma unroll
+                    for (int i = 0; i < 18; i++) {
+                        const int p = 16 * j - 6 + i;
+                        if (p >= 0 && p < m * W && (i + 2) / 8 == b) v[i] ^= x[(i + 2) % 8];
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) w[i] = __funnelshift_l(v[i + 1], v[i], 16);
+            if (j == 0) {
+#pragma unroll
+                for (int i = 0; i < 5; i++) w[i] = pa.w[i];
+                w[5] |= pa.w[5] & 0xffff0000u;
+            }
+            const int pad = 5 + m * W - 16 * j;   // stream word that holds the padding byte
+#pragma unroll
+            for (int i = 0; i < 16; i++)
+                if (i == pad) w[i] |= 0x8000u;
+            if (j == nb - 1) w[15] = (uint32_t)(64 + 22 + m * N) * 8u;
+            sha256_schedule_kw<NBP>(S + j, w);
+        }
+        __syncwarp();
+        uint32_t st[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) st[i] = key.mid[i];
+#pragma unroll 1
+        for (int j = 0; j < nb; j++) rounds(st, S + j);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < W; i++) out[i] = st[i];
+    }
+
+    // robust sets: the H masks of the layer's auth path into the item's
+    // shared words, before climb; every lane of the warp calls this
+    template <int G>
+    SPX_DEV static void h_masks(uint32_t *S, uint32_t g, const KeyRegs<N> &key, int hp, Adrs ad, uint32_t idx) {
+        if constexpr (HF::kRobust) {
+            for (int t = (int)g; t < hp * kMaskH; t += G) {
+                const int h = t / kMaskH;
+                adrs_height(ad, h + 1);
+                adrs_index(ad, idx >> (h + 1));
+                uint32_t x[8];
+                HF::mask_block(x, key.pub, ad, (uint32_t)(t % kMaskH));
+#pragma unroll
+                for (int i = 0; i < 8; i++) S[S_HM + t * 8 + i] = x[i];
+            }
+            __syncwarp();
+        }
+    }
+
+    // root <- compute_root (utils.cu:94-135) of leaf `root` over the auth path
+    // at auth; ad: the layer's HASHTREE address
+    SPX_DEV static void climb(uint32_t root[W], const uint32_t *S, const KeyRegs<N> &key, int hp, Adrs ad, uint32_t idx,
+                              const uint8_t *auth) {
+        uint32_t nx[W];
+        HF::load(nx, auth);
+#pragma unroll 1
+        for (int h = 0; h < hp; h++) {
+            uint32_t in[2 * W], st[8];
+            const bool right = (idx >> h) & 1u;
+#pragma unroll
+            for (int i = 0; i < W; i++) {
+                in[i] = right ? nx[i] : root[i];
+                in[W + i] = right ? root[i] : nx[i];
+            }
+            if (h + 1 < hp) HF::load(nx, auth + (uint64_t)(h + 1) * N);
+            if constexpr (HF::kRobust) {
+#pragma unroll
+                for (int i = 0; i < 2 * W; i++) in[i] ^= S[S_HM + (h * kMaskH + i / 8) * 8 + i % 8];
+            }
+            adrs_height(ad, h + 1);
+            adrs_index(ad, idx >> (h + 1));
+#pragma unroll
+            for (int i = 0; i < 8; i++) st[i] = key.mid[i];
+#pragma unroll 1
+            for (int b = 0; b < HF::template kBlocks<2 * W>; b++) {
+                uint32_t w[16];
+                HF::template core_block<2 * W>(w, ad, in, b);
+                compress_ahead(st, w);
+            }
+#pragma unroll
+            for (int i = 0; i < W; i++) root[i] = st[i];
+        }
+    }
+
+    // checksum digits of a WOTS+ message (chain_lengths, wots.cu:84-166), 4 bits each
+    SPX_DEV static uint32_t checksum(const uint32_t msg[W]) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < W; i++)
+            sum += __dp4a((msg[i] & 0x0f0f0f0fu) + (msg[i] >> 4 & 0x0f0f0f0fu), 0x01010101u, 0u);
+        return (15u * LEN1 - sum) << 4;
+    }
+    // digit c of the message whose words are in S[S_ROOT ..]
+    SPX_DEV static uint32_t digit(const uint32_t *S, uint32_t csum, uint32_t c) {
+        if (c < (uint32_t)LEN1) return S[S_ROOT + (c >> 3)] >> (28 - 4 * (c & 7)) & 15u;
+        return csum >> (12 - 4 * (c - LEN1)) & 15u;
+    }
+
+    // The root of layer L of an item (L = -1: its FORS key), in every lane of
+    // its group; auth: the layer's auth path.  Every lane of the warp calls this.
+    template <int G, class LD>
+    SPX_DEV static void layer_root(uint32_t root[W], const SetParams &P, uint32_t *S, uint32_t g, const KeyRegs<N> &key,
+                                   uint64_t tree, uint32_t idx_leaf, const uint8_t *auth, int L, LD ld) {
+        uint64_t tree_L = tree;
+        uint32_t idx_L = idx_leaf;
+        Adrs pa;
+        adrs_zero(pa);
+        if (L >= 0) {
+            layer_index(P, tree, idx_leaf, L, tree_L, idx_L);
+            adrs_layer(pa, L);
+        }
+        adrs_tree(pa, tree_L);
+        adrs_keypair(pa, idx_L);
+        adrs_type(pa, L < 0 ? ADDR_FORSPK : ADDR_WOTSPK);
+        tl<G>(root, S, g, key, pa, L < 0 ? P.k : LEN, L < 0, ld);
+        if (L < 0) return;
+        Adrs ad;
+        adrs_zero(ad);
+        adrs_layer(ad, L);
+        adrs_tree(ad, tree_L);
+        adrs_type(ad, ADDR_HASHTREE);
+        h_masks<G>(S, g, key, P.hp, ad, idx_L);
+        climb(root, S, key, P.hp, ad, idx_L, auth);
+    }
+};
+
+}  // namespace cuspx

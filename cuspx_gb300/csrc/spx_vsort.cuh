@@ -37,6 +37,7 @@
 // the plain T_len absorb.
 #pragma once
 #include "spx_verify.cuh"
+#include "spx_vgroup.cuh"
 
 #define SPX_HD __host__ __device__ __forceinline__
 
@@ -52,6 +53,7 @@ struct VerifyLists {
     uint64_t stride = 0;         // entries per bucket: at least count x len
     uint8_t *cand = nullptr;     // speculative chain ends: cand_items x d x len x 16 x n, or null
     uint32_t cand_items = 0;
+    bool direct = false;         // the batch is launched kernel by kernel (serving), not as a graph
 };
 
 // steps of WOTS+ chain c for message msg: 15 - digit c (chain_lengths,
@@ -98,17 +100,19 @@ SPX_DEV void tlen_mask_value(uint32_t v[HF::W], const KeyRegs<4 * HF::W> &key, i
         adrs_tree(ta, tree_L);
         adrs_keypair(ta, idx_L);
         adrs_type(ta, ADDR_WOTSPK);
-        const uint32_t q0 = (uint32_t)c * W, b0 = q0 >> 3, b1 = (q0 + W - 1) >> 3;
-        uint32_t m0[8], m1[8];
-        HF::mask_block(m0, key.pub, ta, b0);
-        if (b1 != b0) HF::mask_block(m1, key.pub, ta, b1);
+        const uint32_t q0 = (uint32_t)c * W;
+#pragma unroll 1
+        for (uint32_t b = q0 >> 3; b <= (q0 + W - 1) >> 3; b++) {
+            uint32_t m[8];
+            HF::mask_block(m, key.pub, ta, b);
 #pragma unroll
-        for (int i = 0; i < W; i++) {
-            const uint32_t q = q0 + i, k = q & 7;
-            uint32_t mw = 0;
+            for (int i = 0; i < W; i++) {
+                const uint32_t q = q0 + i;
+                uint32_t mw = 0;
 #pragma unroll
-            for (int t = 0; t < 8; t++) mw = (uint32_t)t == k ? ((q >> 3) == b0 ? m0[t] : m1[t]) : mw;
-            v[i] ^= mw;
+                for (int t = 0; t < 8; t++) mw = 8 * b + t == q ? m[t] : mw;
+                v[i] ^= mw;
+            }
         }
     }
 }
@@ -364,6 +368,75 @@ __global__ void k_vsort_layer(SetParams P, VerifyArgs A, VerifyLists V, int L, u
     }
 }
 
+// The same for SHA-256 sets, by groups of G lanes per item (spx_vgroup.cuh).
+// Dynamic shared memory: blockDim / G x ShaGroup<HF>::kStride words.
+template <class HF, int G>
+__global__ void __launch_bounds__(128) k_vsort_layer_group(SetParams P, VerifyArgs A, VerifyLists V, int L,
+                                                           uint32_t first, uint32_t n, int grp) {
+    using SG = ShaGroup<HF>;
+    constexpr int W = SG::W, N = SG::N, LEN = SG::LEN, kPer = (LEN + G - 1) / G;
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ uint32_t hcount[16], hbase[16];
+    if (threadIdx.x < 16) hcount[threadIdx.x] = 0;
+    const uint32_t g = threadIdx.x % G, t = threadIdx.x / G;
+    const uint32_t j = blockIdx.x * (blockDim.x / G) + t;
+    const bool live = j < n;
+    const uint32_t i = first + (live ? j : 0);   // lanes past the end repeat the first item
+    uint32_t *S = smem + t * SG::kStride;
+    const SignWork &wk = A.work[i];
+    const bool ok = live && !wk.flags;
+    const uint8_t *pkb = A.pk.row(i);
+    KeyRegs<N> key;
+    key_from_work<HF>(key, pkb, pkb, wk);
+    const uint2 *src = reinterpret_cast<const uint2 *>((L < 0 ? A.fors_roots + (uint64_t)i * P.k * N
+                                                             : A.wpk + (uint64_t)i * LEN * N));
+    uint32_t root[W];
+    SG::template layer_root<G>(root, P, S, g, key, wk.tree, wk.idx_leaf,
+                               A.sig + (uint64_t)i * A.sig_stride + (L < 0 ? 0 : sig_layer_off(P, L) + P.wots_bytes), L,
+                               [&](uint32_t q) { return src[q]; });
+    if (L == P.d - 1) {   // uniform over the launch: no barrier follows
+        if (live && g == 0) {
+            uint32_t pr[W];
+            HF::load(pr, pkb + N);
+            bool eq = ok;
+#pragma unroll
+            for (int x = 0; x < W; x++) eq &= pr[x] == root[x];
+            A.verdict[i] = eq ? 0 : -1;
+        }
+        return;
+    }
+    // bucket layer L+1's chains: block-local ranks, one global reservation
+    // per bucket and block, then the entries
+    const uint32_t csum = SG::checksum(root);
+    if (g == 0) {
+#pragma unroll
+        for (int x = 0; x < W; x++) S[SG::S_ROOT + x] = root[x];
+    }
+    __syncthreads();
+    uint32_t lr[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint32_t c = g + G * k;
+        if (ok && c < (uint32_t)LEN) {
+            const uint32_t l = 15u - SG::digit(S, csum, c);
+            lr[k] = l << 16 | atomicAdd(&hcount[l], 1u);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 16 && hcount[threadIdx.x])
+        hbase[threadIdx.x] = atomicAdd(&V.cnt[((uint64_t)grp * P.d + L + 1) * 16 + threadIdx.x], hcount[threadIdx.x]);
+    __syncthreads();
+    uint32_t *base = V.tasks + (uint64_t)first * LEN;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const uint32_t c = g + G * k;
+        if (ok && c < (uint32_t)LEN) {
+            const uint32_t l = lr[k] >> 16;
+            base[(uint64_t)l * V.stride + hbase[l] + (lr[k] & 0xffffu)] = i << 7 | c;
+        }
+    }
+}
+
 // One lane per chain of layer L, in sorted order (most steps first; the
 // zero-step chains, plain copies, last): sorted position p of the group ->
 // bucket and entry.
@@ -537,6 +610,51 @@ __global__ void __launch_bounds__(32) k_vspec_walk(SetParams P, VerifyArgs A, co
 #pragma unroll
     for (int x = 0; x < W; x++) eq &= pr[x] == root[x];
     A.verdict[i] = eq ? 0 : -1;
+}
+
+// The same for SHA-256 sets, a warp per item (spx_vgroup.cuh): a lane that
+// builds a T_len block picks the chain ends it covers.  Dynamic shared
+// memory: ShaGroup<HF>::kWords words.
+template <class HF>
+__global__ void __launch_bounds__(32) k_vspec_walk_group(SetParams P, VerifyArgs A, const uint8_t *cand) {
+    using SG = ShaGroup<HF>;
+    constexpr int W = SG::W, N = SG::N, LEN = SG::LEN, NW = N / 8;
+    extern __shared__ __align__(16) uint32_t S[];
+    const uint32_t i = blockIdx.x, g = threadIdx.x;
+    const SignWork &wk = A.work[i];
+    if (wk.flags) {   // wrong signature length (sign.cu:3063-3065)
+        if (g == 0) A.verdict[i] = -1;
+        return;
+    }
+    const uint8_t *pkb = A.pk.row(i), *sig = A.sig + (uint64_t)i * A.sig_stride;
+    KeyRegs<N> key;
+    key_from_work<HF>(key, pkb, pkb, wk);
+    const uint64_t tree = wk.tree;
+    const uint32_t idx_leaf = wk.idx_leaf;
+    uint32_t root[W], csum = 0;
+#pragma unroll 1
+    for (int L = -1; L < P.d; L++) {
+        const uint8_t *cb = L < 0 ? A.fors_roots + (uint64_t)i * P.k * N
+                                  : cand + ((uint64_t)i * P.d + L) * LEN * 16 * N;
+        const uint8_t *auth = sig + (L < 0 ? 0 : sig_layer_off(P, L) + P.wots_bytes);
+        SG::template layer_root<32>(root, P, S, g, key, tree, idx_leaf, auth, L, [&](uint32_t q) {
+            const uint32_t c = q / NW;
+            const uint8_t *v = cb + (L < 0 ? (uint64_t)c : (uint64_t)c * 16 + SG::digit(S, csum, c)) * N;
+            return reinterpret_cast<const uint2 *>(v)[q % NW];
+        });
+        csum = SG::checksum(root);
+        if (g == 0) {
+#pragma unroll
+            for (int x = 0; x < W; x++) S[SG::S_ROOT + x] = root[x];
+        }
+        __syncwarp();
+    }
+    uint32_t pr[W];
+    HF::load(pr, pkb + N);
+    bool eq = true;
+#pragma unroll
+    for (int x = 0; x < W; x++) eq &= pr[x] == root[x];
+    if (g == 0) A.verdict[i] = eq ? 0 : -1;
 }
 
 }  // namespace cuspx

@@ -68,24 +68,28 @@ typedef struct {
     int tree_warps;       /* warps per block, XMSS tree kernel */
     int chains_per_warp;  /* (item, chain) tasks per warp, verify chain kernel */
     int verify_mode;      /* 0 layered verify kernels, 1 one thread per item over all layers,
-                             2 one persistent launch over the whole hypertree (default),
+                             2 one launch over the whole hypertree (default; SHA-256 batches of
+                             more than 4 items an SM as mode 3 unless verify_sorted_min is 0),
                              3 layered kernels with each layer's WOTS+ chains sorted by length */
     int fors_lanes_log2;  /* lanes per FORS tree = 2^g, g in 0..5 (0: lane per tree, 5: warp per tree) */
     int tree_mode;        /* 0 warp per XMSS subtree, 1 lane per subtree (heights <= 4 only) */
     int chain_mode_max;   /* 0: XMSS leaves one lane per leaf.  Otherwise one lane per WOTS+
                              chain, batches of at most this many signatures (up to 256) with
                              the T_len kernel of the lower latency */
-    int verify_slots;     /* most items a warp holds at once in verify_mode 2 (1..8); batches
-                             below about 4 warps per SM use fewer */
-    int verify_item_max;  /* verify batches of at most this many items (any verify_mode) with one
-                             thread block per item: a thread per WOTS+ chain and a T lane that
-                             streams T_len behind the chains (0: never) */
-    int verify_claim_min; /* verify_mode 2: WOTS+ chains are handed out to free lanes once at
+    int verify_slots;     /* SHAKE: most items a warp holds at once in verify_mode 2 (1..8);
+                             batches below about 4 warps per SM use fewer */
+    int verify_item_max;  /* verify batches of at most this many items (any verify_mode) in one
+                             launch: SHAKE one thread block per item, a thread per WOTS+ chain
+                             and a T lane that streams T_len behind the chains, SHA-256 blocks
+                             of a few items (0: never) */
+    int verify_claim_min; /* SHAKE, verify_mode 2: WOTS+ chains are handed out to free lanes once at
                              least this many lanes of a warp are free (1..32; T streams always
                              at once) */
     int verify_groups;    /* sorted verify: the batch is split into this many groups of items
                              (1..8), each on its own stream, so that one group's serial T_len
-                             and auth-path kernel overlaps another group's chains */
+                             and auth-path kernel overlaps another group's chains (SHA-256
+                             batches of up to 2048 items, 4096 robust, run as one group whose
+                             layer kernel has 8 lanes an item) */
     int verify_sorted_min;/* verify batches of at least this many items run the sorted layered
                              verify whatever verify_mode says (0: only with verify_mode 3);
                              batches up to verify_item_max still run one item per block */

@@ -1,0 +1,100 @@
+"""SHA-256 verify batches through the sorted layers, the fused blocks and the
+speculative walk, by groups of lanes and by a thread per item, at the sizes
+where a block, a warp or an item group is part full: good signatures pass, a
+signature with one byte changed anywhere is rejected, and its neighbours are
+not disturbed.
+"""
+import random
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SETS = ["sha256-%s-%s" % (s, m) for s in ("128s", "128f", "192s", "192f", "256s", "256f") for m in ("simple", "robust")]
+
+
+@pytest.fixture(scope="module")
+def engine():
+    import cuspx_gb300
+    eng = cuspx_gb300.Engine(0)
+    yield eng
+    eng.close()
+
+
+@pytest.fixture(scope="module")
+def pool(engine):
+    """64 signed messages of a set, two of them checked against the oracle (f sets; the s
+    sets' signatures are in test_gpu_sign_paths.py)"""
+    import spx_oracle
+    made = {}
+
+    def get(setname):
+        if setname not in made:
+            sid = engine.set_id(setname)
+            rng = random.Random(3)
+            o = spx_oracle.Oracle(setname)
+            pks, sks = engine.keypair_batch(sid, [rng.randbytes(o.p.seed_bytes) for _ in range(3)])
+            msgs = [rng.randbytes(rng.randrange(0, 300)) for _ in range(64)]
+            sigs, st = engine.sign_batch(sid, [sks[i % 3] for i in range(64)], msgs)
+            assert not any(st)
+            for i in (0, 63) if setname.split("-")[1].endswith("f") else ():
+                assert sigs[i] == o.sign(msgs[i], sks[i % 3])
+            made[setname] = [(pks[i % 3], msgs[i], sigs[i]) for i in range(64)]
+        return made[setname]
+
+    return get
+
+
+def _check(engine, sid, items, count, seed):
+    rng = random.Random(seed)
+    pk, msg, sig, want = [], [], [], []
+    for i in range(count):
+        p, m, s = items[i % len(items)]
+        bad = rng.random() < 0.4
+        if bad:
+            s = bytearray(s)
+            s[rng.randrange(len(s))] ^= 1 << rng.randrange(8)
+        pk.append(p)
+        msg.append(m)
+        sig.append(bytes(s))
+        want.append(-1 if bad else 0)
+    assert list(engine.verify_batch(sid, pk, msg, sig)) == want
+
+
+@pytest.mark.parametrize("setname", SETS)
+def test_sorted_layers(engine, pool, setname):
+    sid = engine.set_id(setname)
+    saved = engine.get_tuning(sid)
+    try:
+        for count, groups in ((1, 1), (7, 1), (9, 2), (65, 4), (301, 1), (1300, 2)):
+            engine.set_tuning(sid, verify_spec_max=0, verify_item_max=0, verify_mode=3, verify_groups=groups)
+            _check(engine, sid, pool(setname), count, count)
+    finally:
+        engine.set_tuning(sid, **saved)
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-128f-simple", 2049), ("sha256-192f-simple", 2500),
+                                           ("sha256-256s-simple", 2049), ("sha256-128s-robust", 4097),
+                                           ("sha256-192s-robust", 4100), ("sha256-256s-robust", 4097)])
+def test_sorted_layers_thread_per_item(engine, pool, setname, count):
+    """the first sizes past the lanes-per-item layer kernel"""
+    _check(engine, engine.set_id(setname), pool(setname), count, count)
+
+
+@pytest.mark.parametrize("setname", SETS)
+def test_default_mapping_edges(engine, pool, setname):
+    """the sizes at which the default mapping changes (of 152 SMs)"""
+    for count in (32, 33, 64, 65, 129, 305, 609, 1023):
+        _check(engine, engine.set_id(setname), pool(setname), count, count)
+
+
+@pytest.mark.parametrize("setname", SETS)
+def test_speculative_walk(engine, pool, setname):
+    sid = engine.set_id(setname)
+    saved = engine.get_tuning(sid)
+    try:
+        engine.set_tuning(sid, verify_spec_max=64)
+        for count in (1, 2, 33, 64):
+            _check(engine, sid, pool(setname), count, count)
+    finally:
+        engine.set_tuning(sid, **saved)
