@@ -296,23 +296,20 @@ int cuspx_create(int device, cuspx_ctx **out) {
         // 4 slots 98.9 ms; 4096 SHA-256-192f-robust 11.9 / 12.8 ms), except
         // robust SHA-256 at n = 32 (4096 SHA-256-256f-robust 22.8 / 21.1 ms)
         if (sd.robust && !(sd.hash == 0 && sd.n == 32)) t.verify_slots = 2;
-        // one item per block up to 128 items: SHA-256-128f 1 item 0.98 ms
-        // against 1.18 ms persistent, 128 items 1.00 / 1.20 ms, 256 items
-        // 1.44 / 1.22 ms (SHAKE-256f and robust SHA-256-192f cross over
-        // between 64 and 256 as well)
-        t.verify_item_max = 128;
-        // the sorted layered verify from 2048 items; from 1024 for the
-        // SHA-256 f sets and robust SHA-256, from 512 for robust SHA-256 at
-        // n = 32 and 192f (4096 SHA-256-128f 2.31 ms against 3.65 ms
-        // persistent, 1024 items 1.39 / 1.64 ms, 512 items 1.38 / 1.42 ms;
-        // SHAKE-256f 1024 items 4.33 / 4.05 ms, 2048 items 6.76 / 8.09 ms;
-        // SHA-256-256f-robust 512 items 4.70 / 9.70 ms, SHA-256-128f-robust
-        // 512 items 2.92 / 2.76 ms, 1024 items 2.99 / 3.36 ms)
+        // one launch of blocks of a few items for SHA-256 up to 128 items
+        // whatever the mode; SHAKE takes the sorted layers at every size
+        // above verify_spec_max (256f, 64 items: 2.29 ms, one item per block
+        // 2.85 ms), except in a server
+        t.verify_item_max = sd.hash == 0 ? 128 : 0;
+        // the sorted layered verify for SHA-256 from 1024 items for the f
+        // sets, 2048 for the s sets, robust from 512 at n = 32 and 192f and
+        // from 1024 otherwise (the launch code takes it from 4 items an SM
+        // where it may, see Family::verify)
         // speculative chains up to 32 items, 64 for robust SHA-256 (1 item
-        // SHA-256-128f 0.54 ms against 0.88 ms one block per item, 32 items
-        // 0.78 / 0.87 ms, 64 items 0.95 / 0.88 ms; SHA-256-192f-robust 1 item
-        // 1.62 / 3.33 ms, 64 items 2.83 / 3.47 ms; SHAKE-256f 1 item 2.01 /
-        // 3.09 ms, 32 items 3.03 / 3.12 ms)
+        // SHA-256-128f 0.43 ms against 0.85 ms in a fused block, 32 items 0.59
+        // / 0.84 ms; SHA-256-192f-robust 1 item 0.89 / 2.2 ms, 64 items 2.07 /
+        // 2.16 ms; SHAKE-256f 1 item 1.13 / 2.29 ms in sorted layers, 32 items
+        // 2.04 / 2.29 ms)
         t.verify_spec_max = (sd.hash == 0 && sd.robust) ? 64 : 32;
         const bool f_set = sd.h / sd.d <= 4;
         if (sd.hash == 0 && sd.robust) t.verify_sorted_min = (sd.n == 32 || (sd.n == 24 && f_set)) ? 512 : 1024;
@@ -602,6 +599,9 @@ extern "C" {
 // ---------------------------------------------------------------------------
 // batches
 // ---------------------------------------------------------------------------
+// bytes of one layer's masks of an item (robust SHAKE, ShakeGroup::mask_lanes)
+static size_t shake_mask_bytes(const SetParams &P) { return (size_t)(P.len + 2 * P.hp) * P.n; }
+
 static int balloc(cuspx_batch *b, void **p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) return CUSPX_OK;
@@ -725,6 +725,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
             b->vlists.stride = cap * P.len;
             A((void **)&b->vlists.tasks, 16 * b->vlists.stride * sizeof(uint32_t));
             A((void **)&b->vlists.cnt, (size_t)VerifyFork::kMaxGroups * P.d * 16 * sizeof(uint32_t));
+            if (sd.hash == 1 && sd.robust) A((void **)&b->vlists.masks, cap * shake_mask_bytes(P));
         }
     }
     if (rc != CUSPX_OK) {
@@ -900,13 +901,17 @@ static void spec_scratch(cuspx_batch *b) {
     if (tu.verify_spec_max <= 0 || b->count > (size_t)tu.verify_spec_max) return;
     const SetParams &P = b->P;
     const size_t items = std::min<size_t>(b->cap, kSpecItems);
+    const SetDesc &sd = kSets[b->set];
+    const size_t ends = items * P.d * P.len * 16 * P.n;
+    const size_t masks = sd.hash == 1 && sd.robust ? items * P.d * shake_mask_bytes(P) : 0;
     void *p = nullptr;
-    if (cudaMalloc(&p, items * P.d * P.len * 16 * P.n) != cudaSuccess) {
+    if (cudaMalloc(&p, ends + masks) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
     b->allocs.push_back(p);
     b->vlists.cand = (uint8_t *)p;
+    if (masks) b->vlists.cand_masks = (uint64_t *)((uint8_t *)p + ends);
     b->vlists.cand_items = (uint32_t)items;
 }
 

@@ -24,11 +24,11 @@
 //
 // Verify: k_verify_msg (+ k_verify_msg_pair / _wide) -> k_verify_fors -> the
 // hypertree: for tiny batches every chain run from all 16 start steps, then a
-// serial walk (k_vspec_cand + k_vspec_walk, spx_vsort.cuh); up to about 4
-// items an SM one launch of blocks that keep 2 to 8 items (k_verify_block,
-// spx_vblock.cuh; SHAKE: k_verify_item and k_verify_hyper, spx_verify.cuh);
-// per-layer kernels over length-sorted chains for larger ones
-// (k_vsort_chains + k_vsort_layer, spx_vsort.cuh); or per-layer
+// serial walk (k_vspec_cand + k_vspec_walk_*, spx_vsort.cuh); for SHA-256 up
+// to about 4 items an SM one launch of blocks that keep 2 to 8 items
+// (k_verify_block, spx_vblock.cuh), for SHAKE in a server k_verify_item and
+// k_verify_hyper (spx_verify.cuh); otherwise per-layer kernels over
+// length-sorted chains (k_vsort_chains + k_vsort_layer*, spx_vsort.cuh); or per-layer
 // k_verify_chains + k_verify_root, or k_verify_ht (one thread per item over
 // all layers).
 // Key generation reuses the leaf and tree kernels on the top layer.

@@ -178,9 +178,6 @@ struct Family {
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
                 return e;
         }
-        if constexpr (HF::kShake)
-            if ((e = cudaFuncSetAttribute(k_vspec_walk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
-                return e;
         if ((e = cudaFuncSetAttribute(k_fors_pk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         // Load every other kernel of the family now: with lazy module loading
         // a kernel's first launch loads it, and in a server that first launch
@@ -200,6 +197,8 @@ struct Family {
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_sign_msg_pair<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_verify_msg_pair<HF>))) return e;
         } else {
+            if ((e = cudaFuncGetAttributes(&fa, (const void *)k_vsort_layer_warp<HF>))) return e;
+            if ((e = cudaFuncGetAttributes(&fa, (const void *)k_vspec_walk_warp<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_sign_msg_wide<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_verify_msg_wide<HF>))) return e;
         }
@@ -409,8 +408,13 @@ struct Family {
     // robust, whose H masks the lanes share out: 4096 items of 192f 6.6 / 8.0
     // ms, of 256s 5.0 / 5.2 ms, 8192 of 256s 10.4 / 9.7 ms).  32, 4 or 2 lanes
     // are slower than 8 from 301 to 2048 items but for 2 at 2048 (1.40 ms).
+    // SHAKE-256: a warp an item, with the masks of robust sets squeezed by
+    // threads of the chain launch (256f, warp / thread an item: 301 items 2.30
+    // / 3.47 ms, 2048 5.76 / 6.00, 4096 9.9 / 9.1; 256f-robust 3.44 / 6.27,
+    // 2048 items 9.8 / 12.0, 8192 34.9 / 34.9); one item group up to 4 items
+    // an SM (128s-robust, 1024 items: 1.76 ms in one, 2.06 in four).
     static constexpr int kGroupLanes = 8;
-    static constexpr uint32_t kGroupItems = HF::kRobust ? 4096 : 2048;
+    static constexpr uint32_t kGroupItems = HF::kShake ? (HF::kRobust ? 8192 : 2048) : (HF::kRobust ? 4096 : 2048);
 
     // verify_mode 3: per group of items, T_k then per layer the sorted
     // chains and the layer roots (spx_vsort.cuh).  Groups run on their own
@@ -421,8 +425,9 @@ struct Family {
     static void verify_sorted(const SetParams &P, const VerifyArgs &A, const Tuning &tu, cudaStream_t s,
                               PhaseTimer *pt, const VerifyLists &V, const VerifyFork *vf) {
         constexpr int LEN = 2 * N + 3;
-        const bool grouped = !HF::kShake && A.count <= kGroupItems;
-        int G = grouped || tu.verify_groups < 1 ? 1 : tu.verify_groups;
+        const bool grouped = A.count <= kGroupItems && (!HF::kShake || !HF::kRobust || V.masks);
+        const bool one = grouped && (!HF::kShake || A.count <= 4u * (uint32_t)device_sms());
+        int G = one || tu.verify_groups < 1 ? 1 : tu.verify_groups;
         const int gmax = pt || !vf ? 1 : vf->sides + 1;
         if (G > gmax) G = gmax;
         if ((uint32_t)G > A.count) G = (int)A.count;
@@ -434,6 +439,12 @@ struct Family {
         int b = tu.verify_block;
         while (b > 32 && VsortSmem<HF>::bytes(P, (uint32_t)b) > kLayerSmem) b /= 2;
         auto layer = [&](int L, uint32_t first, uint32_t n, int g, cudaStream_t st) {
+            if constexpr (HF::kShake) {
+                if (grouped) {
+                    k_vsort_layer_warp<HF><<<ceil_div(n, 4), 128, 0, st>>>(P, A, V, L, first, n, g);
+                    return;
+                }
+            }
             if constexpr (!HF::kShake) {
                 if (grouped) {
                     constexpr int kItems = 64 / kGroupLanes;
@@ -463,7 +474,9 @@ struct Family {
         for (int L = 0; L < P.d; L++) {
             for (int g = 0; g < G; g++) {
                 if (g > 0) cudaStreamWaitEvent(gs[g], vf->chain[g - 1], 0);
-                k_vsort_chains<HF><<<ceil_div((uint64_t)items(g) * LEN, 128), 128, 0, gs[g]>>>(P, A, V, L, first(g), g);
+                const uint32_t mb = grouped && HF::kShake && HF::kRobust ? ceil_div(2ull * items(g), 128) : 0;
+                k_vsort_chains<HF><<<mb + ceil_div((uint64_t)items(g) * LEN, 128), 128, 0, gs[g]>>>(
+                    P, A, V, L, first(g), g, items(g), mb);
                 CUSPX_MARK(pt, "k_vsort_chains", s);
                 if (g + 1 < G) cudaEventRecord(vf->chain[g], gs[g]);
                 layer(L, first(g), items(g), g, gs[g]);
@@ -492,14 +505,17 @@ struct Family {
         }
         const bool spec = tu.verify_mode != 3 && tu.verify_spec_max > 0 && A.count <= (uint32_t)tu.verify_spec_max &&
                           vl && vl->cand && A.count <= vl->cand_items &&
-                          32u * VsortSmem<HF>::slot_stride(P.hp) * 4u <= kLayerSmem && P.len1 == 2 * N && P.len2 == 3;
+                          P.len1 == 2 * N && P.len2 == 3;
         const bool by_size = tu.verify_sorted_min > 0 && A.count >= (uint32_t)tu.verify_sorted_min && !spec;
-        const bool item = tu.verify_item_max > 0 && A.count <= (uint32_t)tu.verify_item_max;
-        // a SHA-256 batch of more than 4 items an SM has the throughput of the
-        // layers' own launches (128f, 700 items: 0.97 ms, fused 1.09), unless
-        // each is a host launch (serving) or sorted_min is 0
-        const bool layers = !HF::kShake && tu.verify_sorted_min > 0 && tu.verify_mode >= 2 && vl && !vl->direct &&
-                            A.count > 4u * (uint32_t)device_sms();
+        const bool direct = vl && vl->direct;   // each launch is a host launch (serving)
+        const bool item = A.count <= (uint32_t)(tu.verify_item_max > 0 ? tu.verify_item_max : 0) ||
+                          (HF::kShake && direct && A.count <= 128);
+        // launches of their own for the layers pay above 4 items an SM for
+        // SHA-256 (128f, 700 items: 0.97 ms, fused 1.09) and at every size for
+        // SHAKE-256 (256f, 64 items: 2.29 ms, one item per block 2.85; 301
+        // items 2.30, persistent 3.11), unless sorted_min is 0
+        const bool layers = tu.verify_sorted_min > 0 && tu.verify_mode >= 2 && !direct && !spec &&
+                            (HF::kShake || A.count > 4u * (uint32_t)device_sms());
         const bool sorted = (tu.verify_mode == 3 || by_size || layers) && vl && vl->tasks &&
                             vl->stride >= (uint64_t)A.count * (2 * N + 3) && A.count < (1u << 25) &&
                             VsortSmem<HF>::bytes(P, 32) <= kLayerSmem && P.len1 == 2 * N && P.len2 == 3 && !item;
@@ -518,7 +534,9 @@ struct Family {
                 cudaEventRecord(vf->fork, s);
                 cudaStreamWaitEvent(cs, vf->fork, 0);
             }
-            k_vspec_cand<HF><<<ceil_div(16ull * A.count * P.d * LEN, 128), 128, 0, cs>>>(P, A, vl->cand);
+            const uint64_t mask_tasks = HF::kShake && HF::kRobust ? 2ull * A.count * P.d : 0;
+            k_vspec_cand<HF><<<ceil_div(16ull * A.count * P.d * LEN + mask_tasks, 128), 128, 0, cs>>>(
+                P, A, vl->cand, vl->cand_masks);
             CUSPX_MARK(pt, "k_vspec_cand", s);
             k_verify_fors<HF><<<ceil_div((uint64_t)A.count * P.k, 128), 128, 0, s>>>(P, A, 0, A.count);
             CUSPX_MARK(pt, "k_verify_fors", s);
@@ -529,8 +547,7 @@ struct Family {
             if constexpr (!HF::kShake)
                 k_vspec_walk_group<HF><<<A.count, 32, ShaGroup<HF>::kWords * 4, s>>>(P, A, vl->cand);
             else
-                k_vspec_walk<HF><<<ceil_div(A.count, 32), 32, 32u * VsortSmem<HF>::slot_stride(P.hp) * 4u, s>>>(
-                    P, A, vl->cand);
+                k_vspec_walk_warp<HF><<<A.count, 32, 0, s>>>(P, A, vl->cand, vl->cand_masks);
             CUSPX_MARK(pt, "k_vspec_walk", s);
             return;
         }

@@ -1,6 +1,6 @@
-// spx_vgroup.cuh -- SHA-256 T_l and auth paths by a group of lanes per item.
+// spx_vgroup.cuh -- verify: T_l and auth paths by a group of lanes per item.
 //
-// What is serial in a verify layer is T_len over the len chain ends (10
+// SHA-256.  What is serial in a verify layer is T_len over the len chain ends (10
 // compressions at n = 16, 35 at n = 32) and the auth path.  A compression's
 // chaining goes through its rounds alone: the message schedules of all of
 // T_len's blocks are independent.  Here the G lanes of an item compute them
@@ -234,5 +234,188 @@ struct ShaGroup {
         climb(root, S, key, P.hp, ad, idx_L, auth);
     }
 };
+
+// ---------------------------------------------------------------------------
+// SHAKE-256 T_l and auth paths by a warp per item: the sponge state spread
+// over the warp (warp_keccak_f1600), lane j < 17 absorbing lane j of each
+// block.  A permutation is 1,080 instructions of the warp instead of 4,300 of
+// one thread: 3.0 us against 4.3 for a warp alone on its SM, and a quarter of
+// the time beside chain warps that share its scheduler.  Robust sets' masks
+// depend on addresses alone: threads of the chain kernels squeeze them
+// (shake_mask_task) while the chains run.
+// ---------------------------------------------------------------------------
+template <class HF>
+struct ShakeGroup {
+    static constexpr int W = HF::W, N = 4 * W, NL = N / 8, LEN = 2 * N + 3, LEN1 = 2 * N, PL = NL + 4;
+    // 64-bit words of a layer's masks of one item: T_len's, then 2n bytes per H
+    static __host__ __device__ constexpr int mask_lanes(int hp) { return LEN * NL + hp * 2 * NL; }
+
+    // lane p of PUB_SEED || ADRS (p < PL)
+    SPX_DEV static uint64_t prefix(const uint8_t *pk, const Adrs &a, uint32_t p) {
+        uint64_t al[4];
+        adrs_lanes(a, al);
+        uint64_t x = p < (uint32_t)NL ? reinterpret_cast<const uint64_t *>(pk)[p < (uint32_t)NL ? p : 0] : 0ull;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (p == (uint32_t)(NL + i)) x = al[i];
+        return x;
+    }
+
+    // T_l of m values under ADRS pa: lane i < NL returns lane i of the result.
+    // ld(q): lane q of the values, masked already unless `mask`.
+    template <class LD>
+    SPX_DEV static uint64_t tl(const KeccakLane &k, uint32_t lane, const uint8_t *pk, const Adrs &pa, int m, bool mask,
+                               LD ld) {
+        const int Q = m * NL, nb = (PL + Q) / 17 + 1;
+        const uint64_t pre = lane < (uint32_t)PL ? prefix(pk, pa, lane) : 0ull;
+        auto block = [&](int b) -> uint64_t {
+            const int q = 17 * b + (int)lane - PL;
+            if (lane >= 17) return 0ull;
+            if (q < 0) return pre;
+            uint64_t x = q < Q ? ld((uint32_t)q) : (q == Q ? 0x1Full : 0ull);
+            if (b == nb - 1 && lane == 16) x ^= 0x8000000000000000ull;
+            return x;
+        };
+        uint64_t a = 0, ms = 0, last = 0, nxt = block(0);
+        if (HF::kRobust && mask) {   // SHAKE256(PUB_SEED || ADRS), squeezed a block ahead
+            ms = pre ^ (lane == (uint32_t)PL ? 0x1Full : 0ull) ^ (lane == 16 ? 0x8000000000000000ull : 0ull);
+        }
+#pragma unroll 1
+        for (int b = 0; b < nb; b++) {
+            uint64_t cur = nxt;
+            if (b + 1 < nb) nxt = block(b + 1);
+            if (HF::kRobust && mask) {
+                // block b's value lanes take mask lanes 17b - PL ..: the end of
+                // mask block b - 1, then block b
+                warp_keccak_f1600(ms, k, lane);
+                const uint64_t hi = shfl64(last, (lane + 17 - PL) & 31), lo = shfl64(ms, (lane - PL) & 31);
+                const int q = 17 * b + (int)lane - PL;
+                if (lane < 17 && q >= 0 && q < Q) cur ^= lane < (uint32_t)PL ? hi : lo;
+                last = ms;
+            }
+            a ^= cur;
+            warp_keccak_f1600(a, k, lane);
+        }
+        return a;
+    }
+
+    // compute_root (utils.cu:94-135) of the leaf in `a` (lane i < NL) over the
+    // auth path at auth; masks: 2 NL lanes per H (robust)
+    SPX_DEV static uint64_t climb(uint64_t a, const KeccakLane &k, uint32_t lane, const uint8_t *pk, int hp, Adrs ad,
+                                  uint32_t idx, const uint8_t *auth, const uint64_t *masks) {
+        const int v = (int)lane - PL;   // value lane of l || r
+        const bool in = v >= 0 && v < 2 * NL;
+        for (int h = 0; h < hp; h++) {
+            const bool right = (idx >> h) & 1u;
+            adrs_height(ad, h + 1);
+            adrs_index(ad, idx >> (h + 1));
+            const uint64_t mine = shfl64(a, (uint32_t)(v - (right ? NL : 0)) & 31u);
+            uint64_t x = lane < (uint32_t)PL ? prefix(pk, ad, lane) : 0ull;
+            if (in) {
+                const bool own = (v >= NL) == right;
+                x = own ? mine : reinterpret_cast<const uint64_t *>(auth + (uint64_t)h * N)[right ? v : v - NL];
+                if (HF::kRobust) x ^= masks[h * 2 * NL + v];
+            }
+            if (lane == PL + 2 * NL) x ^= 0x1Full;
+            if (lane == 16) x ^= 0x8000000000000000ull;
+            a = x;
+            warp_keccak_f1600(a, k, lane);
+        }
+        return a;
+    }
+
+    // the root of layer L (-1: the FORS key): lane i < NL returns lane i;
+    // masks: the layer's, see mask_lanes (robust, L >= 0)
+    template <class LD>
+    SPX_DEV static uint64_t layer_root(const SetParams &P, const KeccakLane &k, uint32_t lane, const uint8_t *pk,
+                                       uint64_t tree, uint32_t idx_leaf, const uint8_t *auth, const uint64_t *masks,
+                                       int L, LD ld) {
+        uint64_t tree_L = tree;
+        uint32_t idx_L = idx_leaf;
+        Adrs pa;
+        adrs_zero(pa);
+        if (L >= 0) {
+            layer_index(P, tree, idx_leaf, L, tree_L, idx_L);
+            adrs_layer(pa, L);
+        }
+        adrs_tree(pa, tree_L);
+        adrs_keypair(pa, idx_L);
+        adrs_type(pa, L < 0 ? ADDR_FORSPK : ADDR_WOTSPK);
+        if (L < 0) return tl(k, lane, pk, pa, P.k, true, ld);
+        const uint64_t a = tl(k, lane, pk, pa, LEN, false,
+                              [&](uint32_t q) { return HF::kRobust ? ld(q) ^ masks[q] : ld(q); });
+        Adrs ad;
+        adrs_zero(ad);
+        adrs_layer(ad, L);
+        adrs_tree(ad, tree_L);
+        adrs_type(ad, ADDR_HASHTREE);
+        return climb(a, k, lane, pk, P.hp, ad, idx_L, auth, masks + LEN * NL);
+    }
+
+    // checksum of the message in lanes i < NL (chain_lengths, wots.cu:84-166), shifted as its digits are read
+    SPX_DEV static uint32_t checksum(uint64_t a, uint32_t lane) {
+        const uint32_t lo = (uint32_t)a, hi = (uint32_t)(a >> 32);
+        uint32_t s = __dp4a((lo & 0x0f0f0f0fu) + (lo >> 4 & 0x0f0f0f0fu), 0x01010101u, 0u);
+        s = __dp4a((hi & 0x0f0f0f0fu) + (hi >> 4 & 0x0f0f0f0fu), 0x01010101u, s);
+        return (15u * LEN1 - __reduce_add_sync(0xffffffffu, lane < (uint32_t)NL ? s : 0u)) << 4;
+    }
+    // digit c (of this lane's choice; every lane calls this)
+    SPX_DEV static uint32_t digit(uint64_t a, uint32_t csum, uint32_t c) {
+        const uint64_t x = shfl64(a, c < (uint32_t)LEN1 ? c >> 4 : 0u);
+        if (c < (uint32_t)LEN1) return (uint32_t)(x >> (8 * (c >> 1 & 7) + (c & 1 ? 0 : 4))) & 15u;
+        return csum >> (12 - 4 * (c - LEN1)) & 15u;
+    }
+};
+
+// One thread's mask task of a robust SHAKE layer: part 0 squeezes T_len's mask,
+// SHAKE256(PUB_SEED || ADRS_T, len n bytes), part 1 the auth path's, 2n bytes
+// per H; both into out (ShakeGroup::mask_lanes).
+template <class HF>
+SPX_DEV void shake_mask_task(const SetParams &P, const KeyRegs<4 * HF::W> &key, uint64_t tree, uint32_t idx_leaf, int L,
+                             int part, uint64_t *out) {
+    using SG = ShakeGroup<HF>;
+    constexpr int NL = SG::NL, Q = SG::LEN * NL;
+    uint64_t tree_L;
+    uint32_t idx_L;
+    layer_index(P, tree, idx_leaf, L, tree_L, idx_L);
+    Adrs a;
+    adrs_zero(a);
+    adrs_layer(a, L);
+    adrs_tree(a, tree_L);
+    const int n = part == 0 ? (Q + 16) / 17 : P.hp;   // permutations
+    uint64_t A[25];
+#pragma unroll 1
+    for (int b = 0; b < n; b++) {
+        if (part == 1 || b == 0) {
+            if (part == 0) {
+                adrs_type(a, ADDR_WOTSPK);
+                adrs_keypair(a, idx_L);
+            } else {
+                adrs_type(a, ADDR_HASHTREE);
+                adrs_height(a, b + 1);
+                adrs_index(a, idx_L >> (b + 1));
+            }
+            uint64_t al[4];
+            adrs_lanes(a, al);
+#pragma unroll
+            for (int i = 0; i < 25; i++) A[i] = 0;
+#pragma unroll
+            for (int i = 0; i < NL; i++) A[i] = HF::vlane(key.pub, i);
+#pragma unroll
+            for (int i = 0; i < 4; i++) A[NL + i] = al[i];
+            A[SG::PL] = 0x1Full;
+            A[16] ^= 0x8000000000000000ull;
+        }
+        keccak_f1600(A);
+        if (part == 0) {
+#pragma unroll
+            for (int i = 0; i < 17; i++)
+                if (17 * b + i < Q) out[17 * b + i] = A[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 2 * NL; i++) out[Q + b * 2 * NL + i] = A[i];
+        }
+    }
+}
 
 }  // namespace cuspx

@@ -53,6 +53,8 @@ struct VerifyLists {
     uint64_t stride = 0;         // entries per bucket: at least count x len
     uint8_t *cand = nullptr;     // speculative chain ends: cand_items x d x len x 16 x n, or null
     uint32_t cand_items = 0;
+    uint64_t *masks = nullptr;   // robust SHAKE: a layer's masks, count x ShakeGroup::mask_lanes
+    uint64_t *cand_masks = nullptr;   // ... of every layer, cand_items x d x mask_lanes, beside cand
     bool direct = false;         // the batch is launched kernel by kernel (serving), not as a graph
 };
 
@@ -437,17 +439,84 @@ __global__ void __launch_bounds__(128) k_vsort_layer_group(SetParams P, VerifyAr
     }
 }
 
+// The same for SHAKE-256 sets, a warp per item (ShakeGroup); robust: the
+// layer's masks are in V.masks (k_vsort_chains).
+template <class HF>
+__global__ void __launch_bounds__(128) k_vsort_layer_warp(SetParams P, VerifyArgs A, VerifyLists V, int L,
+                                                          uint32_t first, uint32_t n, int grp) {
+    using SG = ShakeGroup<HF>;
+    constexpr int N = SG::N, NL = SG::NL, LEN = SG::LEN, kPer = (LEN + 31) / 32;
+    __shared__ uint32_t hcount[16], hbase[16];
+    if (threadIdx.x < 16) hcount[threadIdx.x] = 0;
+    const uint32_t lane = threadIdx.x & 31, j = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    const bool live = j < n;
+    const uint32_t i = first + (live ? j : 0);   // warps past the end repeat the first item
+    const SignWork &wk = A.work[i];
+    const bool ok = live && !wk.flags;
+    const uint8_t *pkb = A.pk.row(i);
+    KeccakLane k;
+    keccak_lane_init(k, lane);
+    const uint64_t *src = reinterpret_cast<const uint64_t *>(L < 0 ? A.fors_roots + (uint64_t)i * P.k * N
+                                                                  : A.wpk + (uint64_t)i * LEN * N);
+    const uint64_t *masks = HF::kRobust ? V.masks + (uint64_t)i * SG::mask_lanes(P.hp) : nullptr;
+    const uint8_t *auth = A.sig + (uint64_t)i * A.sig_stride + (L < 0 ? 0 : sig_layer_off(P, L) + P.wots_bytes);
+    const uint64_t a = SG::layer_root(P, k, lane, pkb, wk.tree, wk.idx_leaf, auth, masks, L,
+                                      [&](uint32_t q) { return src[q]; });
+    if (L == P.d - 1) {   // uniform over the launch: no barrier follows
+        const bool eq = lane >= (uint32_t)NL || reinterpret_cast<const uint64_t *>(pkb + N)[lane] == a;
+        const bool all = __all_sync(0xffffffffu, eq);
+        if (live && lane == 0) A.verdict[i] = ok && all ? 0 : -1;
+        return;
+    }
+    const uint32_t csum = SG::checksum(a, lane);
+    __syncthreads();
+    uint32_t lr[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        const uint32_t c = lane + 32 * q, dg = SG::digit(a, csum, c < (uint32_t)LEN ? c : 0u);
+        if (ok && c < (uint32_t)LEN) lr[q] = (15u - dg) << 16 | atomicAdd(&hcount[15u - dg], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < 16 && hcount[threadIdx.x])
+        hbase[threadIdx.x] = atomicAdd(&V.cnt[((uint64_t)grp * P.d + L + 1) * 16 + threadIdx.x], hcount[threadIdx.x]);
+    __syncthreads();
+    uint32_t *base = V.tasks + (uint64_t)first * LEN;
+#pragma unroll
+    for (int q = 0; q < kPer; q++) {
+        const uint32_t c = lane + 32 * q;
+        if (ok && c < (uint32_t)LEN) {
+            const uint32_t l = lr[q] >> 16;
+            base[(uint64_t)l * V.stride + hbase[l] + (lr[q] & 0xffffu)] = i << 7 | c;
+        }
+    }
+}
+
 // One lane per chain of layer L, in sorted order (most steps first; the
 // zero-step chains, plain copies, last): sorted position p of the group ->
 // bucket and entry.
+// `mask_blocks` blocks before the chains' take the n items' mask tasks of the
+// layer instead (robust SHAKE with the warp-per-item layer kernel; two threads
+// an item, T_len's masks first): 16 and h' permutations at n = 32, where a
+// chain is up to 30, so they end within the launch.
 template <class HF>
 __global__ void __launch_bounds__(128) k_vsort_chains(SetParams P, VerifyArgs A, VerifyLists V, int L,
-                                                      uint32_t first, int grp) {
+                                                      uint32_t first, int grp, uint32_t n, uint32_t mask_blocks) {
     constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
+    if constexpr (HF::kShake && HF::kRobust) {
+        if (blockIdx.x < mask_blocks) {
+            const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, part = x >= n, i = first + x - part * n;
+            if (x >= 2 * n) return;
+            KeyRegs<N> key;
+            HF::load(key.pub, A.pk.row(i));
+            shake_mask_task<HF>(P, key, A.work[i].tree, A.work[i].idx_leaf, L, (int)part,
+                                V.masks + (uint64_t)i * ShakeGroup<HF>::mask_lanes(P.hp));
+            return;
+        }
+    }
     __shared__ uint32_t cnt[16];
     if (threadIdx.x < 16) cnt[threadIdx.x] = V.cnt[((uint64_t)grp * P.d + L) * 16 + threadIdx.x];
     __syncthreads();
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t p = (blockIdx.x - mask_blocks) * blockDim.x + threadIdx.x;
     int l = 15;
     for (; l >= 0; l--) {
         if (p < cnt[l]) break;
@@ -496,11 +565,23 @@ __global__ void __launch_bounds__(128) k_vsort_chains(SetParams P, VerifyArgs A,
 // thread per (start step, item, layer, chain): start-step-major, so a warp's
 // lanes run equally many steps
 template <class HF>
-__global__ void __launch_bounds__(128) k_vspec_cand(SetParams P, VerifyArgs A, uint8_t *cand) {
+__global__ void __launch_bounds__(128) k_vspec_cand(SetParams P, VerifyArgs A, uint8_t *cand, uint64_t *masks) {
     constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
     const uint64_t per_d = (uint64_t)A.count * P.d * LEN;
     const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= 16 * per_d) return;
+    if (gid >= 16 * per_d) {
+        if constexpr (HF::kShake && HF::kRobust) {
+            // behind the chains: the mask tasks of every item and layer
+            const uint32_t x = (uint32_t)(gid - 16 * per_d), n = A.count * (uint32_t)P.d, part = x >= n;
+            const uint32_t y = x - part * n, i = y / (uint32_t)P.d;
+            if (x >= 2 * n) return;
+            KeyRegs<N> key;
+            HF::load(key.pub, A.pk.row(i));
+            shake_mask_task<HF>(P, key, A.work[i].tree, A.work[i].idx_leaf, (int)(y - i * (uint32_t)P.d), (int)part,
+                                masks + (uint64_t)y * ShakeGroup<HF>::mask_lanes(P.hp));
+        }
+        return;
+    }
     const uint32_t dg = (uint32_t)(gid / per_d);
     const uint64_t r = gid - (uint64_t)dg * per_d;
     const uint32_t item = (uint32_t)(r / ((uint64_t)P.d * LEN));
@@ -530,89 +611,9 @@ __global__ void __launch_bounds__(128) k_vspec_cand(SetParams P, VerifyArgs A, u
     HF::store(cand + ((((uint64_t)item * P.d + L) * LEN + c) * 16 + dg) * N, v);
 }
 
-// thread per item: T_k, then per layer the chain ends picked from the
-// speculative table by the digits of the layer's message, T_len and the
-// auth path (vslot_root); the verdict against PK.root.  Dynamic shared
-// memory: blockDim x VsortSmem<HF>::slot_stride words.
-template <class HF>
-__global__ void __launch_bounds__(32) k_vspec_walk(SetParams P, VerifyArgs A, const uint8_t *cand) {
-    using PV = VerifyPolicy<HF>;
-    using SM = VsortSmem<HF>;
-    constexpr int W = PV::W, N = PV::N, LEN = PV::LEN, NW = N / 8;
-    constexpr int kBatch = 24 / NW;   // chain ends loaded before they are stored (24 8-byte words)
-    extern __shared__ __align__(16) uint32_t smem[];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.count) return;   // no barriers in this kernel
-    const SignWork wk = A.work[i];
-    if (wk.flags) {   // wrong signature length (sign.cu:3063-3065)
-        A.verdict[i] = -1;
-        return;
-    }
-    const uint8_t *pkb = A.pk.row(i);
-    uint32_t *S = smem + threadIdx.x * SM::slot_stride(P.hp);
-    uint32_t *stream = S + PV::S_HDR;
-    uint32_t root[W];
-    {
-        const uint2 *src = reinterpret_cast<const uint2 *>(A.fors_roots + (uint64_t)i * P.k * N);
-        const int vw = P.k * NW;
-        for (int q0 = 0; q0 < vw; q0 += 2 * kBatch) {
-            uint2 x[2 * kBatch];
-#pragma unroll
-            for (int k = 0; k < 2 * kBatch; k++)
-                if (q0 + k < vw) x[k] = src[q0 + k];
-#pragma unroll
-            for (int k = 0; k < 2 * kBatch; k++)
-                if (q0 + k < vw) PV::put_value_word(stream, q0 + k, x[k]);
-        }
-    }
-    vslot_root<HF>(P, S, wk, A.work + i, pkb, -1, P.k, root);
-    const uint8_t *sig = A.sig + (uint64_t)i * A.sig_stride;
-    for (int L = 0; L < P.d; L++) {
-        // the layer's auth path behind the stream
-        const uint32_t *sa = reinterpret_cast<const uint32_t *>(sig + sig_layer_off(P, L) + P.wots_bytes);
-        const int aw = P.hp * W;
-        for (int q0 = 0; q0 < aw; q0 += 2 * kBatch) {
-            uint32_t x[2 * kBatch];
-#pragma unroll
-            for (int k = 0; k < 2 * kBatch; k++)
-                if (q0 + k < aw) x[k] = sa[q0 + k];
-#pragma unroll
-            for (int k = 0; k < 2 * kBatch; k++)
-                if (q0 + k < aw) S[PV::S_HDR + PV::kStreamWords + q0 + k] = x[k];
-        }
-        // chain c's end: its run from start step d_c, d_c digit c of the message
-        const uint32_t csum = vsort_checksum<HF>(root);
-        const uint8_t *cb = cand + ((uint64_t)i * P.d + L) * LEN * 16 * N;
-#pragma unroll
-        for (int c0 = 0; c0 < LEN; c0 += kBatch) {
-            uint2 x[kBatch][NW];
-#pragma unroll
-            for (int j = 0; j < kBatch; j++) {
-                if (c0 + j < LEN) {
-                    const uint32_t dg = 15u - vsort_steps<HF>(root, csum, c0 + j);
-                    const uint2 *src = reinterpret_cast<const uint2 *>(cb + ((uint64_t)(c0 + j) * 16 + dg) * N);
-#pragma unroll
-                    for (int h = 0; h < NW; h++) x[j][h] = src[h];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kBatch; j++)
-                if (c0 + j < LEN) {
-#pragma unroll
-                    for (int h = 0; h < NW; h++) PV::put_value_word(stream, (c0 + j) * NW + h, x[j][h]);
-                }
-        }
-        vslot_root<HF>(P, S, wk, A.work + i, pkb, L, LEN, root);
-    }
-    uint32_t pr[W];
-    HF::load(pr, pkb + N);
-    bool eq = true;
-#pragma unroll
-    for (int x = 0; x < W; x++) eq &= pr[x] == root[x];
-    A.verdict[i] = eq ? 0 : -1;
-}
-
-// The same for SHA-256 sets, a warp per item (spx_vgroup.cuh): a lane that
+// Then a warp per item: T_k, and per layer T_len over the chain ends that the
+// digits of the layer's message pick from the table, and the auth path; the
+// verdict against PK.root.  SHA-256 (spx_vgroup.cuh): a lane that
 // builds a T_len block picks the chain ends it covers.  Dynamic shared
 // memory: ShaGroup<HF>::kWords words.
 template <class HF>
@@ -655,6 +656,50 @@ __global__ void __launch_bounds__(32) k_vspec_walk_group(SetParams P, VerifyArgs
 #pragma unroll
     for (int x = 0; x < W; x++) eq &= pr[x] == root[x];
     if (g == 0) A.verdict[i] = eq ? 0 : -1;
+}
+
+// The same for SHAKE-256 sets, a warp per item (ShakeGroup): a lane that
+// absorbs T_len's lanes picks the chain ends they belong to.
+template <class HF>
+__global__ void __launch_bounds__(32) k_vspec_walk_warp(SetParams P, VerifyArgs A, const uint8_t *cand,
+                                                        const uint64_t *masks) {
+    using SG = ShakeGroup<HF>;
+    constexpr int N = SG::N, NL = SG::NL, LEN = SG::LEN;
+    __shared__ uint64_t msg[4];
+    const uint32_t i = blockIdx.x, lane = threadIdx.x;
+    const SignWork &wk = A.work[i];
+    if (wk.flags) {   // wrong signature length (sign.cu:3063-3065)
+        if (lane == 0) A.verdict[i] = -1;
+        return;
+    }
+    const uint8_t *pkb = A.pk.row(i), *sig = A.sig + (uint64_t)i * A.sig_stride;
+    KeccakLane k;
+    keccak_lane_init(k, lane);
+    const uint64_t tree = wk.tree;
+    const uint32_t idx_leaf = wk.idx_leaf;
+    uint64_t a = 0;
+    uint32_t csum = 0;
+#pragma unroll 1
+    for (int L = -1; L < P.d; L++) {
+        const uint64_t *cb = reinterpret_cast<const uint64_t *>(
+            L < 0 ? A.fors_roots + (uint64_t)i * P.k * N : cand + ((uint64_t)i * P.d + L) * LEN * 16 * N);
+        const uint64_t *mk = HF::kRobust ? masks + ((uint64_t)i * P.d + (L < 0 ? 0 : L)) * SG::mask_lanes(P.hp) : nullptr;
+        a = SG::layer_root(P, k, lane, pkb, tree, idx_leaf, sig + (L < 0 ? 0 : sig_layer_off(P, L) + P.wots_bytes), mk,
+                           L, [&](uint32_t q) {
+                               if (L < 0) return cb[q];
+                               const uint32_t c = q / NL;
+                               const uint32_t dg = c < (uint32_t)SG::LEN1
+                                                       ? (uint32_t)(msg[c >> 4] >> (8 * (c >> 1 & 7) + (c & 1 ? 0 : 4))) & 15u
+                                                       : csum >> (12 - 4 * (c - SG::LEN1)) & 15u;
+                               return cb[(c * 16 + dg) * NL + q % NL];
+                           });
+        csum = SG::checksum(a, lane);
+        if (lane < (uint32_t)NL) msg[lane] = a;
+        __syncwarp();
+    }
+    const bool eq = lane >= (uint32_t)NL || reinterpret_cast<const uint64_t *>(pkb + N)[lane] == a;
+    const bool all = __all_sync(0xffffffffu, eq);
+    if (lane == 0) A.verdict[i] = all ? 0 : -1;
 }
 
 }  // namespace cuspx

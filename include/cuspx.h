@@ -68,8 +68,9 @@ typedef struct {
     int tree_warps;       /* warps per block, XMSS tree kernel */
     int chains_per_warp;  /* (item, chain) tasks per warp, verify chain kernel */
     int verify_mode;      /* 0 layered verify kernels, 1 one thread per item over all layers,
-                             2 one launch over the whole hypertree (default; SHA-256 batches of
-                             more than 4 items an SM as mode 3 unless verify_sorted_min is 0),
+                             2 one launch over the whole hypertree (default; unless
+                             verify_sorted_min is 0, SHA-256 batches of more than 4 items an SM
+                             and SHAKE ones as mode 3),
                              3 layered kernels with each layer's WOTS+ chains sorted by length */
     int fors_lanes_log2;  /* lanes per FORS tree = 2^g, g in 0..5 (0: lane per tree, 5: warp per tree) */
     int tree_mode;        /* 0 warp per XMSS subtree, 1 lane per subtree (heights <= 4 only) */
@@ -87,9 +88,8 @@ typedef struct {
                              at once) */
     int verify_groups;    /* sorted verify: the batch is split into this many groups of items
                              (1..8), each on its own stream, so that one group's serial T_len
-                             and auth-path kernel overlaps another group's chains (SHA-256
-                             batches of up to 2048 items, 4096 robust, run as one group whose
-                             layer kernel has 8 lanes an item) */
+                             and auth-path kernel overlaps another group's chains (one group for
+                             SHA-256 up to 2048 items, 4096 robust, and SHAKE up to 4 an SM) */
     int verify_sorted_min;/* verify batches of at least this many items run the sorted layered
                              verify whatever verify_mode says (0: only with verify_mode 3);
                              batches up to verify_item_max still run one item per block */

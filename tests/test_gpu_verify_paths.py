@@ -1,8 +1,7 @@
-"""SHA-256 verify batches through the sorted layers, the fused blocks and the
-speculative walk, by groups of lanes and by a thread per item, at the sizes
-where a block, a warp or an item group is part full: good signatures pass, a
-signature with one byte changed anywhere is rejected, and its neighbours are
-not disturbed.
+"""Verify batches through the sorted layers, the fused blocks and the speculative
+walk, by groups of lanes, a warp and a thread per item, at the sizes where a block, a warp or
+an item group is part full: good signatures pass, a signature with one byte
+changed anywhere is rejected, and its neighbours are not disturbed.
 """
 import random
 
@@ -10,7 +9,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SETS = ["sha256-%s-%s" % (s, m) for s in ("128s", "128f", "192s", "192f", "256s", "256f") for m in ("simple", "robust")]
+SETS = ["%s-%s-%s" % (h, s, m) for h in ("sha256", "shake256") for s in ("128s", "128f", "192s", "192f", "256s", "256f")
+        for m in ("simple", "robust")]
 
 
 @pytest.fixture(scope="module")
