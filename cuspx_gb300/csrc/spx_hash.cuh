@@ -238,14 +238,20 @@ SPX_DEV void sha256_schedule_kw(uint32_t *kw, uint32_t w[16]) {
 }
 
 // s <- compress(s) with the schedule given as kw[t * S] = W_t + K_t (the
-// rounds alone: the schedule was computed elsewhere)
+// rounds alone: the schedule was computed elsewhere), unrolled: for a warp
+// that hashes one message's blocks in succession (1 MiB: 31.6 ms a signature
+// with the last adds of a' on the FMA pipe, 32.4 as an IADD3, 32.2 to 37.4
+// with h + K + W made a round ahead or t1 on the FMA pipe).
 template <int S>
 SPX_DEV void sha256_compress_kw(uint32_t s[8], const uint32_t *kw) {
     uint32_t a = s[0], b = s[1], c = s[2], d = s[3], e = s[4], f = s[5], g = s[6], h = s[7];
 #pragma unroll
     for (int i = 0; i < 64; i++) {
-        const uint32_t t1 = add_fma(h, kw[i * S]) + sha_Sigma1(e) + ((e & f) ^ (~e & g));
-        const uint32_t t2 = sha_Sigma0(a) + ((a & b) | (c & (a | b)));
+        const uint32_t hk = add_fma(h, kw[i * S]);
+        const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
+        const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
+        const uint32_t t1 = hk + S1 + ch;
+        const uint32_t na = add_fma(add_fma(S0, mj), t1);
         h = g;
         g = f;
         f = e;
@@ -253,7 +259,7 @@ SPX_DEV void sha256_compress_kw(uint32_t s[8], const uint32_t *kw) {
         d = c;
         c = b;
         b = a;
-        a = t1 + t2;
+        a = na;
     }
     s[0] += a; s[1] += b; s[2] += c; s[3] += d; s[4] += e; s[5] += f; s[6] += g; s[7] += h;
 }

@@ -276,7 +276,7 @@ __global__ void k_sign_msg(SetParams P, SignArgs A, uint64_t long_msg) {
 template <class HF>
 __global__ void __launch_bounds__(64) k_sign_msg_pair(SetParams P, SignArgs A, uint64_t long_msg) {
     constexpr int W = HF::W, N = 4 * W;
-    __shared__ uint32_t kw[2 * 64 * 32];
+    __shared__ uint32_t kw[HF::kPairWords];
     __shared__ uint32_t xr[8 * 32];
     const uint32_t l = threadIdx.x & 31;
     const uint32_t i = blockIdx.x * 32 + l;
@@ -1090,7 +1090,7 @@ __global__ void k_verify_msg(SetParams P, VerifyArgs A, uint64_t long_msg) {
 template <class HF>
 __global__ void __launch_bounds__(64) k_verify_msg_pair(SetParams P, VerifyArgs A, uint64_t long_msg) {
     constexpr int W = HF::W, N = 4 * W;
-    __shared__ uint32_t kw[2 * 64 * 32];
+    __shared__ uint32_t kw[HF::kPairWords];
     const uint32_t l = threadIdx.x & 31;
     const uint32_t i = blockIdx.x * 32 + l;
     const uint64_t mlen = i < A.count ? A.msg.len[i] : 0;

@@ -629,13 +629,15 @@ struct Sha2 {
     // by its own instruction issue, about 1.3k ALU instructions per block.
     // For message l, lane l of warp 0 (role 0) builds each block and its
     // schedule with the round constants added into kw, and lane l of warp 1
-    // (role 1) runs the 64 rounds from kw a block behind; one __syncthreads
-    // per block hands a buffer over.  kw is a shared 2 x 64 x 32-word double
-    // buffer with the 32 messages interleaved (kw[(buf * 64 + t) * 32 + l]).
+    // (role 1) runs the 64 rounds from kw two blocks behind; one __syncthreads
+    // hands two blocks over (one at a time: 3% slower).  kw is a shared double buffer of kPairBlocks
+    // blocks x 64 words with the 32 messages interleaved (word t of buffer q
+    // at kw[(q * 64 + t) * 32 + l]).
     // Every thread of the block calls this; max_blocks (the same for the
     // whole block) bounds the loop, and threads whose message has fewer
     // blocks, or role 2, only take part in the barriers.  The result is in
     // role 1's st.
+    static constexpr int kPairBlocks = 2, kPairWords = 2 * kPairBlocks * 64 * 32;
     template <int P>
     SPX_DEV static void stream_msg_pair(uint32_t st[8], uint32_t pre_blocks, const uint32_t pre[P],
                                         const uint8_t *m, uint64_t mlen, uint32_t *kw, int role,
@@ -646,13 +648,18 @@ struct Sha2 {
         uint32_t *mine = kw + (threadIdx.x & 31);
         uint32_t nxt[16];
         bool have = false;
-        for (uint64_t b = 0; b <= max_blocks; b++) {
-            if (role == 0 && b < nblocks) {
-                uint32_t w[16];
-                next_block<P>(w, b, nblocks, bits, pre, m, mlen, nxt, have);
-                sha256_schedule_kw<32>(mine + 64 * 32 * (b & 1), w);
+        for (uint64_t q = 0; q <= (max_blocks + kPairBlocks - 1) / kPairBlocks; q++) {
+#pragma unroll 1
+            for (int u = 0; u < kPairBlocks; u++) {
+                const uint64_t b = q * kPairBlocks + u;   // role 1's block is kPairBlocks earlier
+                if (role == 0 && b < nblocks) {
+                    uint32_t w[16];
+                    next_block<P>(w, b, nblocks, bits, pre, m, mlen, nxt, have);
+                    sha256_schedule_kw<32>(mine + 64 * 32 * ((q & 1) * kPairBlocks + u), w);
+                }
+                if (role == 1 && q > 0 && b - kPairBlocks < nblocks)
+                    sha256_compress_kw<32>(st, mine + 64 * 32 * ((~q & 1) * kPairBlocks + u));
             }
-            if (role == 1 && b >= 1 && b <= nblocks) sha256_compress_kw<32>(st, mine + 64 * 32 * ((b - 1) & 1));
             __syncthreads();
         }
     }
