@@ -263,6 +263,34 @@ SPX_DEV void sha256_compress_kw(uint32_t s[8], const uint32_t *kw) {
     }
     s[0] += a; s[1] += b; s[2] += c; s[3] += d; s[4] += e; s[5] += f; s[6] += g; s[7] += h;
 }
+// The same sixteen rounds at a time, 4 KB of code, with h + K + W made a round
+// early: for kernels that run other compressions beside it.
+template <int S>
+SPX_DEV void sha256_compress_kw16(uint32_t s[8], const uint32_t *kw) {
+    uint32_t a = s[0], b = s[1], c = s[2], d = s[3], e = s[4], f = s[5], g = s[6], h = s[7];
+    uint32_t hk = add_fma(h, kw[0]);
+#pragma unroll 1
+    for (int r = 0; r < 64; r += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const uint32_t nx = add_fma(g, kw[((r + i + 1) & 63) * S]);
+            const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
+            const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
+            const uint32_t t1 = hk + S1 + ch;
+            const uint32_t na = add_fma(add_fma(S0, mj), t1);
+            hk = nx;
+            h = g;
+            g = f;
+            f = e;
+            e = add_fma(d, t1);
+            d = c;
+            c = b;
+            b = a;
+            a = na;
+        }
+    }
+    s[0] += a; s[1] += b; s[2] += c; s[3] += d; s[4] += e; s[5] += f; s[6] += g; s[7] += h;
+}
 
 // s <- compress(s, w); w is consumed (overwritten by the schedule).
 template <bool AF>

@@ -14,11 +14,12 @@
 //                                        g shuffle levels, auth path, root
 //   k_fors_top      block / FORS tree    the levels above 2^g > 32 lanes
 //   k_leaf_chains   thread / WOTS+ chain PRF and 15 F; the signing leaf records its chains
-//   k_leaf_tstream  thread / XMSS leaf   T_len over the chain ends (k_leaf_tlen in small
-//                                        batches; k_leaves: both per leaf, without scratch)
+//   k_leaf_tstream  thread / XMSS leaf   T_len over the chain ends (small batches:
+//                                        k_leaf_tlen, lanes / leaf, spx_vgroup.cuh;
+//                                        k_leaves: both per leaf, without scratch)
 //   k_trees         warp / XMSS tree     level-by-level reduction in shared memory,
 //                                        auth path, root (k_trees_lane: lane / tree)
-//   k_fors_pk       thread / signature   FORS pk (T_k)
+//   k_fors_pk       lanes / signature    FORS pk (T_k, spx_vgroup.cuh)
 //   k_sign_finish   block / signature    WOTS signatures gathered from the recorded
 //                                        chains
 //
@@ -738,14 +739,6 @@ __global__ void __launch_bounds__(128) k_leaf_chains(SetParams P, LeafArgs A) {
     HF::store(chain_end<N>(A, x, c), v);
 }
 
-// T_l of m n-byte values in global memory under ADRS pa into out, by one
-// thread over a slot of `VsortSmem<HF>::slot_stride(0)` shared words
-// (spx_vsort.cuh): the values staged with their loads in flight together,
-// then the hash unit by unit through one call site.
-template <class HF>
-SPX_DEV void slot_tl(uint32_t *S, const KeyRegs<4 * HF::W> &key, const uint8_t *pub, const Adrs &pa,
-                     const uint8_t *vals, int m, uint32_t out[HF::W]);
-
 // key, address and output of a T_len thread: the launch's leaf x
 // (null: there is none)
 template <class HF>
@@ -772,23 +765,6 @@ SPX_DEV const uint8_t *tlen_pos(const SetParams &P, const LeafArgs &A, uint32_t 
     adrs_keypair(pa, j);
     leaf = A.leaves + ((((uint64_t)item * A.nlayers + (L - A.layer0)) << P.hp) + j) * N;
     return sk;
-}
-
-// thread per leaf, small sign batches, where the thread's serial latency is
-// what counts: T_len through a slot of slot_words shared words (slot_tl)
-template <class HF>
-__global__ void k_leaf_tlen(SetParams P, LeafArgs A, uint32_t slot_words) {
-    constexpr int W = HF::W, N = 4 * W, LEN = 2 * N + 3;
-    extern __shared__ uint32_t smem[];
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    KeyRegs<N> key;
-    Adrs pa;
-    uint8_t *to;
-    const uint8_t *sk = tlen_pos<HF>(P, A, x, key, pa, to);
-    if (!sk) return;
-    uint32_t leaf[W];
-    slot_tl<HF>(smem + threadIdx.x * slot_words, key, sk + 2 * N, pa, chain_end<N>(A, x, 0), LEN, leaf);
-    HF::store(to, leaf);
 }
 
 // thread per leaf, large batches: T_len over the interleaved ends, block by
@@ -971,33 +947,6 @@ __global__ void k_trees(SetParams P, TreeArgs A) {
         for (int x = 0; x < W; x++) v[x] = nodes[base * W + x];
         HF::store(A.roots + ((uint64_t)item * A.nlayers + (L - A.layer0)) * N, v);
     }
-}
-
-// ===========================================================================
-// FORS public key: thread per signature, T_k over its FORS roots (fors.cu:
-// 141-142) through a verify slot (slot_tl), in place of the first root.  Runs
-// behind k_fors_sign, beside the hypertree: one signature at 128f spends
-// ~20 us here that k_sign_finish added behind the trees before.
-// ===========================================================================
-template <class HF>
-__global__ void __launch_bounds__(32) k_fors_pk(SetParams P, SignArgs A, uint32_t slot_words) {
-    constexpr int W = HF::W, N = 4 * W;
-    extern __shared__ uint32_t smem[];
-    const uint32_t item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= A.count) return;
-    const SignWork &wk = A.work[item];
-    const uint8_t *sk = A.sk.row(item);
-    KeyRegs<N> key;
-    key_from_work<HF>(key, sk, sk + 2 * N, wk);
-    Adrs pa;
-    adrs_zero(pa);
-    adrs_tree(pa, wk.tree);
-    adrs_keypair(pa, wk.idx_leaf);
-    adrs_type(pa, ADDR_FORSPK);
-    uint32_t o[W];
-    uint8_t *roots = A.fors_roots + (uint64_t)item * P.k * N;
-    slot_tl<HF>(smem + threadIdx.x * slot_words, key, sk + 2 * N, pa, roots, P.k, o);
-    HF::store(roots, o);
 }
 
 // ===========================================================================

@@ -152,6 +152,7 @@ __global__ void k_keygen_finish(KeygenArgs A) {
 template <class HF>
 struct Family {
     static constexpr int W = HF::W, N = 4 * W;
+    using TL = TlLanes<HF>;
 
     static cudaError_t configure() {
         cudaError_t e;
@@ -275,11 +276,13 @@ struct Family {
         k_trees<HF><<<ceil_div(warps, wpb), 32 * wpb, per_warp * wpb, s>>>(P, T);
     }
 
-    // XMSS leaves.  With chain-end scratch: a thread per chain, then a thread
-    // per leaf, in chunks of as many trees as the scratch holds; `latency`
-    // picks the T_len kernel of small sign batches (128f, one signature: 25
-    // against 41 us; 37: 25 against 43 us), whose shared slots keep one warp an
-    // SM, while large ones run the streaming one with every warp resident.
+    // XMSS leaves.  With chain-end scratch: a thread per chain, then T_len, in
+    // chunks of as many trees as the scratch holds.  Small sign batches
+    // (`latency`) take several lanes a leaf for T_len up to two warps a
+    // scheduler (128f, one signature 18 us, a thread a leaf 23 us; 37
+    // signatures 35 / 23 us), larger ones the streaming kernel, whose threads
+    // repeat nothing; robust SHA-256, whose lanes share out the mask blocks
+    // too, takes them in every small batch (256f-robust, 37: 0.36 / 0.94 ms).
     // Without scratch (ends_trees 0): a thread per leaf (k_leaves).
     static void leaves(const SetParams &P, LeafArgs L, const Tuning &tu, cudaStream_t s, PhaseTimer *pt,
                        uint32_t ends_trees, bool latency) {
@@ -291,6 +294,7 @@ struct Family {
             return;
         }
         constexpr int LEN = 2 * N + 3;
+        if (HF::kShake || !HF::kRobust) latency = latency && (trees << P.hp) * TL::kLanes <= 256ull * device_sms();
         L.interleaved = !latency;
         for (uint64_t t = 0; t < trees; t += ends_trees) {
             L.tree0 = (uint32_t)t;
@@ -298,9 +302,8 @@ struct Family {
             const uint64_t nl = (uint64_t)L.trees << P.hp;
             k_leaf_chains<HF><<<ceil_div(nl * LEN, 128), 128, 0, s>>>(P, L);
             CUSPX_MARK(pt, "k_leaf_chains", s);
-            if (latency) {   // 32 threads per block, each with a slot of 1-5 KB
-                const uint32_t sw = VsortSmem<HF>::slot_stride(0);
-                k_leaf_tlen<HF><<<ceil_div(nl, 32), 32, (size_t)32 * sw * 4, s>>>(P, L, sw);
+            if (latency) {
+                k_leaf_tlen<HF><<<ceil_div(nl, TL::kPerBlock), TL::kThreads, TL::smem(), s>>>(P, L);
                 CUSPX_MARK(pt, "k_leaf_tlen", s);
             } else {
                 k_leaf_tstream<HF><<<ceil_div(nl, 128), 128, 0, s>>>(P, L);
@@ -376,8 +379,7 @@ struct Family {
                 k_fors_top<HF><<<(unsigned)trees, tb, (size_t)W * 4 << g, sf>>>(P, A, g);
                 CUSPX_MARK(pt, "k_fors_top", s);
             }
-            const uint32_t sw = VsortSmem<HF>::slot_stride(0);
-            k_fors_pk<HF><<<ceil_div(A.count, 32), 32, (size_t)32 * sw * 4, sf>>>(P, A, sw);
+            k_fors_pk<HF><<<ceil_div(A.count, TL::kPerBlock), TL::kThreads, TL::smem(), sf>>>(P, A);
             CUSPX_MARK(pt, "k_fors_pk", s);
         }
         if (split) cudaEventRecord(fk->join, sf);

@@ -29,33 +29,6 @@ struct ShaGroup {
     // a stride of 4 mod 32 keeps the groups of a warp in different banks
     static constexpr int kStride = kWords + (36 - kWords % 32) % 32;
 
-    // rounds of one block from kw (stride NBP): h + K + W is ready a round early
-    SPX_DEV static void rounds(uint32_t st[8], const uint32_t *kw) {
-        uint32_t a = st[0], b = st[1], c = st[2], d = st[3], e = st[4], f = st[5], g = st[6], h = st[7];
-        uint32_t hk = add_fma(h, kw[0]);
-#pragma unroll 1
-        for (int r = 0; r < 64; r += 16) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const uint32_t nx = add_fma(g, kw[((r + i + 1) & 63) * NBP]);
-                const uint32_t S1 = sha_Sigma1(e), ch = (e & f) ^ (~e & g);
-                const uint32_t S0 = sha_Sigma0(a), mj = (a & b) | (c & (a | b));
-                const uint32_t t1 = hk + S1 + ch;
-                const uint32_t na = add_fma(add_fma(S0, mj), t1);
-                hk = nx;
-                h = g;
-                g = f;
-                f = e;
-                e = add_fma(d, t1);
-                d = c;
-                c = b;
-                b = a;
-                a = na;
-            }
-        }
-        st[0] += a; st[1] += b; st[2] += c; st[3] += d; st[4] += e; st[5] += f; st[6] += g; st[7] += h;
-    }
-
     // s <- compress(s, w) with each round's h + K + W made a round early and
     // the schedule a round ahead of its use: for a warp alone on its SM (the
     // walk of one 128f item 0.445 -> 0.432 ms against sha256_compress)
@@ -134,7 +107,10 @@ struct ShaGroup {
 #pragma unroll
         for (int i = 0; i < 8; i++) st[i] = key.mid[i];
 #pragma unroll 1
-        for (int j = 0; j < nb; j++) rounds(st, S + j);
+        for (int j = 0; j < nb; j++) {
+            if constexpr (HF::kRobust) sha256_compress_kw16<NBP>(st, S + j);   // beside mask blocks
+            else sha256_compress_kw<NBP>(st, S + j);
+        }
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < W; i++) out[i] = st[i];
@@ -416,6 +392,81 @@ SPX_DEV void shake_mask_task(const SetParams &P, const KeyRegs<4 * HF::W> &key, 
             for (int i = 0; i < 2 * NL; i++) out[Q + b * 2 * NL + i] = A[i];
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Signing: T_len of a small batch's leaves and T_k, whose latency the
+// signature waits for, by the same lanes (8 a value sequence for SHA-256, a
+// warp for SHAKE-256).  One signature, against one thread a sequence: T_len
+// 23 -> 16 us at 128f, 352 -> 85 us at 256f-robust, 100 -> 60 us at SHAKE-256f.
+// ---------------------------------------------------------------------------
+template <class HF>
+struct TlLanes {
+    static constexpr int kLanes = HF::kShake ? 32 : 8, kThreads = HF::kShake ? 128 : 32;
+    static constexpr int kPerBlock = kThreads / kLanes;
+    // dynamic shared memory of a block
+    static constexpr size_t smem() {
+        if constexpr (HF::kShake) return 0;
+        else return (size_t)kPerBlock * ShaGroup<HF>::kStride * 4;
+    }
+    // out <- T_l of m values at vals under pa (pub: PUB_SEED in memory); every
+    // thread of the block calls this, `live` ones store
+    SPX_DEV static void run(uint8_t *out, bool live, const KeyRegs<4 * HF::W> &key, const uint8_t *pub, const Adrs &pa,
+                            int m, const uint8_t *vals) {
+        extern __shared__ __align__(16) uint32_t smem[];
+        const uint32_t lane = threadIdx.x % kLanes;
+        if constexpr (HF::kShake) {
+            using SG = ShakeGroup<HF>;
+            if (!live) return;   // uniform over the warp
+            KeccakLane k;
+            keccak_lane_init(k, lane);
+            const uint64_t a = SG::tl(k, lane, pub, pa, m, true, [&](uint32_t q) {
+                return reinterpret_cast<const uint64_t *>(vals)[q];
+            });
+            if (lane < (uint32_t)SG::NL) reinterpret_cast<uint64_t *>(out)[lane] = a;
+        } else {
+            using SG = ShaGroup<HF>;
+            uint32_t v[HF::W];
+            SG::template tl<kLanes>(v, smem + threadIdx.x / kLanes * SG::kStride, lane, key, pa, m, true,
+                                    [&](uint32_t q) { return reinterpret_cast<const uint2 *>(vals)[q]; });
+            if (live && lane == 0) HF::store(out, v);
+        }
+    }
+};
+
+// T_len over a leaf's chain ends, in succession (chain_end)
+template <class HF>
+__global__ void __launch_bounds__(TlLanes<HF>::kThreads) k_leaf_tlen(SetParams P, LeafArgs A) {
+    constexpr int N = 4 * HF::W, LEN = 2 * N + 3;
+    const uint32_t x0 = (blockIdx.x * blockDim.x + threadIdx.x) / TlLanes<HF>::kLanes;
+    const bool live = x0 >> P.hp < A.trees;
+    const uint32_t x = live ? x0 : 0;
+    KeyRegs<N> key;
+    Adrs pa;
+    uint8_t *to;
+    const uint8_t *sk = tlen_pos<HF>(P, A, x, key, pa, to);
+    TlLanes<HF>::run(to, live, key, sk + 2 * N, pa, LEN, chain_end<N>(A, x, 0));
+}
+
+// T_k over a signature's FORS roots (fors.cu:141-142), in place of the first
+// root.  Runs behind k_fors_sign, beside the hypertree.
+template <class HF>
+__global__ void __launch_bounds__(TlLanes<HF>::kThreads) k_fors_pk(SetParams P, SignArgs A) {
+    constexpr int N = 4 * HF::W;
+    const uint32_t i0 = (blockIdx.x * blockDim.x + threadIdx.x) / TlLanes<HF>::kLanes;
+    const bool live = i0 < A.count;
+    const uint32_t item = live ? i0 : A.count - 1;
+    const SignWork &wk = A.work[item];
+    const uint8_t *sk = A.sk.row(item);
+    KeyRegs<N> key;
+    key_from_work<HF>(key, sk, sk + 2 * N, wk);
+    Adrs pa;
+    adrs_zero(pa);
+    adrs_tree(pa, wk.tree);
+    adrs_keypair(pa, wk.idx_leaf);
+    adrs_type(pa, ADDR_FORSPK);
+    uint8_t *roots = A.fors_roots + (uint64_t)item * P.k * N;
+    TlLanes<HF>::run(roots, live, key, sk + 2 * N, pa, P.k, roots);
 }
 
 }  // namespace cuspx
