@@ -142,45 +142,49 @@ struct Sha2 {
 #pragma unroll
         for (int i = 0; i < 16; i++) w[i] = NB == 1 || b == 0 ? m[i] : m[16 * (NB - 1) + i];
     }
-    // compression `part` of MGF1-SHA256(PUB_SEED || ADRS_c, .) block `ctr`
-    // (sha256.cu:362-383), from the IV
-    SPX_DEV static void mask_words(uint32_t w[16], const uint32_t pub[W], const Adrs &a, uint32_t ctr, int part) {
+    // first block of MGF1-SHA256(PUB_SEED || ADRS_c, .) block `ctr` (sha256.cu:
+    // 362-383), from the IV; at n = 32 the length block follows (pad_block)
+    SPX_DEV static void mask_words(uint32_t w[16], const uint32_t pub[W], const Adrs &a, uint32_t ctr) {
         constexpr int TOT = N + 26;
-        if (kMaskUnits == 1 || part == 0) {
 #pragma unroll
-            for (int i = 0; i < W; i++) w[i] = pub[i];
+        for (int i = 0; i < W; i++) w[i] = pub[i];
 #pragma unroll
-            for (int i = 0; i < 5; i++) w[W + i] = a.w[i];
-            w[W + 5] = (a.w[5] & 0xffff0000u) | (ctr >> 16);
-            w[W + 6] = (ctr << 16) | 0x8000u;
+        for (int i = 0; i < 5; i++) w[W + i] = a.w[i];
+        w[W + 5] = (a.w[5] & 0xffff0000u) | (ctr >> 16);
+        w[W + 6] = (ctr << 16) | 0x8000u;
 #pragma unroll
-            for (int i = W + 7; i < 16; i++) w[i] = 0;
-            if (kMaskUnits == 1) w[15] = TOT * 8;
-        } else {
+        for (int i = W + 7; i < 16; i++) w[i] = 0;
+        if (kMaskUnits == 1) w[15] = TOT * 8;
+    }
+    SPX_DEV static void pad_block(uint32_t st[8]) {
+        uint32_t t[8];
 #pragma unroll
-            for (int i = 0; i < 15; i++) w[i] = 0;
-            w[15] = TOT * 8;
-        }
+        for (int i = 0; i < 8; i++) t[i] = st[i];
+        sha256_rounds_pad<kFmaA>(t, c_mask_pad);
+#pragma unroll
+        for (int i = 0; i < 8; i++) st[i] += t[i];
     }
     SPX_DEV static void mask_block(uint32_t out[8], const uint32_t pub[W], const Adrs &a, uint32_t ctr) {
+        uint32_t w[16];
+        mask_words(w, pub, a, ctr);
         sha256_iv(out);
-#pragma unroll 1
-        for (int part = 0; part < kMaskUnits; part++) {
-            uint32_t w[16];
-            mask_words(w, pub, a, ctr, part);
-            sha256_compress<kFmaA>(out, w);
-        }
+        sha256_compress<kFmaA>(out, w);
+        if (kMaskUnits == 2) pad_block(out);
     }
-    // block words w and start state st of unit u of thash over in (st holds
-    // the unit before's result where the unit continues it), ...
+    // unit u of thash over in is the length block of a bitmask
+    template <int L>
+    SPX_DEV static bool pad_unit(int u) {
+        return ROBUST && kMaskUnits == 2 && u < kMaskAll<L> && u % 2 == 1;
+    }
+    // block words w and start state st of any other unit (st holds the unit
+    // before's result where the unit continues it), ...
     template <int L>
     SPX_DEV static void unit_block(uint32_t w[16], uint32_t st[8], const KeyRegs<N> &k, const Adrs &a,
                                    const uint32_t in[L], int u) {
         constexpr int MU = kMaskAll<L>;
         if (ROBUST && u < MU) {
-            const int part = u % kMaskUnits;
-            if (part == 0) sha256_iv(st);
-            mask_words(w, k.pub, a, (uint32_t)(u / kMaskUnits), part);
+            sha256_iv(st);
+            mask_words(w, k.pub, a, (uint32_t)(u / kMaskUnits));
         } else {
             if (u == MU) {
 #pragma unroll
@@ -209,9 +213,13 @@ struct Sha2 {
         for (int i = 0; i < 8; i++) st[i] = k.mid[i];
 #pragma unroll 1
         for (int u = 0; u < kUnits<L>; u++) {
-            uint32_t w[16];
-            unit_block<L>(w, st, k, a, in, u);
-            sha256_compress<kFmaA>(st, w);
+            if (pad_unit<L>(u)) {
+                pad_block(st);
+            } else {
+                uint32_t w[16];
+                unit_block<L>(w, st, k, a, in, u);
+                sha256_compress<kFmaA>(st, w);
+            }
             unit_done<L>(st, in, u);
         }
 #pragma unroll
@@ -288,13 +296,7 @@ struct Sha2 {
             sha256_rounds<W + 5, 64, kFmaA>(t, mw);
 #pragma unroll
             for (int i = 0; i < 8; i++) ms[i] = t[i] + sha256_iv_word(i);
-            if (NB == 2) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) t[i] = ms[i];
-                sha256_rounds_pad<kFmaA>(t, c_mask_pad);
-#pragma unroll
-                for (int i = 0; i < 8; i++) ms[i] += t[i];
-            }
+            if (NB == 2) pad_block(ms);
 #pragma unroll
             for (int i = 0; i < W; i++) x[i] ^= ms[i];
         }
@@ -353,16 +355,20 @@ struct Sha2 {
         adrs_index(ad, off + j0);
 #pragma unroll 1
         for (;;) {
-            uint32_t w[16];
-            if (hgt < 0) {
-                prf_words(w, ad, k);
-                sha256_iv(st);
-            } else if (hgt == 0) {
-                unit_block<W>(w, st, k, ad, x, u);
+            if ((hgt == 0 && pad_unit<W>(u)) || (hgt > 0 && pad_unit<2 * W>(u))) {
+                pad_block(st);
             } else {
-                unit_block<2 * W>(w, st, k, ad, x, u);
+                uint32_t w[16];
+                if (hgt < 0) {
+                    prf_words(w, ad, k);
+                    sha256_iv(st);
+                } else if (hgt == 0) {
+                    unit_block<W>(w, st, k, ad, x, u);
+                } else {
+                    unit_block<2 * W>(w, st, k, ad, x, u);
+                }
+                sha256_compress<kFmaA>(st, w);
             }
-            sha256_compress<kFmaA>(st, w);
             if (hgt < 0) {
 #pragma unroll
                 for (int i = 0; i < W; i++) x[i] = st[i];
