@@ -172,6 +172,12 @@ struct cuspx_batch {
     ShareArgs share;
     size_t count = 0;
     bool use_keyrow = false, use_aux = false, use_siglen = false;
+    // One-shot calls: the inputs arrive in one copy (upload_packed), at
+    // offsets that the item count and the use_ flags decide, and a sign
+    // batch's statuses lie behind its signatures.  Null after cuspx_batch_upload.
+    const uint8_t *packed = nullptr;
+    uint8_t *packed_buf = nullptr;
+    size_t packed_cap = 0;
     const uint8_t *bound_keys = nullptr;   // external device key table (not owned)
     size_t bound_nkeys = 0;
     // captured launch sequences keyed by everything baked into them; an item
@@ -180,11 +186,11 @@ struct cuspx_batch {
     struct GraphKey {
         size_t count;
         bool keyrow, aux, siglen, long_msgs;
-        const uint8_t *keys;
+        const uint8_t *keys, *packed;
         Tuning tune;
         bool operator==(const GraphKey &o) const {
             return count == o.count && keyrow == o.keyrow && aux == o.aux && siglen == o.siglen &&
-                   long_msgs == o.long_msgs && keys == o.keys && memcmp(&tune, &o.tune, sizeof(Tuning)) == 0;
+                   long_msgs == o.long_msgs && keys == o.keys && packed == o.packed && memcmp(&tune, &o.tune, sizeof(Tuning)) == 0;
         }
     };
     struct GraphEntry {
@@ -695,7 +701,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
         A((void **)&b->fors_roots, cap * P.k * n);
         if (op == CUSPX_OP_SIGN) {
             A((void **)&b->aux, cap * n);
-            A((void **)&b->out, cap * P.sig_bytes);
+            A((void **)&b->out, cap * (P.sig_bytes + sizeof(int32_t)));   // + statuses, see packed
             A((void **)&b->leaves, cap * P.d * ((size_t)1 << P.hp) * n);
             A((void **)&b->roots, cap * P.d * n);
             A((void **)&b->chains, cap * P.d * P.len * 16 * n);
@@ -775,6 +781,7 @@ int cuspx_batch_upload(cuspx_batch *b, size_t count, const uint8_t *keys, size_t
     const bool bound = b->bound_keys != nullptr && b->op != CUSPX_OP_KEYGEN;
     if (count && !keys && !bound) return fail(ctx, CUSPX_EINVAL, "upload: keys is null");
     CK(cudaSetDevice(ctx->device), ctx);
+    b->packed = nullptr;
     if (b->op == CUSPX_OP_KEYGEN) {
         // seeds (count x 3n) into the first 3n bytes of each sk row
         if (count) CK(cudaMemcpy2DAsync(b->keys, 4 * n, keys, 3 * n, 3 * n, count, cudaMemcpyHostToDevice, b->s), ctx);
@@ -827,25 +834,68 @@ int cuspx_batch_upload(cuspx_batch *b, size_t count, const uint8_t *keys, size_t
 #define CUSPX_SIGN_FORK 1
 #endif
 
+// Offsets of a packed input (upload_packed) of `count` items of a batch: every
+// part but the messages has a size that the count decides, so they come last.
+struct Packed {
+    size_t keys, off, len, opt, siglen, sigs, msgs;
+    Packed(const cuspx_batch *b, size_t count, bool opt_, bool siglen_) {
+        const SetParams &P = b->P;
+        const bool sign = b->op == CUSPX_OP_SIGN;
+        size_t at = 0;
+        auto take = [&](size_t bytes) {
+            const size_t o = at;
+            at += (bytes + 15) & ~(size_t)15;
+            return o;
+        };
+        keys = take(count * (sign ? P.sk_bytes : P.pk_bytes));
+        off = take(count * 8);
+        len = take(count * 8);
+        opt = take(opt_ ? count * P.n : 0);
+        siglen = take(siglen_ ? count * 8 : 0);
+        sigs = take(sign ? 0 : count * P.sig_bytes);
+        msgs = at;
+    }
+};
+
+// the batch's inputs and statuses on the device: its own buffers, or a packed input
+struct BatchIo {
+    const uint8_t *keys, *msg, *aux;
+    const uint64_t *off, *len, *siglen;
+    int32_t *status;
+    explicit BatchIo(const cuspx_batch *b)
+        : keys(b->bound_keys ? b->bound_keys : b->keys), msg(b->msg), aux(b->aux), off(b->off), len(b->len),
+          siglen(b->siglen), status(b->status) {
+        if (!b->packed) return;
+        const Packed p(b, b->count, b->op == CUSPX_OP_SIGN && b->use_aux, b->use_siglen);
+        keys = b->packed + p.keys;
+        off = (const uint64_t *)(b->packed + p.off);
+        len = (const uint64_t *)(b->packed + p.len);
+        aux = b->packed + (b->op == CUSPX_OP_SIGN ? p.opt : p.sigs);
+        siglen = (const uint64_t *)(b->packed + p.siglen);
+        msg = b->packed + p.msgs;
+        if (b->op == CUSPX_OP_SIGN) status = (int32_t *)(b->out + b->count * b->P.sig_bytes);
+    }
+};
+
 static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
     const FamilyOps &ops = family_of(b->set);
     const Tuning &tu = effective_tuning(b->ctx, b->set, b->op, b->count);
     const SetParams &P = b->P;
     const uint32_t cnt = (uint32_t)b->count;
+    const BatchIo io(b);
     if (b->op == CUSPX_OP_SIGN) {
         SignArgs A;
         A.count = cnt;
-        A.sk = KeyRef{b->bound_keys ? b->bound_keys : b->keys, b->use_keyrow ? b->keyrow : nullptr,
-                      (uint32_t)P.sk_bytes};
-        A.msg = MsgRef{b->msg, b->off, b->len};
-        A.optrand = b->use_aux ? b->aux : nullptr;
+        A.sk = KeyRef{io.keys, b->use_keyrow ? b->keyrow : nullptr, (uint32_t)P.sk_bytes};
+        A.msg = MsgRef{io.msg, io.off, io.len};
+        A.optrand = b->use_aux ? io.aux : nullptr;
         A.sig = b->out;
         A.work = b->work;
         A.fors_roots = b->fors_roots;
         A.leaves = b->leaves;
         A.roots = b->roots;
         A.chains = b->chains;
-        A.status = b->status;
+        A.status = io.status;
         A.ends = b->ends;
         A.ends_trees = b->ends_trees;
         A.fors_nodes = b->fors_nodes;
@@ -856,12 +906,11 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
     } else if (b->op == CUSPX_OP_VERIFY) {
         VerifyArgs A;
         A.count = cnt;
-        A.pk = KeyRef{b->bound_keys ? b->bound_keys : b->keys, b->use_keyrow ? b->keyrow : nullptr,
-                      (uint32_t)P.pk_bytes};
-        A.msg = MsgRef{b->msg, b->off, b->len};
-        A.sig = b->aux;
+        A.pk = KeyRef{io.keys, b->use_keyrow ? b->keyrow : nullptr, (uint32_t)P.pk_bytes};
+        A.msg = MsgRef{io.msg, io.off, io.len};
+        A.sig = io.aux;
         A.sig_stride = P.sig_bytes;
-        A.siglen = b->use_siglen ? b->siglen : nullptr;
+        A.siglen = b->use_siglen ? io.siglen : nullptr;
         A.work = b->work;
         A.fors_roots = b->fors_roots;
         A.verdict = b->status;
@@ -942,7 +991,7 @@ int cuspx_batch_run(cuspx_batch *b) {
         return CUSPX_OK;
     }
     const Tuning &tu = effective_tuning(ctx, b->set, b->op, b->count);
-    cuspx_batch::GraphKey key{b->count, b->use_keyrow, b->use_aux, b->use_siglen, b->long_msgs, b->bound_keys, tu};
+    cuspx_batch::GraphKey key{b->count, b->use_keyrow, b->use_aux, b->use_siglen, b->long_msgs, b->bound_keys, b->packed, tu};
     b->use_clock++;
     cuspx_batch::GraphEntry *hit = nullptr;
     for (auto &g : b->graphs)
@@ -1235,6 +1284,43 @@ struct OneshotJob {
 };
 
 // Run jobs of one (op, set) as one batch; under ctx->mu.
+// Most input bytes of a one-shot call that go to the device in one copy, and
+// its outputs back in one: a call of one item made four to six small copies
+// before its launch and two after it, each 1.5 to 3 us of the host's time and
+// of the stream's (crypto_sign_signature 139 -> 122 us, crypto_sign_open 500
+// -> 486 us).  Larger calls are bound by the bytes.
+constexpr size_t kPackedBytes = (size_t)1 << 20;
+
+// cuspx_batch_upload of `bytes` packed input bytes (struct Packed) in pinned
+// host memory; false if there is no device memory for them
+static bool upload_packed(cuspx_batch *b, size_t count, const uint8_t *in, size_t bytes, bool opt, bool siglen) {
+    if (b->packed_cap < bytes) {
+        const size_t cap = std::max(bytes, std::min<size_t>(2 * bytes, kPackedBytes));
+        void *p = nullptr;
+        if (cudaMalloc(&p, cap) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        b->allocs.push_back(p);   // a smaller one before it stays until the batch goes: graphs may hold it
+        b->packed_buf = (uint8_t *)p;
+        b->packed_cap = cap;
+    }
+    if (cudaMemcpyAsync(b->packed_buf, in, bytes, cudaMemcpyHostToDevice, b->s) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const Packed p(b, count, opt, siglen);
+    const uint64_t *len = (const uint64_t *)(in + p.len);
+    b->long_msgs = false;
+    for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = len[i] >= kPairMsgBytes;
+    b->packed = b->packed_buf;
+    b->use_keyrow = false;
+    b->use_aux = b->op == CUSPX_OP_VERIFY || opt;
+    b->use_siglen = siglen;
+    b->count = count;
+    return true;
+}
+
 static int oneshot_run(cuspx_ctx *ctx, int op, int set, const std::vector<OneshotJob *> &jobs) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     size_t count = 0, total = 0;
@@ -1282,13 +1368,16 @@ static int oneshot_run(cuspx_ctx *ctx, int op, int set, const std::vector<Onesho
     if ((rc = oneshot_stage(ctx, al16(key_b) + 2 * al16(count * 8) + al16(opt_b) + al16(sl_b) + al16(total + 16) +
                                      al16(sig_b) + al16(count * 4), st)))
         return rc;
+    // the inputs in the order of a packed input, then the outputs
     uint8_t *h_key = (uint8_t *)st.take(key_b);
     uint64_t *h_off = (uint64_t *)st.take(count * 8);
     uint64_t *h_len = (uint64_t *)st.take(count * 8);
     uint8_t *h_opt = opt_b ? (uint8_t *)st.take(opt_b) : nullptr;
     uint64_t *h_sl = sl_b ? (uint64_t *)st.take(sl_b) : nullptr;
+    uint8_t *h_sig = sign ? nullptr : (uint8_t *)st.take(sig_b);
     uint8_t *h_msg = (uint8_t *)st.take(total + 16);
-    uint8_t *h_sig = (uint8_t *)st.take(sig_b);
+    const size_t in_b = st.used;
+    if (sign) h_sig = (uint8_t *)st.take(sig_b);
     int32_t *h_st = (int32_t *)st.take(count * 4);
     memset(h_msg, 0, total + 16);
     size_t at = 0, o = 0;
@@ -1312,11 +1401,18 @@ static int oneshot_run(cuspx_ctx *ctx, int op, int set, const std::vector<Onesho
         }
         at += j->count;
     }
-    if ((rc = cuspx_batch_upload(b, count, h_key, count, nullptr, h_msg, total, h_off, h_len,
-                                 sign ? h_opt : h_sig, h_sl)))
-        return rc;
-    if ((rc = cuspx_batch_run(b))) return rc;
-    if ((rc = cuspx_batch_download(b, sign ? h_sig : nullptr, nullptr, h_st))) return rc;
+    if (in_b <= kPackedBytes && upload_packed(b, count, h_key, in_b, opt_b != 0, !sign)) {
+        if ((rc = cuspx_batch_run(b))) return rc;
+        if (sign) CK(cudaMemcpyAsync(h_sig, b->out, sig_b + count * 4, cudaMemcpyDeviceToHost, b->s), ctx);
+        else CK(cudaMemcpyAsync(h_st, b->status, count * 4, cudaMemcpyDeviceToHost, b->s), ctx);
+        if ((rc = cuspx_batch_sync(b))) return rc;
+    } else {
+        if ((rc = cuspx_batch_upload(b, count, h_key, count, nullptr, h_msg, total, h_off, h_len,
+                                     sign ? h_opt : h_sig, h_sl)))
+            return rc;
+        if ((rc = cuspx_batch_run(b))) return rc;
+        if ((rc = cuspx_batch_download(b, sign ? h_sig : nullptr, nullptr, h_st))) return rc;
+    }
     at = 0;
     for (const OneshotJob *j : jobs) {
         if (sign) memcpy(j->out, h_sig + at * P.sig_bytes, j->count * P.sig_bytes);
