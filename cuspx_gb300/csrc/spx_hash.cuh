@@ -379,6 +379,99 @@ SPX_DEV void keccak_f1600_short(uint64_t A[25]) {
 }
 
 // ---------------------------------------------------------------------------
+// The same permutation on bit-interleaved lanes: the low half of a lane holds
+// its even bits, the high half its odd ones, so a rotation by 2k rotates both
+// halves by k and one by 2k + 1 swaps them and rotates them by k + 1 and k.
+// Rotations by one (theta's five, rho's first) then cost one funnel shift
+// instead of two: 174 ALU instructions a round instead of 180.  For chains of
+// permutations, which convert once per chain.
+// ---------------------------------------------------------------------------
+// even bits of x to the low half, odd ones to the high half, and back
+__host__ __device__ constexpr uint32_t unzip32(uint32_t x) {
+    uint32_t t = (x ^ (x >> 1)) & 0x22222222u;
+    x ^= t ^ (t << 1);
+    t = (x ^ (x >> 2)) & 0x0c0c0c0cu;
+    x ^= t ^ (t << 2);
+    t = (x ^ (x >> 4)) & 0x00f000f0u;
+    x ^= t ^ (t << 4);
+    t = (x ^ (x >> 8)) & 0x0000ff00u;
+    return x ^ t ^ (t << 8);
+}
+__host__ __device__ constexpr uint32_t zip32(uint32_t x) {
+    uint32_t t = (x ^ (x >> 8)) & 0x0000ff00u;
+    x ^= t ^ (t << 8);
+    t = (x ^ (x >> 4)) & 0x00f000f0u;
+    x ^= t ^ (t << 4);
+    t = (x ^ (x >> 2)) & 0x0c0c0c0cu;
+    x ^= t ^ (t << 2);
+    t = (x ^ (x >> 1)) & 0x22222222u;
+    return x ^ t ^ (t << 1);
+}
+__host__ __device__ constexpr uint64_t interleave(uint64_t x) {
+    const uint32_t a = unzip32((uint32_t)x), b = unzip32((uint32_t)(x >> 32));
+    return (uint64_t)((a >> 16) | (b & 0xffff0000u)) << 32 | ((a & 0xffffu) | (b << 16));
+}
+__host__ __device__ constexpr uint64_t deinterleave(uint64_t x) {
+    const uint32_t e = (uint32_t)x, o = (uint32_t)(x >> 32);
+    return (uint64_t)zip32((e >> 16) | (o & 0xffff0000u)) << 32 | zip32((e & 0xffffu) | (o << 16));
+}
+struct KeccakIlRc {
+    uint64_t v[24];
+};
+__host__ __device__ constexpr KeccakIlRc keccak_il_rc() {
+    constexpr uint64_t rc[24] = {
+        0x0000000000000001ull, 0x0000000000008082ull, 0x800000000000808aull, 0x8000000080008000ull,
+        0x000000000000808bull, 0x0000000080000001ull, 0x8000000080008081ull, 0x8000000000008009ull,
+        0x000000000000008aull, 0x0000000000000088ull, 0x0000000080008009ull, 0x000000008000000aull,
+        0x000000008000808bull, 0x800000000000008bull, 0x8000000000008089ull, 0x8000000000008003ull,
+        0x8000000000008002ull, 0x8000000000000080ull, 0x000000000000800aull, 0x800000008000000aull,
+        0x8000000080008081ull, 0x8000000000008080ull, 0x0000000080000001ull, 0x8000000080008008ull};
+    KeccakIlRc k{};
+    for (int i = 0; i < 24; i++) k.v[i] = interleave(rc[i]);
+    return k;
+}
+static __constant__ KeccakIlRc KECCAK_IL_RC = keccak_il_rc();
+
+// rotate left by a constant c in 0..63
+SPX_DEV uint64_t rotl64_il(uint64_t x, int c) {
+    uint32_t e = (uint32_t)x, o = (uint32_t)(x >> 32);
+    if (c & 1) {
+        const uint32_t t = e;
+        e = o;
+        o = t;
+    }
+    const int ke = (c + 1) / 2, ko = c / 2;
+    return lane_of(ke & 31 ? __funnelshift_l(e, e, ke & 31) : e, ko & 31 ? __funnelshift_l(o, o, ko & 31) : o);
+}
+SPX_DEV void keccak_round_il(uint64_t A[25], uint64_t rc) {
+    constexpr int rho[25] = {0,  1,  62, 28, 27, 36, 44, 6,  55, 20, 3,  10, 43,
+                             25, 39, 41, 45, 15, 21, 8,  18, 2,  61, 56, 14};
+    uint64_t C[5], R[5], B[25];
+#pragma unroll
+    for (int x = 0; x < 5; x++) C[x] = A[x] ^ A[x + 5] ^ A[x + 10] ^ A[x + 15] ^ A[x + 20];
+#pragma unroll
+    for (int x = 0; x < 5; x++) R[x] = rotl64_il(C[x], 1);
+#pragma unroll
+    for (int i = 0; i < 25; i++) {
+        const int x = i % 5, y = i / 5;
+        B[y + 5 * ((2 * x + 3 * y) % 5)] = rotl64_il(A[i] ^ (C[(x + 4) % 5] ^ R[(x + 1) % 5]), rho[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 25; i++) {
+        const int y = 5 * (i / 5), x = i % 5;
+        A[i] = B[i] ^ (~B[y + (x + 1) % 5] & B[y + (x + 2) % 5]);
+    }
+    A[0] ^= rc;
+}
+// keccak_f1600_short on interleaved lanes
+SPX_DEV void keccak_f1600_short_il(uint64_t A[25]) {
+    keccak_round_il(A, interleave(0x0000000000000001ull));
+#pragma unroll 2
+    for (int r = 1; r < 23; r++) keccak_round_il(A, KECCAK_IL_RC.v[r]);
+    keccak_round_il(A, interleave(0x8000000080008008ull));
+}
+
+// ---------------------------------------------------------------------------
 // Keccak-f[1600] spread over one warp, for the serial sponge of a long
 // message: lane i < 25 holds state lane i (x = i % 5, y = i / 5); lanes
 // 25..31 compute values nobody reads and only take part in the shuffles.

@@ -629,10 +629,12 @@ __global__ void __launch_bounds__(256, HF::kLeafMinBlocks) k_leaves(SetParams P,
         if (rec) HF::store(chain + ((uint64_t)c * 16) * N, v);
         typename HF::FCtx fc;
         HF::f_prepare(fc, wa, key);
+        HF::chain_in(v);
         for (int s = 0; s < 15; s++) {
             HF::f_step(v, v, fc, s, key);
-            if (rec) HF::store(chain + ((uint64_t)c * 16 + s + 1) * N, v);
+            if (rec) HF::chain_store(chain + ((uint64_t)c * 16 + s + 1) * N, v);
         }
+        HF::chain_out(v);
         HF::t_absorb(ts, v, key);
     }
     uint32_t leaf[W];
@@ -732,11 +734,12 @@ __global__ void __launch_bounds__(128) k_leaf_chains(SetParams P, LeafArgs A) {
     if (rec) HF::store(chain, v);
     typename HF::FCtx fc;
     HF::f_prepare(fc, wa, key);
+    HF::chain_in(v);
     for (int s = 0; s < 15; s++) {
         HF::f_step(v, v, fc, s, key);
-        if (rec) HF::store(chain + (uint64_t)(s + 1) * N, v);
+        if (rec) HF::chain_store(chain + (uint64_t)(s + 1) * N, v);
     }
-    HF::store(chain_end<N>(A, x, c), v);
+    HF::chain_store(chain_end<N>(A, x, c), v);
 }
 
 // key, address and output of a T_len thread: the launch's leaf x
@@ -1212,7 +1215,9 @@ __global__ void k_verify_ht(SetParams P, VerifyArgs A) {
             adrs_chain(wa, c);
             typename HF::FCtx fc;
             HF::f_prepare(fc, wa, key);
+            HF::chain_in(v);
             for (uint32_t s = ln; s < 15; s++) HF::f_step(v, v, fc, s, key);
+            HF::chain_out(v);
             HF::t_absorb(ts, v, key);
         }
         uint32_t leaf[W];
@@ -1360,7 +1365,7 @@ __global__ void k_verify_chains(SetParams P, VerifyArgs A, int L, int per_warp) 
         // has a chain with steps left or the range is exhausted
         while (true) {
             if (have && s >= 15) {
-                HF::store(A.wpk + ((uint64_t)item * LEN + c) * N, v);
+                HF::chain_store(A.wpk + ((uint64_t)item * LEN + c) * N, v);
                 have = false;
             }
             const uint32_t need = __ballot_sync(0xffffffffu, !have);
@@ -1390,6 +1395,7 @@ __global__ void k_verify_chains(SetParams P, VerifyArgs A, int L, int per_warp) 
                     HF::f_prepare(fc, wa, key);
                     HF::load(v, A.sig + (uint64_t)item * A.sig_stride + N + P.fors_bytes +
                                     (uint64_t)L * (P.wots_bytes + P.hp * N) + (uint64_t)c * N);
+                    HF::chain_in(v);
                     have = true;
                 }
             }

@@ -269,6 +269,10 @@ struct Sha2 {
             sha256_rounds<0, W + 5, kFmaA>(f.mst, x);
         }
     }
+    // a chain's value needs no form of its own here (see Shake)
+    SPX_DEV static void chain_in(uint32_t *) {}
+    SPX_DEV static void chain_out(uint32_t *) {}
+    SPX_DEV static void chain_store(uint8_t *p, const uint32_t v[W]) { store(p, v); }
     // out = F(in) at hash address `hash` of the prepared chain
     SPX_DEV static void f_step(uint32_t out[W], const uint32_t in[W], const FCtx &f, uint32_t hash,
                                const KeyRegs<N> &k) {
@@ -898,17 +902,78 @@ struct Shake {
         for (int i = 0; i < W; i++) { t[i] = l[i]; t[W + i] = r[i]; }
         thash<2 * NL>(out, k, a, t);
     }
-    // WOTS+ chain steps: a Keccak permutation has no reusable prefix, so the
-    // prepared chain is just its address
+    // WOTS+ chain steps, on bit-interleaved lanes (keccak_f1600_short_il):
+    // the chain's value is interleaved by chain_in before the first step and
+    // back by chain_out (or chain_store) after the last; the prepared chain is
+    // its PUB_SEED and ADRS lanes.  (1024 signatures of SHAKE-256f: chains
+    // 62.2 -> 60.9 ms.)
     struct FCtx {
-        Adrs a;
+        uint64_t pre[NL], ad[3];   // ad[2] without the hash byte
     };
-    SPX_DEV static void f_prepare(FCtx &f, const Adrs &a, const KeyRegs<N> &) { f.a = a; }
+    SPX_DEV static void f_prepare(FCtx &f, const Adrs &a, const KeyRegs<N> &k) {
+        Adrs b = a;
+        adrs_hash(b, 0);
+        uint64_t al[4];
+        adrs_lanes(b, al);
+#pragma unroll
+        for (int i = 0; i < NL; i++) f.pre[i] = interleave(vlane(k.pub, i));
+#pragma unroll
+        for (int i = 0; i < 3; i++) f.ad[i] = interleave(al[i]);
+    }
+    SPX_DEV static void chain_in(uint32_t v[W]) {
+#pragma unroll
+        for (int i = 0; i < NL; i++) {
+            const uint64_t x = interleave(vlane(v, i));
+            v[2 * i] = (uint32_t)x;
+            v[2 * i + 1] = (uint32_t)(x >> 32);
+        }
+    }
+    SPX_DEV static void chain_out(uint32_t v[W]) {
+#pragma unroll
+        for (int i = 0; i < NL; i++) {
+            const uint64_t x = deinterleave(vlane(v, i));
+            v[2 * i] = (uint32_t)x;
+            v[2 * i + 1] = (uint32_t)(x >> 32);
+        }
+    }
+    SPX_DEV static void chain_store(uint8_t *p, const uint32_t v[W]) {
+        uint32_t t[W];
+#pragma unroll
+        for (int i = 0; i < W; i++) t[i] = v[i];
+        chain_out(t);
+        store(p, t);
+    }
     SPX_DEV static void f_step(uint32_t out[W], const uint32_t in[W], const FCtx &f, uint32_t hash,
-                               const KeyRegs<N> &k) {
-        Adrs a = f.a;
-        adrs_hash(a, hash);
-        F(out, in, a, k);
+                               const KeyRegs<N> &) {
+        // hash byte: ADRS byte 21, bits 40..43 of lane 2
+        const uint64_t ad2 = f.ad[2] | (uint64_t)((hash >> 1 & 1u) | (hash >> 2 & 2u)) << 52 |
+                             (uint64_t)((hash & 1u) | (hash >> 1 & 2u)) << 20;
+        uint64_t mk[NL], A[25];
+#pragma unroll
+        for (int i = 0; i < NL; i++) mk[i] = 0;
+#pragma unroll
+        for (int pass = ROBUST ? 0 : 1; pass < 2; pass++) {   // robust: the bitmask, then F
+#pragma unroll
+            for (int i = 0; i < 25; i++) A[i] = 0;
+#pragma unroll
+            for (int i = 0; i < NL; i++) A[i] = f.pre[i];
+            A[NL] = f.ad[0];
+            A[NL + 1] = f.ad[1];
+            A[NL + 2] = ad2;
+            if (pass == 1) {
+#pragma unroll
+                for (int i = 0; i < NL; i++) A[NL + 4 + i] = vlane(in, i) ^ mk[i];
+            }
+            A[NL + 4 + (pass == 1 ? NL : 0)] = interleave(0x1Full);
+            A[16] ^= interleave(0x8000000000000000ull);
+            keccak_f1600_short_il(A);
+            if (pass == 0) {
+#pragma unroll
+                for (int i = 0; i < NL; i++) mk[i] = A[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NL; i++) { out[2 * i] = (uint32_t)A[i]; out[2 * i + 1] = (uint32_t)(A[i] >> 32); }
     }
 
     // PRF = SHAKE256(SK_SEED || ADRS) (hash_shake256.cu:38-47)

@@ -115,7 +115,9 @@ __global__ void __launch_bounds__(VerifyBlock<HF, I>::kThreads) k_verify_block(S
                 HF::load(v, reinterpret_cast<const uint8_t *>(rows(L, it) + c * W));
                 typename HF::FCtx fc;
                 HF::f_prepare(fc, wa, key);
+                HF::chain_in(v);
                 for (uint32_t s = 15u - (e >> 16); s < 15u; s++) HF::f_step(v, v, fc, s, key);
+                HF::chain_out(v);
                 tlen_mask_value<HF>(v, key, L, tree_L, idx_L, (int)c);
                 HF::store(reinterpret_cast<uint8_t *>(vals + id * W), v);
             }

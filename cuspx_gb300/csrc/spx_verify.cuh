@@ -1340,7 +1340,9 @@ __global__ void __launch_bounds__(128) k_verify_item(SetParams P, VerifyArgs A) 
                 const uint32_t ln = chain_len<HF>(P, root, c);
 #pragma unroll
                 for (int i = 0; i < W; i++) v[i] = nv[i];
+                HF::chain_in(v);
                 for (uint32_t s = ln; s < 15; s++) HF::f_step(v, v, fc, s, key);
+                HF::chain_out(v);
                 PV::write_value(stream, c, v);
                 __threadfence_block();   // the value before its done bit
                 PV::mark_done(S, c);

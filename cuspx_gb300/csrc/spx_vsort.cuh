@@ -497,7 +497,9 @@ __global__ void __launch_bounds__(128) k_vsort_chains(SetParams P, VerifyArgs A,
     HF::f_prepare(fc, wa, key);
     uint32_t v[W];
     HF::load(v, A.sig + (uint64_t)item * A.sig_stride + sig_layer_off(P, L) + (uint64_t)c * N);
+    HF::chain_in(v);
     for (uint32_t s = 15u - (uint32_t)l; s < 15u; s++) HF::f_step(v, v, fc, s, key);
+    HF::chain_out(v);
     tlen_mask_value<HF>(v, key, L, tree_L, idx_L, c);
     HF::store(A.wpk + ((uint64_t)item * LEN + c) * N, v);
 }
@@ -559,7 +561,9 @@ __global__ void __launch_bounds__(128) k_vspec_cand(SetParams P, VerifyArgs A, u
     HF::f_prepare(fc, wa, key);
     uint32_t v[W];
     HF::load(v, A.sig + (uint64_t)item * A.sig_stride + sig_layer_off(P, L) + (uint64_t)c * N);
+    HF::chain_in(v);
     for (uint32_t st = dg; st < 15u; st++) HF::f_step(v, v, fc, st, key);
+    HF::chain_out(v);
     tlen_mask_value<HF>(v, key, L, tree_L, idx_L, c);
     HF::store(cand + ((((uint64_t)item * P.d + L) * LEN + c) * 16 + dg) * N, v);
 }
