@@ -153,10 +153,19 @@ template <class HF>
 struct Family {
     static constexpr int W = HF::W, N = 4 * W;
     using TL = TlLanes<HF>;
+    // Dynamic shared memory that k_leaf_chains asks for, to leave room on each
+    // SM for the FORS trees beside it: with as many chain blocks as fit, robust
+    // FORS at n = 32 (PRF and six-unit H) and the chains (three blocks of code)
+    // took their SMs in turn.  With three chain blocks an SM, 1024 signatures
+    // of 256f take 57.3 ms, 61.2 without, 100 of 256s 54.5 and 57.4; asking for
+    // 56 or 44 KB gave 57.9 and 59.8 for the first.  128f-robust and
+    // 192f-simple gained 1 % or less from a cap, 128f-simple nothing.
+    static constexpr size_t kChainSmem = !HF::kShake && HF::kRobust && N == 32 ? 74u * 1024u : 0;
 
     static cudaError_t configure() {
         cudaError_t e;
         const int big = 200 * 1024;
+        if ((e = cudaFuncSetAttribute(k_leaf_chains<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         if ((e = cudaFuncSetAttribute(k_leaves<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         if ((e = cudaFuncSetAttribute(k_leaf_tlen<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         if ((e = cudaFuncSetAttribute(k_fors_sign<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
@@ -185,7 +194,7 @@ struct Family {
         // is a request's (one took ~50 ms of host time and held back every
         // queued request of its class).
         cudaFuncAttributes fa;
-        const void *rest[] = {(const void *)k_sign_msg<HF>, (const void *)k_leaf_chains<HF>, (const void *)k_leaf_tstream<HF>,
+        const void *rest[] = {(const void *)k_sign_msg<HF>, (const void *)k_leaf_tstream<HF>,
                               (const void *)k_trees_lane<HF>, (const void *)k_fors_top<HF>, (const void *)k_share<HF>, (const void *)k_share_leaves<HF>,
                               (const void *)k_verify_msg<HF>, (const void *)k_verify_fors<HF>,
                               (const void *)k_verify_chains<HF>, (const void *)k_vsort_chains<HF>,
@@ -300,7 +309,12 @@ struct Family {
             L.tree0 = (uint32_t)t;
             L.trees = (uint32_t)(trees - t < ends_trees ? trees - t : ends_trees);
             const uint64_t nl = (uint64_t)L.trees << P.hp;
-            k_leaf_chains<HF><<<ceil_div(nl * LEN, 128), 128, 0, s>>>(P, L);
+            const uint32_t blocks = ceil_div(nl * LEN, 128);
+            // from a few rounds of capped blocks on; one signature of 256f, 142
+            // blocks, takes 0.41 ms capped and 0.35 not, and key generation has
+            // no FORS trees to make room for
+            const bool cap = L.work && blocks >= 16u * (uint32_t)device_sms();
+            k_leaf_chains<HF><<<blocks, 128, cap ? kChainSmem : 0, s>>>(P, L);
             CUSPX_MARK(pt, "k_leaf_chains", s);
             if (latency) {
                 k_leaf_tlen<HF><<<ceil_div(nl, TL::kPerBlock), TL::kThreads, TL::smem(), s>>>(P, L);

@@ -126,3 +126,15 @@ def test_fors_lane_spread(engine, setname, count):
     assert not any(st)
     assert sigs[count - 1] == _oracle(setname).sign(msgs[count - 1], sks[count - 1])
     assert not any(engine.verify_batch(sid, pks, msgs, sigs))
+
+
+@pytest.mark.parametrize("count", [17, 18, 40])
+def test_chain_block_cap(engine, count):
+    """256f-robust below, at and above 16 chain blocks an SM (152 of them),
+    where the chain blocks' number per SM is capped"""
+    sid = engine.set_id("sha256-256f-robust")
+    pks, sks, msgs = _requests(engine, sid, count, count, 10)
+    sigs, st = engine.sign_batch(sid, sks, msgs)
+    assert not any(st)
+    assert sigs == _in_pieces(engine, sid, sks, msgs, 9)
+    assert sigs[count - 1] == _oracle("sha256-256f-robust").sign(msgs[count - 1], sks[count - 1])
