@@ -158,6 +158,7 @@ struct cuspx_batch {
     int32_t *status = nullptr;
     SignWork *work = nullptr;
     uint8_t *fors_roots = nullptr, *leaves = nullptr, *roots = nullptr, *chains = nullptr;
+    uint32_t *mids = nullptr;  // key generation, SHA-256: 8 words per key
     uint8_t *wpk = nullptr, *cur_root = nullptr;
     uint32_t *ctr = nullptr;   // persistent verify item counter
     VerifyLists vlists{};      // verify_mode 3: chains bucketed by steps
@@ -691,6 +692,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
         A((void **)&b->out, cap * 2 * n);
         A((void **)&b->leaves, cap * ((size_t)1 << P.hp) * n);
         A((void **)&b->roots, cap * n);
+        A((void **)&b->mids, cap * 8 * sizeof(uint32_t));
         ends(cap);
     } else {
         A((void **)&b->keyrow, cap * sizeof(uint32_t));
@@ -919,7 +921,7 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.ctr = b->ctr;
         ops.verify(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0, &b->vlists, &b->vfork);
     } else {
-        KeygenArgs K{cnt, b->keys, b->out, b->leaves, b->roots, b->ends, b->ends_trees};
+        KeygenArgs K{cnt, b->keys, b->out, b->leaves, b->roots, b->ends, b->ends_trees, b->mids};
         ops.keygen(P, K, tu, b->s, pt);
     }
 }

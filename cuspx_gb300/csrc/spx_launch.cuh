@@ -43,6 +43,7 @@ struct KeygenArgs {
     uint8_t *roots;    // count x n scratch
     uint8_t *ends;        // chain-parallel scratch (ends_trees x 2^hp x len x n) or null
     uint32_t ends_trees;
+    uint32_t *mids;       // SHA-256: 8 words per key
 };
 
 // Optional per-kernel timing: an event is recorded on the launch stream
@@ -204,6 +205,7 @@ struct Family {
             if ((e = cudaFuncGetAttributes(&fa, f))) return e;
         if constexpr (!HF::kShake) {
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_vspec_walk_group<HF>))) return e;
+            if ((e = cudaFuncGetAttributes(&fa, (const void *)k_key_mid<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_sign_msg_pair<HF>))) return e;
             if ((e = cudaFuncGetAttributes(&fa, (const void *)k_verify_msg_pair<HF>))) return e;
         } else {
@@ -398,12 +400,12 @@ struct Family {
         }
         if (split) cudaEventRecord(fk->join, sf);
         {
-            LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false, A.share};
+            LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false, A.share, nullptr};
             leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? A.ends_trees : 0,
                    A.count <= (uint32_t)tu.chain_mode_max && A.count <= 256);
         }
         {
-            TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig, A.share};
+            TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig, A.share, nullptr};
             trees(P, T, tu, s);
             CUSPX_MARK(pt, "k_trees", s);
         }
@@ -609,9 +611,13 @@ struct Family {
     static void keygen(const SetParams &P, const KeygenArgs &K, const Tuning &tu, cudaStream_t s, PhaseTimer *pt) {
         if (K.count == 0) return;
         KeyRef kr{K.sk, nullptr, (uint32_t)(4 * N)};
-        LeafArgs L{K.count, P.d - 1, 1, kr, nullptr, K.leaves, nullptr, K.ends, 0, 0, false, {}};
+        if constexpr (!HF::kShake) {
+            k_key_mid<HF><<<ceil_div(K.count, 128), 128, 0, s>>>(kr, K.count, K.mids);
+            CUSPX_MARK(pt, "k_key_mid", s);
+        }
+        LeafArgs L{K.count, P.d - 1, 1, kr, nullptr, K.leaves, nullptr, K.ends, 0, 0, false, {}, K.mids};
         leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? K.ends_trees : 0, false);
-        TreeArgs T{K.count, P.d - 1, 1, kr, nullptr, K.leaves, K.roots, nullptr, {}};
+        TreeArgs T{K.count, P.d - 1, 1, kr, nullptr, K.leaves, K.roots, nullptr, {}, K.mids};
         trees(P, T, tu, s);
         CUSPX_MARK(pt, "k_trees", s);
         k_keygen_finish<N><<<ceil_div(K.count, 128), 128, 0, s>>>(K);

@@ -138,3 +138,18 @@ def test_chain_block_cap(engine, count):
     assert not any(st)
     assert sigs == _in_pieces(engine, sid, sks, msgs, 9)
     assert sigs[count - 1] == _oracle("sha256-256f-robust").sign(msgs[count - 1], sks[count - 1])
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-128f-simple", 1), ("sha256-192f-robust", 127),
+                                           ("sha256-256f-simple", 129), ("shake256-128f-simple", 129)])
+def test_keygen_midstates(engine, setname, count):
+    """a key, the last of a block of keys and the first of the next: as the
+    oracle's, and as each key by itself"""
+    import cuspx_gb300 as c
+    rng = random.Random(11)
+    sid = engine.set_id(setname)
+    seeds = [rng.randbytes(c.set_sizes(sid)["seed"]) for _ in range(count)]
+    pks, sks = engine.keypair_batch(sid, seeds)
+    for i in sorted({0, count // 2, count - 1}):
+        assert (pks[i], sks[i]) == _oracle(setname).seed_keypair(seeds[i])
+        assert ([pks[i]], [sks[i]]) == engine.keypair_batch(sid, [seeds[i]])
