@@ -73,6 +73,21 @@ static const FamilyOps &family_of(int set) {
     return g_family[s.hash][s.n / 8 - 2][s.robust];
 }
 
+// Messages of at least this many bytes are hashed by the long-message kernels,
+// two warps per 32 messages (SHA-256) or a warp per message (SHAKE-256), the
+// rest by a thread each.  Below, the second kernel costs more than the threads'
+// hashing; above, the batch waits for its longest message.  Against 2048 bytes:
+// a message of 1024 B verified under 128f 439 -> 429 us, one of 1536 B signed
+// 163 -> 149 us (of 1024 B 138 -> 134, but batches of 100 and more lose 0.3 %),
+// one of 1024 B signed under shake256-128f 212 -> 187 us, of 300 B 168 -> 159.
+// Larger SHAKE-256 batches fill the SMs with a thread a message (16384 verified
+// 1000-B messages: 21.7 ms, 21.9 with a warp each).
+static uint64_t long_msg_bytes(int set, int op, size_t count) {
+    const bool shake = kSets[set].hash, verify = op == CUSPX_OP_VERIFY;
+    if (count > (verify && !shake ? 4096 : 1024)) return 2048;
+    return shake ? 256 : (verify ? 1024 : 1536);
+}
+
 // registration for other translation units of the library
 void ensure_registered() { register_all(); }
 }  // namespace cuspx
@@ -88,9 +103,6 @@ static const size_t kEndsBytes = (size_t)256 << 20;
 // items per verify batch that the speculative chain table covers (the
 // largest verify_spec_max; 64 x 22 x 35 x 16 x 16 B = 12.6 MB at 128f)
 static const int kSpecItems = 64;
-// messages of at least this many bytes (32 SHA-256 blocks) are hashed by the
-// two-warp message kernels of the SHA-256 sets
-static const uint64_t kPairMsgBytes = 2048;
 
 struct OneshotJob;
 
@@ -163,9 +175,9 @@ struct cuspx_batch {
     uint32_t *ctr = nullptr;   // persistent verify item counter
     VerifyLists vlists{};      // verify_mode 3: chains bucketed by steps
     VerifyFork vfork{};        // verify_mode 3: streams of the item groups
-    bool long_msgs = false;    // the last upload held a message of >= kPairMsgBytes (SHA-256:
-                               // hash those over two warps; both kernels read the device
-                               // lengths, so the split is right whatever the flag says)
+    bool long_msgs = false;    // the last upload held a message of >= long_msg_bytes (both
+                               // kernels read the device lengths, so the split is right
+                               // whatever the flag says)
     uint8_t *ends = nullptr;   // chain-parallel leaf scratch, for ends_trees trees
     uint32_t ends_trees = 0;
     uint8_t *fors_nodes = nullptr;
@@ -815,8 +827,9 @@ int cuspx_batch_upload(cuspx_batch *b, size_t count, const uint8_t *keys, size_t
         CK(cudaMemcpyAsync(b->off, msg_off, count * 8, cudaMemcpyHostToDevice, b->s), ctx);
         CK(cudaMemcpyAsync(b->len, msg_len, count * 8, cudaMemcpyHostToDevice, b->s), ctx);
     }
+    const uint64_t lb = long_msg_bytes(b->set, b->op, count);
     b->long_msgs = false;
-    for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = msg_len[i] >= kPairMsgBytes;
+    for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = msg_len[i] >= lb;
     b->use_keyrow = key_index != nullptr;
     if (b->op == CUSPX_OP_SIGN) {
         b->use_aux = aux != nullptr;
@@ -903,7 +916,7 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.fors_nodes = b->fors_nodes;
         A.fors_lanes = b->fors_lanes;
         A.share = b->share;
-        ops.sign(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0,
+        ops.sign(P, A, tu, b->s, pt, b->long_msgs ? long_msg_bytes(b->set, b->op, b->count) : 0,
                  (CUSPX_SIGN_FORK && b->fork.side) ? &b->fork : nullptr);
     } else if (b->op == CUSPX_OP_VERIFY) {
         VerifyArgs A;
@@ -919,7 +932,7 @@ static void launch_seq(cuspx_batch *b, PhaseTimer *pt) {
         A.wpk = b->wpk;
         A.cur_root = b->cur_root;
         A.ctr = b->ctr;
-        ops.verify(P, A, tu, b->s, pt, b->long_msgs ? kPairMsgBytes : 0, &b->vlists, &b->vfork);
+        ops.verify(P, A, tu, b->s, pt, b->long_msgs ? long_msg_bytes(b->set, b->op, b->count) : 0, &b->vlists, &b->vfork);
     } else {
         KeygenArgs K{cnt, b->keys, b->out, b->leaves, b->roots, b->ends, b->ends_trees, b->mids};
         ops.keygen(P, K, tu, b->s, pt);
@@ -1313,8 +1326,9 @@ static bool upload_packed(cuspx_batch *b, size_t count, const uint8_t *in, size_
     }
     const Packed p(b, count, opt, siglen);
     const uint64_t *len = (const uint64_t *)(in + p.len);
+    const uint64_t lb = long_msg_bytes(b->set, b->op, count);
     b->long_msgs = false;
-    for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = len[i] >= kPairMsgBytes;
+    for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = len[i] >= lb;
     b->packed = b->packed_buf;
     b->use_keyrow = false;
     b->use_aux = b->op == CUSPX_OP_VERIFY || opt;

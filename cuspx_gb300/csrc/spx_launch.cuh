@@ -89,7 +89,7 @@ struct VerifyFork {
 struct FamilyOps {
     cudaError_t (*configure)();
     // long_msg: messages of at least this many bytes are hashed two warps per
-    // 32 messages (SHA-256 sets; 0 or a SHAKE set: one thread each).
+    // 32 messages (SHA-256) or a warp each (SHAKE-256); 0: all by one thread.
     // fk: optional side stream (ignored while per-kernel timing is on).
     void (*sign)(const SetParams &, SignArgs, const Tuning &, cudaStream_t, PhaseTimer *, uint64_t long_msg,
                  const StreamFork *fk);

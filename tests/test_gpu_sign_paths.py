@@ -153,3 +153,23 @@ def test_keygen_midstates(engine, setname, count):
     for i in sorted({0, count // 2, count - 1}):
         assert (pks[i], sks[i]) == _oracle(setname).seed_keypair(seeds[i])
         assert ([pks[i]], [sks[i]]) == engine.keypair_batch(sid, [seeds[i]])
+
+
+@pytest.mark.parametrize("setname", ["sha256-128f-simple", "sha256-192f-robust", "sha256-256f-simple",
+                                     "shake256-128f-simple", "shake256-192f-simple", "shake256-256f-robust"])
+@pytest.mark.parametrize("edge", [256, 1024, 1536])
+def test_message_kernels_around_threshold(engine, setname, edge):
+    """messages about the lengths from which the long-message kernels take
+    them, alone in a batch and beside short and longer ones"""
+    rng = random.Random(edge)
+    sid, o = engine.set_id(setname), _oracle(setname)
+    pk, sk = o.seed_keypair(rng.randbytes(3 * o.p.n))
+    msgs = [rng.randbytes(x) for x in (edge - 1, edge, edge + 1, 0, 3 * edge, 77)]
+    for some in ([msgs[0]], [msgs[1]], msgs):
+        sigs, st = engine.sign_batch(sid, [sk] * len(some), some)
+        assert not any(st)
+        assert sigs == [o.sign(m, sk) for m in some]
+        wrong = [m[:-1] + bytes([m[-1] ^ 1]) for m in some if m]
+        keep = [s for m, s in zip(some, sigs) if m]
+        got = engine.verify_batch(sid, [pk] * (len(some) + len(wrong)), some + wrong, sigs + keep)
+        assert list(got) == [0] * len(some) + [-1] * len(wrong)
