@@ -75,17 +75,23 @@ static const FamilyOps &family_of(int set) {
 
 // Messages of at least this many bytes are hashed by the long-message kernels,
 // two warps per 32 messages (SHA-256) or a warp per message (SHAKE-256), the
-// rest by a thread each.  Below, the second kernel costs more than the threads'
-// hashing; above, the batch waits for its longest message.  Against 2048 bytes:
-// a message of 1024 B verified under 128f 439 -> 429 us, one of 1536 B signed
-// 163 -> 149 us (of 1024 B 138 -> 134, but batches of 100 and more lose 0.3 %),
-// one of 1024 B signed under shake256-128f 212 -> 187 us, of 300 B 168 -> 159.
-// Larger SHAKE-256 batches fill the SMs with a thread a message (16384 verified
-// 1000-B messages: 21.7 ms, 21.9 with a warp each).
+// rest by a thread each, or by a warp each in small SHA-256 batches.  Below, the
+// second kernel costs more than it saves; above, the batch waits for its
+// longest message.  Against 2048 bytes: 1024 messages of 1536 B verified under
+// 128f 1.062 -> 1.044 ms; one of 1024 B signed under shake256-128f 212 -> 187
+// us, of 300 B 168 -> 159.  Larger SHAKE-256 batches fill the SMs with a thread
+// a message (16384 verified messages of 1000 B: 21.7 ms, 21.9 with a warp each).
 static uint64_t long_msg_bytes(int set, int op, size_t count) {
     const bool shake = kSets[set].hash, verify = op == CUSPX_OP_VERIFY;
+    if (!shake && group_messages(count)) return 1024;
     if (count > (verify && !shake ? 4096 : 1024)) return 2048;
     return shake ? 256 : (verify ? 1024 : 1536);
+}
+// The long-message kernels run if a message has at least this many bytes.  A
+// warp a message is as fast up to some 4 KiB (20000 B signed under 128f: 732
+// us, 703 by two warps; 1 MiB: 34.2 ms and 31.5) and one launch less.
+static uint64_t long_msg_min(int set, int op, size_t count) {
+    return !kSets[set].hash && group_messages(count) ? 4096 : long_msg_bytes(set, op, count);
 }
 
 // registration for other translation units of the library
@@ -175,7 +181,7 @@ struct cuspx_batch {
     uint32_t *ctr = nullptr;   // persistent verify item counter
     VerifyLists vlists{};      // verify_mode 3: chains bucketed by steps
     VerifyFork vfork{};        // verify_mode 3: streams of the item groups
-    bool long_msgs = false;    // the last upload held a message of >= long_msg_bytes (both
+    bool long_msgs = false;    // the last upload held a message of >= long_msg_min (the
                                // kernels read the device lengths, so the split is right
                                // whatever the flag says)
     uint8_t *ends = nullptr;   // chain-parallel leaf scratch, for ends_trees trees
@@ -827,7 +833,7 @@ int cuspx_batch_upload(cuspx_batch *b, size_t count, const uint8_t *keys, size_t
         CK(cudaMemcpyAsync(b->off, msg_off, count * 8, cudaMemcpyHostToDevice, b->s), ctx);
         CK(cudaMemcpyAsync(b->len, msg_len, count * 8, cudaMemcpyHostToDevice, b->s), ctx);
     }
-    const uint64_t lb = long_msg_bytes(b->set, b->op, count);
+    const uint64_t lb = long_msg_min(b->set, b->op, count);
     b->long_msgs = false;
     for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = msg_len[i] >= lb;
     b->use_keyrow = key_index != nullptr;
@@ -1326,7 +1332,7 @@ static bool upload_packed(cuspx_batch *b, size_t count, const uint8_t *in, size_
     }
     const Packed p(b, count, opt, siglen);
     const uint64_t *len = (const uint64_t *)(in + p.len);
-    const uint64_t lb = long_msg_bytes(b->set, b->op, count);
+    const uint64_t lb = long_msg_min(b->set, b->op, count);
     b->long_msgs = false;
     for (size_t i = 0; i < count && !b->long_msgs; i++) b->long_msgs = len[i] >= lb;
     b->packed = b->packed_buf;

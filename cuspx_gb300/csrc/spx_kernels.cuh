@@ -224,10 +224,9 @@ SPX_DEV uint32_t chain_len(const SetParams &P, const uint32_t msg[HF::W], int c)
 }
 
 // Work record of an item from its H_msg digest (hash_sha256.cu:249-261):
-// FORS digest, tree and leaf index, and the key's midstate from PUB_SEED.
-template <class HF>
-SPX_DEV SignWork work_from_digest(const SetParams &P, const uint8_t *dg, const uint8_t *pub) {
-    constexpr int N = 4 * HF::W;
+// FORS digest, tree and leaf index (work_indices), and the key's midstate from
+// PUB_SEED.
+SPX_DEV SignWork work_indices(const SetParams &P, const uint8_t *dg) {
     SignWork w;
     for (int j = 0; j < 48; j++) w.mhash[j] = j < P.fors_msg_bytes ? dg[j] : 0;
     uint64_t t = 0;
@@ -239,6 +238,12 @@ SPX_DEV SignWork work_from_digest(const SetParams &P, const uint8_t *dg, const u
     w.tree = t;
     w.idx_leaf = l;
     w.flags = 0;
+    return w;
+}
+template <class HF>
+SPX_DEV SignWork work_from_digest(const SetParams &P, const uint8_t *dg, const uint8_t *pub) {
+    constexpr int N = 4 * HF::W;
+    SignWork w = work_indices(P, dg);
     KeyRegs<N> key;
     HF::key_init(key, pub, pub);
 #pragma unroll

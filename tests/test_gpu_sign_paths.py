@@ -173,3 +173,39 @@ def test_message_kernels_around_threshold(engine, setname, edge):
         keep = [s for m, s in zip(some, sigs) if m]
         got = engine.verify_batch(sid, [pk] * (len(some) + len(wrong)), some + wrong, sigs + keep)
         assert list(got) == [0] * len(some) + [-1] * len(wrong)
+
+
+@pytest.mark.parametrize("setname", ["sha256-128f-simple", "sha256-192f-robust", "sha256-256f-simple"])
+def test_message_warps(engine, setname):
+    """a warp per message: the padding about a block's end, one and two rounds
+    of 32 blocks, and lengths about that from which the batch's long messages
+    are hashed apart, alone and with a wrong-length signature beside them"""
+    rng = random.Random(12)
+    sid, o = engine.set_id(setname), _oracle(setname)
+    n = o.p.n
+    pk, sk = o.seed_keypair(rng.randbytes(3 * n))
+    lens = [0, 1, 3, 4]
+    for pre in (n, 3 * n):
+        for blocks in (2, 32, 33):
+            lens += [64 * blocks - 9 - pre + x for x in (-1, 0, 1)]
+    for some in (lens + [4095], lens + [1023, 1024, 4095, 4096, 4097, 9000], [4096]):
+        msgs = [rng.randbytes(x) for x in some]
+        sigs, st = engine.sign_batch(sid, [sk] * len(msgs), msgs)
+        assert not any(st)
+        assert sigs == [o.sign(m, sk) for m in msgs]
+        vm, vs = msgs + msgs[-1:] * 2, sigs + [sigs[-1], bytes([sigs[-1][0] ^ 1]) + sigs[-1][1:]]
+        got = engine.verify_batch(sid, [pk] * len(vm), vm, vs,
+                                  siglens=[len(x) for x in sigs] + [len(sigs[0]) - 1, len(sigs[0])])
+        assert list(got) == [0] * len(msgs) + [-1, -1]
+
+
+@pytest.mark.parametrize("count", [608, 609])
+def test_message_warps_batch_limit(engine, count):
+    """the last batch with a warp a message and the first with a thread each"""
+    sid = engine.set_id("sha256-128f-simple")
+    pks, sks, msgs = _requests(engine, sid, count, 5, 13)
+    sigs, st = engine.sign_batch(sid, sks, msgs)
+    assert not any(st)
+    assert sigs == _in_pieces(engine, sid, sks, msgs)
+    assert sigs[-1] == _oracle("sha256-128f-simple").sign(msgs[-1], sks[-1])
+    assert not any(engine.verify_batch(sid, pks, msgs, sigs))
