@@ -13,7 +13,7 @@ signatures inside every timed step, streamed over two batch objects (step i
 launches while step i-1's signatures copy back); `e2e.serial` is the same
 one call at a time.  Verify throughput, the plain
 one-signature-per-call path and the roofline of the dominant kernel
-(k_leaves) ride along on the same JSON line.
+(k_leaf_chains) ride along on the same JSON line.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -344,10 +344,8 @@ def main():
             tj = json.load(f)
         traffic = tj.get("dram_bytes_per_launch_scaled_to_4096")
 
-    # ---- verify at 16384 items (4 copies of the batch): batch parallelism
-    # beside kernel quality -- the persistent kernel keeps ~4 warps per SM
-    # busy per 600 items, and the ALU pipe needs ~8 warps per SM
-    # (cuspx_cmp_rate) ----
+    # ---- verify at 16384 items (4 copies of the batch): the kernels with
+    # enough items to fill the GPU between the layers ----
     verify16k = None
     if rank == 0:
         big = 4 * BATCH
