@@ -190,9 +190,10 @@ struct Family {
                                     (const void *)k_verify_block<HF, 8>};
             for (const void *f : blocks)
                 if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
-            if ((e = cudaFuncSetAttribute(k_vsort_layer_group<HF, kGroupLanes>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, big)))
-                return e;
+            const void *layer[] = {(const void *)k_vsort_layer_group<HF, kGroupLanes>,
+                                   (const void *)k_vsort_layer_group<HF, 4>};
+            for (const void *f : layer)
+                if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         }
         if ((e = cudaFuncSetAttribute(k_fors_pk<HF>, cudaFuncAttributeMaxDynamicSharedMemorySize, big))) return e;
         // Load every other kernel of the family now: with lazy module loading
@@ -446,6 +447,27 @@ struct Family {
     static constexpr int kGroupLanes = 8;
     static constexpr uint32_t kGroupItems = HF::kShake ? (HF::kRobust ? 8192 : 2048) : (HF::kRobust ? 4096 : 2048);
 
+    // SHA-256 batches of several item groups with lanes in the layer kernel as
+    // well: it then ends before the other groups' chains do, and still leaves
+    // them more of the SMs than 8 lanes would.  Returns the lanes an item (0:
+    // none of these batches) and how many groups at most.  Simple f sets, 4
+    // lanes: 128f 2048 items 1.384 ms (one group of 8 lanes 1.461), 4096 2.161
+    // (a thread an item 2.20), 8192 3.586 / 3.649, but 12000 4.97 / 4.85; 192f
+    // 3000 items 2.71 / 3.01; 256f 3000 2.95 / 3.22, but 4096 3.77 / 3.68; the
+    // s sets, whose layers are few, lose (128s, 4096: 0.90 / 0.86).  Robust
+    // sets, whose H masks the lanes share out, in two groups, 8 lanes at n = 32
+    // (256f 3000 items 6.69 / 7.22, 8192 16.6 / 17.9; 256s 3000 3.51 / 3.89,
+    // but 2048 2.76 / 2.62) and 4 at n < 32 (192f 6000 items 8.80 / 10.3, 12000
+    // 17.1 / 18.9; 128f 8192 7.30 / 7.73, but 4096 4.39 / 4.11; 192s 4200 2.56
+    // / 3.30), up to 32768 items, the largest measured.
+    static int side_lanes(const SetParams &P, uint32_t count, int &groups) {
+        if (HF::kShake) return 0;
+        if (!HF::kRobust) return P.d > 8 && count >= 1500 && count <= (N < 32 ? 8192u : 3072u) ? 4 : 0;
+        if (N == 32 ? count < 3000 : count <= 4096) return 0;
+        groups = 2;
+        return N == 32 ? 8 : 4;
+    }
+
     // verify_mode 3: per group of items, T_k then per layer the sorted
     // chains and the layer roots (spx_vsort.cuh).  Groups run on their own
     // streams; a group's chain kernel of layer L starts after the previous
@@ -455,11 +477,14 @@ struct Family {
     static void verify_sorted(const SetParams &P, const VerifyArgs &A, const Tuning &tu, cudaStream_t s,
                               PhaseTimer *pt, const VerifyLists &V, const VerifyFork *vf) {
         constexpr int LEN = 2 * N + 3;
-        const bool grouped = A.count <= kGroupItems && (!HF::kShake || !HF::kRobust || V.masks);
-        const bool one = grouped && (!HF::kShake || A.count <= 4u * (uint32_t)device_sms());
-        int G = one || tu.verify_groups < 1 ? 1 : tu.verify_groups;
         const int gmax = pt || !vf ? 1 : vf->sides + 1;
+        int G = tu.verify_groups < 1 ? 1 : tu.verify_groups;
         if (G > gmax) G = gmax;
+        int most = G;
+        const int side = G > 1 ? side_lanes(P, A.count, most) : 0;
+        if (G > most) G = most;
+        const bool grouped = side > 0 || (A.count <= kGroupItems && (!HF::kShake || !HF::kRobust || V.masks));
+        if (!side && grouped && (!HF::kShake || A.count <= 4u * (uint32_t)device_sms())) G = 1;
         if ((uint32_t)G > A.count) G = (int)A.count;
         const uint32_t per = (A.count + G - 1) / G;
         G = (int)((A.count + per - 1) / per);
@@ -476,6 +501,12 @@ struct Family {
                 }
             }
             if constexpr (!HF::kShake) {
+                if (side == 4) {
+                    constexpr int kItems = 16;
+                    k_vsort_layer_group<HF, 4>
+                        <<<ceil_div(n, kItems), 64, kItems * ShaGroup<HF>::kStride * 4, st>>>(P, A, V, L, first, n, g);
+                    return;
+                }
                 if (grouped) {
                     constexpr int kItems = 64 / kGroupLanes;
                     k_vsort_layer_group<HF, kGroupLanes>

@@ -98,3 +98,14 @@ def test_speculative_walk(engine, pool, setname):
             _check(engine, sid, pool(setname), count, count)
     finally:
         engine.set_tuning(sid, **saved)
+
+
+@pytest.mark.parametrize("setname,counts", [("sha256-128f-simple", (1499, 1500, 8192, 8193)),
+                                            ("sha256-192f-simple", (1500, 3001)),
+                                            ("sha256-256f-simple", (3072, 3073)),
+                                            ("sha256-128f-robust", (4097,)), ("sha256-192s-robust", (4097,)),
+                                            ("sha256-256s-robust", (2999, 3000)), ("sha256-256f-robust", (3001,))])
+def test_lanes_in_item_groups(engine, pool, setname, counts):
+    """the sizes between which several item groups run with lanes in the layer kernel"""
+    for count in counts:
+        _check(engine, engine.set_id(setname), pool(setname), count, count)
