@@ -125,30 +125,12 @@ struct VerifySha2 : VerifySlot<4 * HF::W, 22, 64> {
     SPX_DEV static void put16(uint32_t *base, int byte_off, uint32_t v) {
         reinterpret_cast<uint16_t *>(base)[byte_off >> 1] = (uint16_t)v;
     }
-    // value c (big-endian words) at stream byte 22 + c n
-    SPX_DEV static void write_value(uint32_t *stream, int c, const uint32_t v[W]) {
-        const int off = 22 + c * N;
-        put16(stream, off, __byte_perm(v[0], 0, 0x0023));
-#pragma unroll
-        for (int i = 0; i + 1 < W; i++) stream[(off + 2) / 4 + i] = __byte_perm(v[i], v[i + 1], 0x6701);
-        put16(stream, off + N - 2, __byte_perm(v[W - 1], 0, 0x0001));
-    }
-    SPX_DEV static void read_value(const uint32_t *stream, int c, uint32_t v[W]) {
-        const int w0 = (20 + c * N) / 4;
-#pragma unroll
-        for (int i = 0; i < W; i++) v[i] = __byte_perm(stream[w0 + i], stream[w0 + i + 1], 0x2345);
-    }
     // value bytes 8q .. 8q+7 (memory order) to stream byte 22 + 8q
     SPX_DEV static void put_value_word(uint32_t *stream, int q, uint2 x) {
         const int o = 22 + 8 * q;
         put16(stream, o, x.x);
         stream[(o + 2) / 4] = __byte_perm(x.x, x.y, 0x5432);
         put16(stream, o + 6, x.y >> 16);
-    }
-    // `bytes` (multiple of 8) from 8-byte aligned global memory to stream
-    // byte 22 onwards, warp-cooperatively
-    SPX_DEV static void copy_values(uint32_t *stream, const uint8_t *src, int bytes, uint32_t lane) {
-        for (int q = lane; q < bytes / 8; q += 32) put_value_word(stream, q, reinterpret_cast<const uint2 *>(src)[q]);
     }
     // ADRS_c prefix and the padding after m values (the length counts the
     // 64-byte midstate block)
@@ -169,32 +151,11 @@ struct VerifySha2 : VerifySlot<4 * HF::W, 22, 64> {
         if (lane < 8) S[B::S_KEY + lane] = wk->mid[lane];
     }
 
-    SPX_DEV static void claim_chain(LaneRegs &r, const uint32_t *S) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) r.kmid[i] = S[B::S_KEY + i];
-    }
     SPX_DEV static void claim_t(LaneRegs &r, uint32_t *S, int) {
 #pragma unroll
         for (int i = 0; i < 8; i++) r.kmid[i] = r.tst[i] = S[B::S_KEY + i];
     }
 
-    SPX_DEV static void build_chain(Unit &u, const LaneRegs &r, const uint32_t *S, int c, int s, int,
-                                    const uint32_t v[W]) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) u.st[i] = r.kmid[i];
-        u.blk[0] = S[B::S_AW0];
-        u.blk[1] = S[B::S_AW1];
-        u.blk[2] = S[B::S_AW2];
-        u.blk[3] = S[B::S_IDXL] << 16;
-        u.blk[4] = (uint32_t)c << 16;
-        u.blk[5] = ((uint32_t)s << 16) | (v[0] >> 16);
-#pragma unroll
-        for (int i = 1; i < W; i++) u.blk[5 + i] = __funnelshift_l(v[i], v[i - 1], 16);
-        u.blk[5 + W] = (v[W - 1] << 16) | 0x8000u;
-#pragma unroll
-        for (int i = 6 + W; i < 15; i++) u.blk[i] = 0;
-        u.blk[15] = (64 + 22 + N) * 8;
-    }
     SPX_DEV static void build_t(Unit &u, const LaneRegs &r, uint32_t *S, int j, int) {
         const uint32_t *b = S + B::S_HDR + j * 16;
 #pragma unroll
@@ -247,12 +208,6 @@ struct VerifySha2 : VerifySlot<4 * HF::W, 22, 64> {
 #pragma unroll
             for (int i = 0; i < 16; i++) u.blk[i] = m[16 * (kHBlocks - 1) + i];
         }
-    }
-    SPX_DEV static void build_idle(Unit &u) {
-#pragma unroll
-        for (int i = 0; i < 8; i++) u.st[i] = 0;
-#pragma unroll
-        for (int i = 0; i < 16; i++) u.blk[i] = 0;
     }
     SPX_DEV static void run(Unit &u) {
 #pragma unroll
@@ -646,28 +601,6 @@ struct VerifySha2Robust : VerifySha2<HF> {
         }
     }
 
-    SPX_DEV static void build_chain(Unit &u, const LaneRegs &r, const uint32_t *S, int c, int s, int sub,
-                                    const uint32_t v[W]) {
-        if (sub < kMB) {
-            const uint32_t aw[6] = {S[B::S_AW0], S[B::S_AW1], S[B::S_AW2], S[B::S_IDXL] << 16,
-                                    (uint32_t)c << 16, (uint32_t)s << 16};
-            mask_unit(u, S, aw, 0, sub, r.tst);
-        } else {
-            uint32_t x[W];
-#pragma unroll
-            for (int i = 0; i < W; i++) x[i] = v[i] ^ r.mk[i];
-            S0::build_chain(u, r, S, c, s, 0, x);
-        }
-    }
-    SPX_DEV static void after_f_unit(const Unit &u, LaneRegs &r, int sub) {
-        if (sub < kMB - 1) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) r.tst[i] = u.out[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < W; i++) r.mk[i] = u.out[i];
-        }
-    }
 
     // H of compute_root at height h -> h + 1 for node index idx; sub: mask
     // units first, then the H blocks
