@@ -89,7 +89,8 @@ typedef struct {
     int verify_groups;    /* sorted verify: the batch is split into this many groups of items
                              (1..8), each on its own stream, so that one group's serial T_len
                              and auth-path kernel overlaps another group's chains (one group for
-                             small batches, at most two for robust SHA-256) */
+                             small batches, at most two or four for SHA-256 batches with several lanes an
+                             item) */
     int verify_sorted_min;/* verify batches of at least this many items run the sorted layered
                              verify whatever verify_mode says (0: only with verify_mode 3);
                              batches up to verify_item_max still run one item per block */
