@@ -119,6 +119,19 @@ struct TuneEntry {
 };
 constexpr int kMaxTuneEntries = 16;
 
+// everything a captured launch sequence of a batch has baked into it
+struct GraphKey {
+    size_t count;
+    bool keyrow, aux, siglen, long_msgs;
+    const uint8_t *keys, *packed;
+    Tuning tune;
+    bool operator==(const GraphKey &o) const {
+        return count == o.count && keyrow == o.keyrow && aux == o.aux && siglen == o.siglen &&
+               long_msgs == o.long_msgs && keys == o.keys && packed == o.packed &&
+               memcmp(&tune, &o.tune, sizeof(Tuning)) == 0;
+    }
+};
+
 struct cuspx_ctx {
     int device = 0;
     std::mutex err_mu;   // err is written by any calling thread
@@ -141,9 +154,7 @@ struct cuspx_ctx {
     // multi-batch (mixed parameter set) graphs
     struct GroupGraph {
         std::vector<cuspx_batch *> batches;
-        std::vector<size_t> counts;
-        std::vector<bool> long_msgs;
-        std::vector<Tuning> tunes;
+        std::vector<GraphKey> keys;
         cudaGraphExec_t exec;
         cudaStream_t origin;
         cudaEvent_t e0, e1;
@@ -199,19 +210,8 @@ struct cuspx_batch {
     size_t packed_cap = 0;
     const uint8_t *bound_keys = nullptr;   // external device key table (not owned)
     size_t bound_nkeys = 0;
-    // captured launch sequences keyed by everything baked into them; an item
-    // count seen for the first time launches directly and is captured on
-    // its second use
-    struct GraphKey {
-        size_t count;
-        bool keyrow, aux, siglen, long_msgs;
-        const uint8_t *keys, *packed;
-        Tuning tune;
-        bool operator==(const GraphKey &o) const {
-            return count == o.count && keyrow == o.keyrow && aux == o.aux && siglen == o.siglen &&
-                   long_msgs == o.long_msgs && keys == o.keys && packed == o.packed && memcmp(&tune, &o.tune, sizeof(Tuning)) == 0;
-        }
-    };
+    // captured launch sequences; an item count seen for the first time launches
+    // directly and is captured on its second use
     struct GraphEntry {
         GraphKey key;
         cudaGraphExec_t exec;
@@ -624,6 +624,11 @@ extern "C" {
 // ---------------------------------------------------------------------------
 // batches
 // ---------------------------------------------------------------------------
+static GraphKey graph_key(const cuspx_batch *b) {
+    return GraphKey{b->count, b->use_keyrow, b->use_aux, b->use_siglen, b->long_msgs, b->bound_keys, b->packed,
+                    effective_tuning(b->ctx, b->set, b->op, b->count)};
+}
+
 // bytes of one layer's masks of an item (robust SHAKE, ShakeGroup::mask_lanes)
 static size_t shake_mask_bytes(const SetParams &P) { return (size_t)(P.len + 2 * P.hp) * P.n; }
 
@@ -1011,8 +1016,7 @@ int cuspx_batch_run(cuspx_batch *b) {
         b->ran = true;
         return CUSPX_OK;
     }
-    const Tuning &tu = effective_tuning(ctx, b->set, b->op, b->count);
-    cuspx_batch::GraphKey key{b->count, b->use_keyrow, b->use_aux, b->use_siglen, b->long_msgs, b->bound_keys, b->packed, tu};
+    const GraphKey key = graph_key(b);
     b->use_clock++;
     cuspx_batch::GraphEntry *hit = nullptr;
     for (auto &g : b->graphs)
@@ -1562,21 +1566,13 @@ int cuspx_group_run(cuspx_ctx *ctx, cuspx_batch *const *batches, int nb, float *
     for (auto &g : ctx->groups) {
         if ((int)g.batches.size() != nb) continue;
         bool same = true;
-        for (int i = 0; i < nb && same; i++) {
-            cuspx_batch *b = batches[i];
-            same = g.batches[i] == b && g.counts[i] == b->count && g.long_msgs[i] == b->long_msgs &&
-                   memcmp(&g.tunes[i], &effective_tuning(ctx, b->set, b->op, b->count), sizeof(Tuning)) == 0;
-        }
+        for (int i = 0; i < nb && same; i++) same = g.batches[i] == batches[i] && g.keys[i] == graph_key(batches[i]);
         if (same) hit = &g;
     }
     if (!hit) {
         cuspx_ctx::GroupGraph gg;
         gg.batches.assign(batches, batches + nb);
-        for (int i = 0; i < nb; i++) {
-            gg.counts.push_back(batches[i]->count);
-            gg.long_msgs.push_back(batches[i]->long_msgs);
-            gg.tunes.push_back(effective_tuning(ctx, batches[i]->set, batches[i]->op, batches[i]->count));
-        }
+        for (int i = 0; i < nb; i++) gg.keys.push_back(graph_key(batches[i]));
         CK(cudaStreamCreateWithFlags(&gg.origin, cudaStreamNonBlocking), ctx);
         cudaEventCreate(&gg.e0);
         cudaEventCreate(&gg.e1);
