@@ -13,6 +13,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -132,6 +133,37 @@ struct GraphKey {
     }
 };
 
+// Captured multi-batch (mixed parameter set) launches of a context.  They hold
+// their batches' device pointers, so a batch takes its graphs with it when it
+// goes; batches share ownership because they may outlive the context.
+struct GroupGraphs {
+    struct Entry {
+        std::vector<cuspx_batch *> batches;
+        std::vector<GraphKey> keys;
+        cudaGraphExec_t exec;
+        cudaStream_t origin;
+        cudaEvent_t e0, e1;
+        void destroy() {
+            cudaStreamSynchronize(origin);
+            cudaGraphExecDestroy(exec);
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            cudaStreamDestroy(origin);
+        }
+    };
+    std::mutex mu;
+    std::vector<Entry> list;
+    // the graphs that b is in, or all of them (null)
+    void drop(const cuspx_batch *b) {
+        std::lock_guard<std::mutex> lk(mu);
+        auto keep = std::stable_partition(list.begin(), list.end(), [&](const Entry &g) {
+            return b && std::find(g.batches.begin(), g.batches.end(), b) == g.batches.end();
+        });
+        for (auto it = keep; it != list.end(); ++it) it->destroy();
+        list.erase(keep, list.end());
+    }
+};
+
 struct cuspx_ctx {
     int device = 0;
     std::mutex err_mu;   // err is written by any calling thread
@@ -151,16 +183,7 @@ struct cuspx_ctx {
     cuspx_batch *oneshot[3][kNumSets] = {};
     uint8_t *stage = nullptr;   // pinned staging of the one-shot calls (under mu)
     size_t stage_cap = 0;
-    // multi-batch (mixed parameter set) graphs
-    struct GroupGraph {
-        std::vector<cuspx_batch *> batches;
-        std::vector<GraphKey> keys;
-        cudaGraphExec_t exec;
-        cudaStream_t origin;
-        cudaEvent_t e0, e1;
-    };
-    std::vector<GroupGraph> groups;
-    std::mutex group_mu;
+    std::shared_ptr<GroupGraphs> groups = std::make_shared<GroupGraphs>();
 };
 
 struct ProfEntry {
@@ -171,6 +194,7 @@ struct ProfEntry {
 
 struct cuspx_batch {
     cuspx_ctx *ctx = nullptr;
+    std::shared_ptr<GroupGraphs> groups;   // the context's
     int op = 0, set = 0;
     SetParams P{};
     size_t cap = 0, msg_cap = 0, key_cap = 0;
@@ -363,13 +387,7 @@ int cuspx_create(int device, cuspx_ctx **out) {
 
 void cuspx_destroy(cuspx_ctx *ctx) {
     if (!ctx) return;
-    for (auto &g : ctx->groups) {
-        cudaStreamSynchronize(g.origin);
-        cudaGraphExecDestroy(g.exec);
-        cudaEventDestroy(g.e0);
-        cudaEventDestroy(g.e1);
-        cudaStreamDestroy(g.origin);
-    }
+    ctx->groups->drop(nullptr);
     for (auto &row : ctx->oneshot)
         for (auto *b : row)
             if (b) cuspx_batch_destroy(b);
@@ -661,6 +679,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
     }
     cuspx_batch *b = new cuspx_batch();
     b->ctx = ctx;
+    b->groups = ctx->groups;
     b->op = op;
     b->set = set;
     b->P = make_params(sd);
@@ -770,6 +789,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
 void cuspx_batch_destroy(cuspx_batch *b) {
     if (!b) return;
     if (b->s) cudaStreamSynchronize(b->s);
+    if (b->groups) b->groups->drop(b);
     for (auto &g : b->graphs) cudaGraphExecDestroy(g.exec);
     for (void *p : b->allocs) cudaFree(p);
     if (b->e0) cudaEventDestroy(b->e0);
@@ -1557,20 +1577,21 @@ int cuspx_group_run(cuspx_ctx *ctx, cuspx_batch *const *batches, int nb, float *
         if (!batches[i] || batches[i]->ctx != ctx || batches[i]->profile)
             return fail(ctx, CUSPX_EINVAL, "group_run: batch missing, from another context, or profiling");
     CK(cudaSetDevice(ctx->device), ctx);
-    std::lock_guard<std::mutex> lk(ctx->group_mu);
+    auto &groups = ctx->groups->list;
+    std::lock_guard<std::mutex> lk(ctx->groups->mu);
     // the batches' uploads (on their own streams) must be complete before the
     // streams join a capture or the graph reads their buffers
     for (int i = 0; i < nb; i++) CK(cudaStreamSynchronize(batches[i]->s), ctx);
     for (int i = 0; i < nb; i++) spec_scratch(batches[i]);
-    cuspx_ctx::GroupGraph *hit = nullptr;
-    for (auto &g : ctx->groups) {
+    GroupGraphs::Entry *hit = nullptr;
+    for (auto &g : groups) {
         if ((int)g.batches.size() != nb) continue;
         bool same = true;
         for (int i = 0; i < nb && same; i++) same = g.batches[i] == batches[i] && g.keys[i] == graph_key(batches[i]);
         if (same) hit = &g;
     }
     if (!hit) {
-        cuspx_ctx::GroupGraph gg;
+        GroupGraphs::Entry gg;
         gg.batches.assign(batches, batches + nb);
         for (int i = 0; i < nb; i++) gg.keys.push_back(graph_key(batches[i]));
         CK(cudaStreamCreateWithFlags(&gg.origin, cudaStreamNonBlocking), ctx);
@@ -1597,17 +1618,12 @@ int cuspx_group_run(cuspx_ctx *ctx, cuspx_batch *const *batches, int nb, float *
         cudaError_t ie = cudaGraphInstantiate(&gg.exec, graph, 0);
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) return cuda_fail(ctx, ie, "group cudaGraphInstantiate");
-        if (ctx->groups.size() >= 16) {
-            auto &old = ctx->groups.front();
-            cudaStreamSynchronize(old.origin);
-            cudaGraphExecDestroy(old.exec);
-            cudaEventDestroy(old.e0);
-            cudaEventDestroy(old.e1);
-            cudaStreamDestroy(old.origin);
-            ctx->groups.erase(ctx->groups.begin());
+        if (groups.size() >= 16) {
+            groups.front().destroy();
+            groups.erase(groups.begin());
         }
-        ctx->groups.push_back(gg);
-        hit = &ctx->groups.back();
+        groups.push_back(gg);
+        hit = &groups.back();
     }
     CK(cudaEventRecord(hit->e0, hit->origin), ctx);
     CK(cudaGraphLaunch(hit->exec, hit->origin), ctx);

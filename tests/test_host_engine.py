@@ -126,3 +126,53 @@ def test_group_run_reads_bound_keys_and_lengths(engine, fake):
         b.download(None, None, st)
         assert list(st) == want
     b.close()
+
+
+def test_group_graphs_go_with_their_batches(engine, fake):
+    """a graph launches into its batches' memory: none may be left, and none
+    found for a new batch at the old one's address, once a batch is gone"""
+    c, live = fake, fake.lib().fake_live_execs
+    sid = [engine.set_id(s) for s in SETS]
+    bs = [engine.batch(c.OP_SIGN, s, 4, 4096, 4) for s in sid]
+    for count in (2, 3, 4):
+        for k in range(2):
+            _upload(c, bs[k], count, _rows(c.set_sizes(sid[k])["sk"], count, k))
+        c.group_run(engine, bs)
+        c.group_run(engine, bs[1:])
+    assert live() == 6
+    bs[0].close()
+    assert live() == 3
+    c.group_run(engine, bs[1:])
+    assert live() == 3
+    bs[1].close()
+    assert live() == 0
+
+
+def test_mixed_signer_grows_and_shrinks(engine, fake):
+    """batches that are replaced by larger ones, then used at the old sizes"""
+    c = fake
+    ms = c.MixedSigner(engine)
+    sid = [engine.set_id(s) for s in SETS]
+    for step, count in enumerate((10, 20, 10, 10, 20, 33, 10, 20)):
+        sks, msgs = [], []
+        for k in range(2):
+            sks += [r.tobytes() for r in _rows(c.set_sizes(sid[k])["sk"], count, 10 * step + k)]
+            msgs += [b"%d" % i for i in range(count)]
+        ids = [sid[0]] * count + [sid[1]] * count
+        sigs, status, _ = ms.sign(ids, sks, msgs)
+        for s, sk, sig, st in zip(ids, sks, sigs, status):
+            n = c.set_sizes(s)["n"]
+            assert st == 0 and sig[:n] == b"\xad" * n and sig[n:2 * n] == sk[n:2 * n]
+    ms.close()
+    assert c.lib().fake_live_execs() == 0
+
+
+def test_batches_outlive_their_engine(fake):
+    c = fake
+    eng = c.Engine(0)
+    b = eng.batch(c.OP_SIGN, eng.set_id(SETS[0]), 4, 4096, 4)
+    _upload(c, b, 2, _rows(c.set_sizes(b.sid)["sk"], 2, 1))
+    c.group_run(eng, [b])
+    eng.close()
+    b.close()
+    assert c.lib().fake_live_execs() == 0 and c.lib().fake_faults() == 0
