@@ -1369,6 +1369,7 @@ static bool upload_packed(cuspx_batch *b, size_t count, const uint8_t *in, size_
 
 static int oneshot_run(cuspx_ctx *ctx, int op, int set, const std::vector<OneshotJob *> &jobs) {
     std::lock_guard<std::mutex> lk(ctx->mu);
+    CK(cudaSetDevice(ctx->device), ctx);   // any thread may call
     size_t count = 0, total = 0;
     bool any_opt = false;
     for (const OneshotJob *j : jobs) {

@@ -176,3 +176,34 @@ def test_batches_outlive_their_engine(fake):
     eng.close()
     b.close()
     assert c.lib().fake_live_execs() == 0 and c.lib().fake_faults() == 0
+
+
+def test_oneshot_memory_is_on_the_engines_device(fake):
+    """calls from threads whose current device is another one (each new
+    thread's is device 0), whose packed input grows with and without a new batch"""
+    c = fake
+    c.lib().cudaSetDevice(0)
+    eng = c.Engine(1)
+    sid = eng.set_id(SETS[0])
+    z = c.set_sizes(sid)
+    res = []
+
+    def call(count, size):
+        msgs = [b"m" * size] * count
+        c.lib().cudaSetDevice(0)
+        sks = [r.tobytes() for r in _rows(z["sk"], count, count)]
+        opt = [r.tobytes() for r in _rows(z["n"], count, 99)]
+        sigs, st = eng.sign_batch(sid, sks, msgs, opt)
+        ok = list(st) == [0] * count and [s[:z["n"]] for s in sigs] == opt
+        got = eng.verify_batch(sid, [s[z["n"]:2 * z["n"]] + bytes(z["n"]) for s in sigs], msgs, sigs)
+        res.append(ok and list(got) == [0] * count)
+
+    try:
+        for count, size in ((5, 40), (3, 0), (5, 800), (9, 40), (70, 100), (2, 3000), (70, 112)):
+            t = threading.Thread(target=call, args=(count, size))
+            t.start()
+            t.join()
+        assert res == [True] * 7 and c.lib().fake_faults() == 0
+    finally:
+        eng.close()
+        c.lib().cudaSetDevice(0)
