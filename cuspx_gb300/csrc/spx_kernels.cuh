@@ -160,7 +160,8 @@ SPX_DEV void layer_index(const SetParams &P, uint64_t tree, uint32_t idx_leaf, i
     }
 }
 
-// whether items i and r sign under the same key (the seeds decide every tree)
+// whether items i and r sign under the same key: the seeds, which decide every
+// tree, and the root, which share_insert looks keys up by
 template <int N>
 SPX_DEV bool same_key(const KeyRef &sk, uint32_t i, uint32_t r) {
     const uint64_t *x = reinterpret_cast<const uint64_t *>(sk.row(i));
@@ -168,20 +169,31 @@ SPX_DEV bool same_key(const KeyRef &sk, uint32_t i, uint32_t r) {
     bool eq = true;
     if (x != y) {
 #pragma unroll
-        for (int j = 0; j < N / 8; j++) eq &= x[j] == y[j] && x[2 * N / 8 + j] == y[2 * N / 8 + j];
+        for (int j = 0; j < 4 * N / 8; j++)
+            if (j / (N / 8) != 1) eq &= x[j] == y[j];
     }
     return eq;
 }
 // The item that item i's tree of `layer` is kept under: the first to come into
 // the layer's table with that tree and key.  The table is at most half full,
-// so a probe ends.
+// so a probe ends.  Its start is a hash of the tree and of every word of the
+// public key (PUB_SEED and ROOT, the row's second half): addresses do not
+// depend on secrets, and keys spread over the table however alike their seeds
+// are.  (From the first word of SK_SEED, 4096 keys alike in it all walked one
+// run of the table for layer d-1, whose tree is 0 for every item: 4.1 ms at
+// 128f, random keys 0.043.)
 template <int N>
 SPX_DEV uint32_t share_insert(const SetParams &P, const ShareArgs &S, const KeyRef &sk, const SignWork *work,
                               int layer, uint64_t tree, uint32_t i) {
     uint32_t *tab = S.tab + (uint64_t)(layer + 1 - S.layer0) * (S.mask + 1);
-    const uint32_t k = *reinterpret_cast<const uint32_t *>(sk.row(i));
-    uint32_t h = ((uint32_t)tree ^ (uint32_t)(tree >> 32) * 0x85ebca6bu ^ k) * 0x9e3779b1u;
-    h ^= h >> 15;
+    const uint64_t *pk = reinterpret_cast<const uint64_t *>(sk.row(i) + 2 * N);
+    uint64_t g = tree;
+#pragma unroll
+    for (int j = 0; j < 2 * N / 8; j++) {
+        g = (g ^ pk[j]) * 0x9e3779b97f4a7c15ull;
+        g ^= g >> 32;
+    }
+    uint32_t h = (uint32_t)g;
     for (uint32_t n = 0; n <= S.mask; n++, h++) {
         const uint32_t e = atomicCAS(tab + (h & S.mask), 0u, i + 1);
         if (e == 0) break;

@@ -209,3 +209,44 @@ def test_message_warps_batch_limit(engine, count):
     assert sigs == _in_pieces(engine, sid, sks, msgs)
     assert sigs[-1] == _oracle("sha256-128f-simple").sign(msgs[-1], sks[-1])
     assert not any(engine.verify_batch(sid, pks, msgs, sigs))
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-128f-simple", 4096), ("shake256-192f-robust", 300)])
+@pytest.mark.parametrize("part", [0, 2])
+def test_shared_trees_of_keys_with_alike_seeds(engine, setname, count, part):
+    """a key per item whose seeds differ in the last two bytes of SK_SEED or of
+    PUB_SEED alone: the search for trees that items share takes no longer than
+    with random seeds (five times as long at most, where a walk over all the
+    batch's keys takes ten to a hundred times) and the signatures are the keys' own"""
+    import numpy as np
+    import cuspx_gb300 as c
+    rng = random.Random(14)
+    sid = engine.set_id(setname)
+    z = c.set_sizes(sid)
+    n = z["n"]
+    base = rng.randbytes(3 * n)
+    alike = [base[:(part + 1) * n - 2] + i.to_bytes(2, "big") + base[(part + 1) * n:] for i in range(count)]
+    apart = [rng.randbytes(3 * n) for _ in range(count)]
+    msgs = [rng.randbytes(20) for _ in range(count)]
+    slab, offs, lens = c.pack_messages(msgs)
+    b = engine.batch(c.OP_SIGN, sid, count, len(slab), count)
+    b.profile()
+    took = []
+    for seeds in (apart, alike):
+        pks, sks = engine.keypair_batch(sid, seeds)
+        best = None
+        for _ in range(4):
+            b.upload(count, b"".join(sks), count, None, slab, len(slab), offs, lens)
+            b.profile()
+            b.run()
+            ms = dict((k, t) for k, t, _ in b.kernel_ms())["k_share"]
+            best = ms if best is None else min(best, ms)
+        took.append(best)
+    out, st = np.zeros(count * z["sig"], np.uint8), np.zeros(count, np.int32)
+    b.download(out, None, st)
+    b.close()
+    assert not st.any()
+    sigs = [out[i * z["sig"]:(i + 1) * z["sig"]].tobytes() for i in range(count)]
+    assert sigs[:60] == _in_pieces(engine, sid, sks[:60], msgs[:60])
+    assert sigs[-1] == _oracle(setname).sign(msgs[-1], sks[-1])
+    assert took[1] < 5 * took[0], took
