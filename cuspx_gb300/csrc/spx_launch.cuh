@@ -26,7 +26,9 @@ struct Tuning {
                              // 2 persistent hypertree kernel, 3 layered with sorted chains
     int fors_lanes_log2 = 5; // lanes per FORS tree = 2^g (0: lane per tree, 5: warp per tree)
     int tree_mode = 0;       // 0 warp per XMSS tree, 1 lane per tree (subtrees of height <= 4)
-    int chain_mode_max = 64; // batches of at most this many items run XMSS leaves chain-parallel
+    int chain_mode_max = 64; // sign batches of at most this many items take the T_len kernel of the
+                             // lower latency; 0: XMSS leaves a lane each (up to kChainModeItems, and
+                             // key generation)
     int verify_slots = 4;    // most items per warp in the persistent verify kernel
     int verify_item_max = 0; // batches of at most this many items verify one item per block
     int verify_claim_min = 1;// persistent verify: free lanes before chains are handed out
@@ -116,6 +118,11 @@ inline uint32_t share_table(uint64_t count) {
     while (n < 2 * count) n *= 2;
     return n;
 }
+
+// Sign batches that chain_mode_max decides about.  Larger ones always run a
+// lane per WOTS+ chain and look for shared trees (1024 signatures of 128f:
+// 5.38 ms, a lane per leaf 5.99).
+constexpr uint32_t kChainModeItems = 256;
 
 inline unsigned ceil_div(uint64_t a, uint64_t b) { return (unsigned)((a + b - 1) / b); }
 
@@ -379,8 +386,9 @@ struct Family {
                 CUSPX_MARK(pt, "k_sign_msg_wide", s);
             }
         }
-        // (k_leaves, without chain-end scratch, computes every item's trees)
-        A.share.layer0 = A.ends_trees && tu.chain_mode_max > 0 ? share_layer(P, A.count, tu, A.share) : 0;
+        // (k_leaves computes every item's trees)
+        if (tu.chain_mode_max <= 0 && A.count <= kChainModeItems) A.ends_trees = 0;
+        A.share.layer0 = A.ends_trees ? share_layer(P, A.count, tu, A.share) : 0;
         if (A.share.layer0) {
             const int tabs = P.d - A.share.layer0 + 1;
             A.share.mask = share_table(A.count) - 1;
@@ -414,8 +422,8 @@ struct Family {
         if (split) cudaEventRecord(fk->join, sf);
         {
             LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false, A.share, nullptr};
-            leaves(P, L, tu, s, pt, tu.chain_mode_max > 0 ? A.ends_trees : 0,
-                   A.count <= (uint32_t)tu.chain_mode_max && A.count <= 256);
+            leaves(P, L, tu, s, pt, A.ends_trees,
+                   A.count <= (uint32_t)tu.chain_mode_max && A.count <= kChainModeItems);
         }
         {
             TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig, A.share, nullptr};

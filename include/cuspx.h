@@ -74,9 +74,10 @@ typedef struct {
                              3 layered kernels with each layer's WOTS+ chains sorted by length */
     int fors_lanes_log2;  /* lanes per FORS tree = 2^g, g in 0..5 (0: lane per tree, 5: warp per tree) */
     int tree_mode;        /* 0 warp per XMSS subtree, 1 lane per subtree (heights <= 4 only) */
-    int chain_mode_max;   /* 0: XMSS leaves one lane per leaf.  Otherwise one lane per WOTS+
-                             chain, batches of at most this many signatures (up to 256) with
-                             the T_len kernel of the lower latency */
+    int chain_mode_max;   /* 0: XMSS leaves one lane per leaf, in key generation and in batches of
+                             up to 256 signatures.  Otherwise, and in larger batches, one lane
+                             per WOTS+ chain; batches of at most this many signatures (up to
+                             256) with the T_len kernel of the lower latency */
     int verify_slots;     /* SHAKE: most items a warp holds at once in verify_mode 2 (1..8);
                              batches below about 4 warps per SM use fewer */
     int verify_item_max;  /* verify batches of at most this many items (any verify_mode) in one

@@ -250,3 +250,30 @@ def test_shared_trees_of_keys_with_alike_seeds(engine, setname, count, part):
     assert sigs[:60] == _in_pieces(engine, sid, sks[:60], msgs[:60])
     assert sigs[-1] == _oracle(setname).sign(msgs[-1], sks[-1])
     assert took[1] < 5 * took[0], took
+
+
+@pytest.mark.parametrize("count,kernel", [(256, "k_leaves"), (257, "k_leaf_chains")])
+def test_chain_mode_max_decides_up_to_256_items(engine, count, kernel):
+    """chain_mode_max 0, as tuning files may hold it for any batch size: a lane
+    per leaf where the knob decides, chain lanes and shared trees above"""
+    import numpy as np
+    import cuspx_gb300 as c
+    sid = engine.set_id("sha256-128f-simple")
+    z = c.set_sizes(sid)
+    pks, sks, msgs = _requests(engine, sid, count, 1, 15)
+    slab, offs, lens = c.pack_messages(msgs)
+    saved = engine.get_tuning(sid)
+    b = engine.batch(c.OP_SIGN, sid, count, len(slab), 1)
+    try:
+        engine.set_tuning(sid, chain_mode_max=0)
+        b.profile()
+        b.upload(count, sks[0], 1, np.zeros(count, np.uint32), slab, len(slab), offs, lens)
+        b.run()
+        names = [k for k, _, _ in b.kernel_ms()]
+        out = np.zeros(count * z["sig"], np.uint8)
+        b.download(out)
+    finally:
+        b.close()
+        engine.set_tuning(sid, **saved)
+    assert kernel in names and ("k_share" in names) == (count > 256)
+    assert [out[i * z["sig"]:(i + 1) * z["sig"]].tobytes() for i in range(count)] == _in_pieces(engine, sid, sks, msgs)
