@@ -5,14 +5,17 @@ HP_PARALLELISM, block-size and load-balancing switches).  Here the mapping is
 a runtime cuspx_tuning per parameter set, refined per (operation, batch-size
 bucket), and this module picks it by timing real batches on the device:
 
-  sign:   chain_mode_max (lane per chain vs lane per leaf for this batch
-          size), fors_lanes_log2 (lanes per FORS tree), tree_mode,
-          leaf_block, fors_block, tree_warps
-  verify: verify_item_max (one item per block at this size or not),
-          verify_mode (layered kernels, one persistent launch, or layered
-          kernels over length-sorted chains), and for each the chains per
-          warp / items per warp, block size, the persistent kernel's claim
-          threshold and the sorted mode's item groups
+  sign:   chain_mode_max (up to 256 items: lane per leaf, with leaf_block, or
+          lane per chain), fors_lanes_log2 (lanes per FORS tree), tree_mode,
+          fors_block, tree_warps
+  verify: verify_item_max (one launch at this size or not),
+          verify_mode (layered kernels, one launch, or layered kernels over
+          length-sorted chains), and for each the chains per warp, block
+          size, the sorted mode's item groups and, SHAKE, the persistent
+          kernel's items per warp and claim threshold
+
+Knobs that no kernel of the set and batch size reads are not swept: their
+trials would differ by noise alone, which could be recorded as a choice.
 
 Search is coordinate descent: each knob is swept with the others held, the
 best value kept, for two passes.  Every candidate is timed with CUDA events
@@ -54,6 +57,8 @@ VERIFY_SPACE = {
 }
 OP_NAMES = {OP_SIGN: "sign", OP_VERIFY: "verify"}
 SPEC_MAX_ITEMS = 64   # largest verify_spec_max the library accepts
+CHAIN_MODE_ITEMS = 256   # largest sign batch that chain_mode_max decides about
+SHAKE_KNOBS = ("verify_slots", "verify_claim_min")   # read by the persistent verify kernel, which only SHAKE sets have
 
 
 def cache_path():
@@ -120,13 +125,18 @@ def _time(batch, reps):
     return best
 
 
-def search_space(op, b):
+def search_space(op, b, sid=None):
     """The knob values swept for `op` in batch-size bucket b (None in the
-    tables stands for b itself)."""
+    tables stands for b itself), of set `sid` those that it reads there."""
     space = {k: [b if v is None else v for v in vals]
              for k, vals in (SIGN_SPACE if op == OP_SIGN else VERIFY_SPACE).items()}
     if "verify_spec_max" in space and b > SPEC_MAX_ITEMS:   # the speculative path covers up to 64 items
         space["verify_spec_max"] = [0]
+    if sid is not None:
+        drop = SHAKE_KNOBS if set_name(sid).startswith("sha256") else ()
+        if op == OP_SIGN and b > CHAIN_MODE_ITEMS:   # bucket_range(b) lies above it
+            drop = ("chain_mode_max", "leaf_block")
+        space = {k: v for k, v in space.items() if k not in drop}
     return space
 
 
@@ -161,13 +171,15 @@ def tune(eng, sid, op=OP_SIGN, count=1024, mlen=64, msgs=None, reps=2, passes=2,
         vb = eng.batch(OP_VERIFY, sid, count, len(slab), 1)
         vb.upload(count, pks[0], 1, kidx, slab, len(slab), offs, lens, sigs)
         batch = vb
-    space = search_space(op, b)
+    space = search_space(op, b, sid)
     cur = {k: v for k, v in eng.get_tuning_for(sid, op, count).items() if k in space}
     eng.set_tuning_for(sid, op, *bucket_range(b), **cur)
     best_ms = _time(batch, reps)
     for _ in range(passes):
         improved = False
         for knob, values in space.items():
+            if knob == "leaf_block" and cur["chain_mode_max"]:
+                continue   # read by the lane-per-leaf kernel alone
             for v in values:
                 if v == cur[knob]:
                     continue

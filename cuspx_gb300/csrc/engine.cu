@@ -342,9 +342,8 @@ int cuspx_create(int device, cuspx_ctx **out) {
         t.verify_mode = 2;
         // a robust item is several units per F and H: fewer items per warp
         // keep enough warps busy (16384 SHAKE-256f-robust: 2 slots 93.9 ms,
-        // 4 slots 98.9 ms; 4096 SHA-256-192f-robust 11.9 / 12.8 ms), except
-        // robust SHA-256 at n = 32 (4096 SHA-256-256f-robust 22.8 / 21.1 ms)
-        if (sd.robust && !(sd.hash == 0 && sd.n == 32)) t.verify_slots = 2;
+        // 4 slots 98.9 ms; no SHA-256 kernel reads it)
+        if (sd.hash == 1 && sd.robust) t.verify_slots = 2;
         // one launch of blocks of a few items for SHA-256 up to 128 items
         // whatever the mode; SHAKE takes the sorted layers at every size
         // above verify_spec_max (256f, 64 items: 2.29 ms, one item per block

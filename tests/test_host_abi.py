@@ -198,3 +198,21 @@ def test_autotune_search_space():
     sign = autotune.search_space(c.OP_SIGN, 1024)
     assert "verify_spec_max" not in sign and sign["chain_mode_max"] == [0, 256]
     assert [autotune.bucket(n) for n in (1, 2, 5, 64, 65, 4096)] == [1, 4, 16, 64, 256, 4096]
+
+
+def test_autotune_sweeps_knobs_that_are_read():
+    """SHA-256 sets have no persistent verify kernel, and sign batches above
+    256 items always run a lane per chain: the knobs of what a set and size
+    never run are not swept, the others are."""
+    import cuspx_gb300 as c
+    from cuspx_gb300 import autotune
+    sha, shake = c.set_id("sha256-128f-robust"), c.set_id("shake256-128f-robust")
+    for b in (1, 64, 256, 1024):
+        v = autotune.search_space(c.OP_VERIFY, b)
+        assert autotune.search_space(c.OP_VERIFY, b, shake) == v
+        assert autotune.search_space(c.OP_VERIFY, b, sha) == \
+            {k: x for k, x in v.items() if k not in ("verify_slots", "verify_claim_min")}
+        s = autotune.search_space(c.OP_SIGN, b)
+        for sid in (sha, shake):
+            assert autotune.search_space(c.OP_SIGN, b, sid) == \
+                {k: x for k, x in s.items() if b <= 256 or k not in ("chain_mode_max", "leaf_block")}
