@@ -95,6 +95,12 @@ static uint64_t long_msg_min(int set, int op, size_t count) {
     return !kSets[set].hash && group_messages(count) ? 4096 : long_msg_bytes(set, op, count);
 }
 
+// bytes of one layer's masks of a verify item (robust SHAKE, ShakeGroup::mask_lanes)
+size_t verify_mask_bytes(const SetDesc &s) {
+    const SetParams P = make_params(s);
+    return s.hash == 1 && s.robust ? (size_t)(P.len + 2 * P.hp) * P.n : 0;
+}
+
 // registration for other translation units of the library
 void ensure_registered() { register_all(); }
 }  // namespace cuspx
@@ -646,9 +652,6 @@ static GraphKey graph_key(const cuspx_batch *b) {
                     effective_tuning(b->ctx, b->set, b->op, b->count)};
 }
 
-// bytes of one layer's masks of an item (robust SHAKE, ShakeGroup::mask_lanes)
-static size_t shake_mask_bytes(const SetParams &P) { return (size_t)(P.len + 2 * P.hp) * P.n; }
-
 static int balloc(cuspx_batch *b, void **p, size_t bytes) {
     *p = nullptr;
     if (bytes == 0) return CUSPX_OK;
@@ -774,7 +777,7 @@ int cuspx_batch_create(cuspx_ctx *ctx, int op, int set, size_t capacity, size_t 
             b->vlists.stride = cap * P.len;
             A((void **)&b->vlists.tasks, 16 * b->vlists.stride * sizeof(uint32_t));
             A((void **)&b->vlists.cnt, (size_t)VerifyFork::kMaxGroups * P.d * 16 * sizeof(uint32_t));
-            if (sd.hash == 1 && sd.robust) A((void **)&b->vlists.masks, cap * shake_mask_bytes(P));
+            A((void **)&b->vlists.masks, cap * verify_mask_bytes(sd));
         }
     }
     if (rc != CUSPX_OK) {
@@ -997,7 +1000,7 @@ static void spec_scratch(cuspx_batch *b) {
     const size_t items = std::min<size_t>(b->cap, kSpecItems);
     const SetDesc &sd = kSets[b->set];
     const size_t ends = items * P.d * P.len * 16 * P.n;
-    const size_t masks = sd.hash == 1 && sd.robust ? items * P.d * shake_mask_bytes(P) : 0;
+    const size_t masks = items * P.d * verify_mask_bytes(sd);
     void *p = nullptr;
     if (cudaMalloc(&p, ends + masks) != cudaSuccess) {
         cudaGetLastError();

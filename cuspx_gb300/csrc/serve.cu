@@ -32,6 +32,7 @@
 
 namespace cuspx {
 SetParams make_params(const SetDesc &s);
+size_t verify_mask_bytes(const SetDesc &s);
 int batch_share_stream(cuspx_batch *b, cudaStream_t s);
 void batch_use_stream(cuspx_batch *b, cudaStream_t s);
 void batch_direct_launch(cuspx_batch *b, bool on);
@@ -225,13 +226,16 @@ struct cuspx_server {
 
 static int len_bucket(size_t mlen) { return mlen <= 1024 ? 0 : (mlen <= 65536 ? 1 : 2); }
 
-static size_t item_bytes(int op, const SetParams &P) {
+// device bytes that an item takes in a launch
+static size_t item_bytes(int op, int set) {
+    const SetParams P = make_params(kSets[set]);
     const size_t n = P.n;
     size_t b = sizeof(SignWork) + P.k * n + 64;
     if (op == CUSPX_OP_SIGN)
         b += P.sig_bytes + n + (size_t)P.d * ((size_t)1 << P.hp) * n + P.d * n + (size_t)P.d * P.len * 16 * n;
-    else   // signature, its length, WOTS+ public key, root, sorted-verify bucket entries
-        b += P.sig_bytes + 8 + (size_t)P.len * n + n + 16 * (size_t)P.len * sizeof(uint32_t);
+    else   // signature, its length, WOTS+ public key, root, sorted-verify bucket entries, masks
+        b += P.sig_bytes + 8 + (size_t)P.len * n + n + 16 * (size_t)P.len * sizeof(uint32_t) +
+             verify_mask_bytes(kSets[set]);
     return b;
 }
 
@@ -515,7 +519,7 @@ int cuspx_serve_create(cuspx_ctx *ctx, const cuspx_serve_config *cfg, cuspx_serv
                 g.set = set;
                 g.cls = lc;
                 g.P = make_params(kSets[set]);
-                g.per_item = item_bytes(op, g.P);
+                g.per_item = item_bytes(op, set);
                 double su, vu, opu;
                 op_units(kSets[set], su, vu, opu);
                 g.item_ops = (op == CUSPX_OP_SIGN ? su : vu) * opu;

@@ -22,7 +22,7 @@ struct Graph {
 };
 std::mutex g_mu;
 std::map<const char *, Alloc> g_allocs;
-int g_faults = 0, g_execs = 0, g_captures = 0;
+int g_faults = 0, g_execs = 0;
 thread_local int t_dev = 0;
 thread_local Graph *t_capture = nullptr;
 
@@ -67,7 +67,12 @@ void fake_launch(std::function<void()> kernel) {
 extern "C" {
 int fake_faults() { return g_faults; }
 int fake_live_execs() { return g_execs; }
-int fake_captures() { return g_captures; }
+size_t fake_live_bytes() {
+    std::lock_guard<std::mutex> lk(g_mu);
+    size_t n = 0;
+    for (auto &a : g_allocs) n += a.second.live ? a.second.bytes : 0;
+    return n;
+}
 
 cudaError_t cudaGetDeviceCount(int *n) { *n = 2; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { t_dev = d; return cudaSuccess; }
@@ -125,7 +130,6 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
     t_capture = new Graph;
-    g_captures++;
     return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) {

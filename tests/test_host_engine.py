@@ -207,3 +207,32 @@ def test_oneshot_memory_is_on_the_engines_device(fake):
     finally:
         eng.close()
         c.lib().cudaSetDevice(0)
+
+
+@pytest.mark.parametrize("setname", ["sha256-128f-simple", "sha256-256s-robust", "shake256-128f-simple",
+                                     "shake256-256f-robust"])
+def test_served_verify_request_counts_its_device_bytes(engine, fake, setname):
+    """what a verify request is admitted with is what an item more takes in a
+    batch, within the 64 bytes set aside for its offsets, indices and status"""
+    c = fake
+    live = c.lib().fake_live_bytes
+    live.restype = ctypes.c_size_t
+    sid = engine.set_id(setname)
+    z = c.set_sizes(sid)
+
+    def batch_bytes(items):
+        before = live()
+        b = engine.batch(c.OP_VERIFY, sid, items, 4096, 1)
+        got = live() - before
+        b.close()
+        return got
+
+    item = batch_bytes(101) - batch_bytes(100)
+    srv = c.Server(engine, max_batch=16, max_inflight=1)
+    try:
+        kid = srv.add_pubkeys(sid, [bytes(z["pk"])])[0]
+        assert srv.wait(srv.submit(c.OP_VERIFY, sid, kid, b"x" * 16, bytes(z["sig"])), 10_000_000)[1] == 0
+        counted = srv.stats()["bytes_peak"] - 16
+    finally:
+        srv.close()
+    assert item <= counted <= item + 64
