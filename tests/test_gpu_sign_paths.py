@@ -277,3 +277,32 @@ def test_chain_mode_max_decides_up_to_256_items(engine, count, kernel):
         engine.set_tuning(sid, **saved)
     assert kernel in names and ("k_share" in names) == (count > 256)
     assert [out[i * z["sig"]:(i + 1) * z["sig"]].tobytes() for i in range(count)] == _in_pieces(engine, sid, sks, msgs)
+
+
+@pytest.mark.parametrize("setname", ["sha256-128f-simple", "shake256-192f-robust"])
+def test_oneshot_inputs_packed_and_apart(setname):
+    """one engine's calls whose inputs go up in one copy, in a growing one and
+    buffer by buffer (above 1 MiB), there and back, with and without
+    randomisers; each shape three times (launched, captured, replayed), a key
+    row with a wrong root and a signature of a wrong length among them"""
+    import cuspx_gb300
+    rng = random.Random(16)
+    o = _oracle(setname)
+    eng = cuspx_gb300.Engine(0)
+    try:
+        sid = eng.set_id(setname)
+        pk, sk = o.seed_keypair(rng.randbytes(o.p.seed_bytes))
+        bad = sk[:-1] + bytes([sk[-1] ^ 1])
+        for count, size, opt in ((3, 40, False), (3, 900, True), (2, 40, True), (3, 400_000, True), (3, 40, True),
+                                 (3, 40, False), (3, 400_000, False), (2, 900, False)):
+            msgs = [rng.randbytes(size + i) for i in range(count)]
+            rand = [rng.randbytes(o.p.n) for _ in range(count)] if opt else None
+            want = [o.sign(m, sk, rand[i] if opt else None) for i, m in enumerate(msgs[:-1])]
+            for _ in range(3):
+                sigs, st = eng.sign_batch(sid, [sk] * (count - 1) + [bad], msgs, rand)
+                assert list(st) == [0] * (count - 1) + [-2] and sigs[:-1] == want
+                got = eng.verify_batch(sid, [pk] * (2 * count - 2), msgs[:-1] * 2, want * 2,
+                                       siglens=[len(x) for x in want] + [len(x) - 1 for x in want])
+                assert list(got) == [0] * (count - 1) + [-1] * (count - 1)
+    finally:
+        eng.close()

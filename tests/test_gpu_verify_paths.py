@@ -109,3 +109,58 @@ def test_lanes_in_item_groups(engine, pool, setname, counts):
     """the sizes between which several item groups run with lanes in the layer kernel"""
     for count in counts:
         _check(engine, engine.set_id(setname), pool(setname), count, count)
+
+
+@pytest.mark.parametrize("setname,count", [("sha256-128f-simple", 2049), ("sha256-192s-simple", 2049),
+                                           ("sha256-256f-simple", 2049), ("sha256-128s-robust", 4097),
+                                           ("sha256-192s-robust", 4097), ("sha256-256f-robust", 4097),
+                                           ("shake256-128f-simple", 2049), ("shake256-192s-simple", 2049),
+                                           ("shake256-256s-simple", 2049), ("shake256-128s-robust", 8193),
+                                           ("shake256-192s-robust", 8193), ("shake256-256s-robust", 8193)])
+def test_layer_thread_per_item(engine, pool, setname, count):
+    """one item group past the sizes of the lanes and warps per item: a thread
+    per item in the layer kernel, its last block part full"""
+    sid = engine.set_id(setname)
+    saved = engine.get_tuning(sid)
+    try:
+        engine.set_tuning(sid, verify_groups=1)
+        _check(engine, sid, pool(setname), count, count)
+    finally:
+        engine.set_tuning(sid, **saved)
+
+
+@pytest.mark.parametrize("setname", ["shake256-128f-simple", "shake256-192f-robust", "shake256-256s-simple"])
+@pytest.mark.parametrize("slots,block", [(1, 32), (2, 128)])
+def test_persistent_kernel_refills_slots(engine, pool, setname, slots, block):
+    """more items than all resident warps hold at once (152 SMs x 32 blocks of
+    a warp, or x 16 warps of two items), a wrong-length signature in five: warps
+    take new items as theirs finish"""
+    import numpy as np
+    import cuspx_gb300 as c
+    count, items = 6000, pool(setname)
+    sid = engine.set_id(setname)
+    z = c.set_sizes(sid)
+    slab, offs, lens = c.pack_messages([items[i % 64][1] for i in range(count)])
+    sigs = np.frombuffer(b"".join(s for _, _, s in items), np.uint8).reshape(64, -1)[np.arange(count) % 64].copy()
+    rng = np.random.default_rng(count + slots)
+    bad = rng.random(count) < 0.4
+    sigs[bad, rng.integers(0, z["sig"], count)[bad]] ^= 1
+    short = rng.random(count) < 0.2
+    siglen = np.where(short, z["sig"] - 1, z["sig"]).astype(np.uint64)
+    saved = engine.get_tuning(sid)
+    b = engine.batch(c.OP_VERIFY, sid, count, len(slab), count)
+    got = np.zeros(count, np.int32)
+    try:
+        engine.set_tuning(sid, verify_mode=2, verify_sorted_min=0, verify_spec_max=0, verify_item_max=0,
+                          verify_slots=slots, verify_block=block)
+        b.profile()
+        b.upload(count, b"".join(items[i % 64][0] for i in range(count)), count, None, slab, len(slab), offs, lens,
+                 sigs.reshape(-1), siglen)
+        b.run()
+        names = [k for k, _, _ in b.kernel_ms()]
+        b.download(None, None, got)
+    finally:
+        b.close()
+        engine.set_tuning(sid, **saved)
+    assert "k_verify_hyper" in names
+    assert np.array_equal(got, np.where(bad | short, -1, 0))
