@@ -584,7 +584,7 @@ struct Family {
         const bool spec = tu.verify_mode != 3 && tu.verify_spec_max > 0 && A.count <= (uint32_t)tu.verify_spec_max &&
                           vl && vl->cand && A.count <= vl->cand_items &&
                           P.len1 == 2 * N && P.len2 == 3;
-        const bool by_size = tu.verify_sorted_min > 0 && A.count >= (uint32_t)tu.verify_sorted_min && !spec;
+        const bool by_size = tu.verify_sorted_min > 0 && A.count >= (uint32_t)tu.verify_sorted_min;
         const bool direct = vl && vl->direct;   // each launch is a host launch (serving)
         const bool item = A.count <= (uint32_t)(tu.verify_item_max > 0 ? tu.verify_item_max : 0) ||
                           (HF::kShake && direct && A.count <= 128);

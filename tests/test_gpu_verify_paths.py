@@ -129,6 +129,41 @@ def test_layer_thread_per_item(engine, pool, setname, count):
         engine.set_tuning(sid, **saved)
 
 
+@pytest.mark.parametrize("setname", ["sha256-128f-simple", "sha256-256s-robust", "shake256-192f-robust"])
+def test_sorted_min_below_spec_max(engine, pool, setname):
+    """verify_sorted_min decides whatever verify_mode says, also for batches that
+    the speculative chains would take, and only from its size on"""
+    import numpy as np
+    import cuspx_gb300 as c
+    sid = engine.set_id(setname)
+    z = c.set_sizes(sid)
+    saved = engine.get_tuning(sid)
+    ran = {}
+    try:
+        engine.set_tuning(sid, verify_sorted_min=8, verify_spec_max=16, verify_item_max=0)
+        for count in (7, 8, 16):
+            items = pool(setname)[:count]
+            slab, offs, lens = c.pack_messages([m for _, m, _ in items])
+            sigs = np.frombuffer(b"".join(s for _, _, s in items), np.uint8).reshape(count, z["sig"]).copy()
+            sigs[1, 3] ^= 1
+            b = engine.batch(c.OP_VERIFY, sid, count, len(slab), count)
+            got = np.zeros(count, np.int32)
+            try:
+                b.profile()
+                b.upload(count, b"".join(p for p, _, _ in items), count, None, slab, len(slab), offs, lens,
+                         sigs.reshape(-1))
+                b.run()
+                ran[count] = {k for k, _, _ in b.kernel_ms()}
+                b.download(None, None, got)
+            finally:
+                b.close()
+            assert [int(x) for x in got] == [-1 if i == 1 else 0 for i in range(count)]
+    finally:
+        engine.set_tuning(sid, **saved)
+    assert "k_vspec_walk" in ran[7]
+    assert all("k_vsort_layer" in ran[n] and "k_vspec_walk" not in ran[n] for n in (8, 16))
+
+
 @pytest.mark.parametrize("setname", ["shake256-128f-simple", "shake256-192f-robust", "shake256-256s-simple"])
 @pytest.mark.parametrize("slots,block", [(1, 32), (2, 128)])
 def test_persistent_kernel_refills_slots(engine, pool, setname, slots, block):
