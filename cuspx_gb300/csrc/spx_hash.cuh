@@ -316,13 +316,19 @@ SPX_DEV void sha256_compress(uint32_t s[8], uint32_t w[16]) {
 // all: -19%): those multiplies hold the issue port longer than the funnel
 // shifts hold the ALU pipe.
 // ---------------------------------------------------------------------------
-__constant__ static const uint64_t KECCAK_RC[24] = {
-    0x0000000000000001ull, 0x0000000000008082ull, 0x800000000000808aull, 0x8000000080008000ull,
-    0x000000000000808bull, 0x0000000080000001ull, 0x8000000080008081ull, 0x8000000000008009ull,
-    0x000000000000008aull, 0x0000000000000088ull, 0x0000000080008009ull, 0x000000008000000aull,
-    0x000000008000808bull, 0x800000000000008bull, 0x8000000000008089ull, 0x8000000000008003ull,
-    0x8000000000008002ull, 0x8000000000000080ull, 0x000000000000800aull, 0x800000008000000aull,
-    0x8000000080008081ull, 0x8000000000008080ull, 0x0000000080000001ull, 0x8000000080008008ull};
+struct KeccakRc {
+    uint64_t v[24];
+};
+__host__ __device__ constexpr KeccakRc keccak_rc() {
+    return {{
+        0x0000000000000001ull, 0x0000000000008082ull, 0x800000000000808aull, 0x8000000080008000ull,
+        0x000000000000808bull, 0x0000000080000001ull, 0x8000000080008081ull, 0x8000000000008009ull,
+        0x000000000000008aull, 0x0000000000000088ull, 0x0000000080008009ull, 0x000000008000000aull,
+        0x000000008000808bull, 0x800000000000008bull, 0x8000000000008089ull, 0x8000000000008003ull,
+        0x8000000000008002ull, 0x8000000000000080ull, 0x000000000000800aull, 0x800000008000000aull,
+        0x8000000080008081ull, 0x8000000000008080ull, 0x0000000080000001ull, 0x8000000080008008ull}};
+}
+static __constant__ KeccakRc KECCAK_RC = keccak_rc();
 
 SPX_DEV uint64_t lane_of(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
 
@@ -363,7 +369,7 @@ SPX_DEV void keccak_round(uint64_t A[25], uint64_t rc) {
 
 SPX_DEV void keccak_f1600(uint64_t A[25]) {
 #pragma unroll 2
-    for (int r = 0; r < 24; r++) keccak_round(A, KECCAK_RC[r]);
+    for (int r = 0; r < 24; r++) keccak_round(A, KECCAK_RC.v[r]);
 }
 
 // The permutation of a short input's state, of which the caller reads only
@@ -372,21 +378,24 @@ SPX_DEV void keccak_f1600(uint64_t A[25]) {
 // instructions) and the last one computes the lanes that are read and no
 // others (about 50 instructions for two lanes).
 SPX_DEV void keccak_f1600_short(uint64_t A[25]) {
-    keccak_round(A, 0x0000000000000001ull);
+    constexpr KeccakRc rc = keccak_rc();
+    keccak_round(A, rc.v[0]);
 #pragma unroll 2
-    for (int r = 1; r < 23; r++) keccak_round(A, KECCAK_RC[r]);
-    keccak_round(A, 0x8000000080008008ull);
+    for (int r = 1; r < 23; r++) keccak_round(A, KECCAK_RC.v[r]);
+    keccak_round(A, rc.v[23]);
 }
 
 // ---------------------------------------------------------------------------
-// The same permutation on bit-interleaved lanes: the low half of a lane holds
+// The same permutation on bit-interleaved lanes (the bit interleaving of the Keccak
+// team's "Keccak implementation overview"): the low half of a lane holds
 // its even bits, the high half its odd ones, so a rotation by 2k rotates both
 // halves by k and one by 2k + 1 swaps them and rotates them by k + 1 and k.
 // Rotations by one (theta's five, rho's first) then cost one funnel shift
 // instead of two: 174 ALU instructions a round instead of 180.  For chains of
 // permutations, which convert once per chain.
 // ---------------------------------------------------------------------------
-// even bits of x to the low half, odd ones to the high half, and back
+// even bits of x to the low half, odd ones to the high half, and back: the
+// masked swaps of the shuffles in Warren's "Hacker's Delight"
 __host__ __device__ constexpr uint32_t unzip32(uint32_t x) {
     uint32_t t = (x ^ (x >> 1)) & 0x22222222u;
     x ^= t ^ (t << 1);
@@ -415,22 +424,12 @@ __host__ __device__ constexpr uint64_t deinterleave(uint64_t x) {
     const uint32_t e = (uint32_t)x, o = (uint32_t)(x >> 32);
     return (uint64_t)zip32((e >> 16) | (o & 0xffff0000u)) << 32 | zip32((e & 0xffffu) | (o << 16));
 }
-struct KeccakIlRc {
-    uint64_t v[24];
-};
-__host__ __device__ constexpr KeccakIlRc keccak_il_rc() {
-    constexpr uint64_t rc[24] = {
-        0x0000000000000001ull, 0x0000000000008082ull, 0x800000000000808aull, 0x8000000080008000ull,
-        0x000000000000808bull, 0x0000000080000001ull, 0x8000000080008081ull, 0x8000000000008009ull,
-        0x000000000000008aull, 0x0000000000000088ull, 0x0000000080008009ull, 0x000000008000000aull,
-        0x000000008000808bull, 0x800000000000008bull, 0x8000000000008089ull, 0x8000000000008003ull,
-        0x8000000000008002ull, 0x8000000000000080ull, 0x000000000000800aull, 0x800000008000000aull,
-        0x8000000080008081ull, 0x8000000000008080ull, 0x0000000080000001ull, 0x8000000080008008ull};
-    KeccakIlRc k{};
-    for (int i = 0; i < 24; i++) k.v[i] = interleave(rc[i]);
+__host__ __device__ constexpr KeccakRc keccak_il_rc() {
+    KeccakRc k = keccak_rc();
+    for (int i = 0; i < 24; i++) k.v[i] = interleave(k.v[i]);
     return k;
 }
-static __constant__ KeccakIlRc KECCAK_IL_RC = keccak_il_rc();
+static __constant__ KeccakRc KECCAK_IL_RC = keccak_il_rc();
 
 // rotate left by a constant c in 0..63
 SPX_DEV uint64_t rotl64_il(uint64_t x, int c) {
@@ -465,10 +464,11 @@ SPX_DEV void keccak_round_il(uint64_t A[25], uint64_t rc) {
 }
 // keccak_f1600_short on interleaved lanes
 SPX_DEV void keccak_f1600_short_il(uint64_t A[25]) {
-    keccak_round_il(A, interleave(0x0000000000000001ull));
+    constexpr KeccakRc rc = keccak_il_rc();
+    keccak_round_il(A, rc.v[0]);
 #pragma unroll 2
     for (int r = 1; r < 23; r++) keccak_round_il(A, KECCAK_IL_RC.v[r]);
-    keccak_round_il(A, interleave(0x8000000080008008ull));
+    keccak_round_il(A, rc.v[23]);
 }
 
 // ---------------------------------------------------------------------------
@@ -532,7 +532,7 @@ SPX_DEV void warp_keccak_f1600(uint64_t &a, const KeccakLane &k, uint32_t lane) 
         const uint64_t b = shfl64(((uint64_t)hi << 32) | lo, k.src);
         // chi + iota
         a = b ^ (~shfl64(b, k.rp1) & shfl64(b, k.rp2));
-        if (lane == 0) a ^= KECCAK_RC[r];
+        if (lane == 0) a ^= KECCAK_RC.v[r];
     }
 }
 
