@@ -1330,7 +1330,6 @@ struct OneshotJob {
     bool done = false;
 };
 
-// Run jobs of one (op, set) as one batch; under ctx->mu.
 // Most input bytes of a one-shot call that go to the device in one copy, and
 // its outputs back in one: a call of one item made four to six small copies
 // before its launch and two after it, each 1.5 to 3 us of the host's time and
@@ -1369,6 +1368,7 @@ static bool upload_packed(cuspx_batch *b, size_t count, const uint8_t *in, size_
     return true;
 }
 
+// Run jobs of one (op, set) as one batch; under ctx->mu.
 static int oneshot_run(cuspx_ctx *ctx, int op, int set, const std::vector<OneshotJob *> &jobs) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     CK(cudaSetDevice(ctx->device), ctx);   // any thread may call

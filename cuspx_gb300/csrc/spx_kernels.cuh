@@ -6,8 +6,11 @@
 // batch of thousands of signatures fills all 152 SMs:
 //
 //   k_sign_msg      thread / signature   PRF_msg, H_msg -> R, FORS digest, tree, leaf
-//   k_sign_msg_wide warp / signature     the same for messages of >= 2 KiB (SHAKE)
-//   k_sign_msg_pair 2 warps / 32 sigs    the same for messages of >= 2 KiB (SHA-256):
+//                                        (small SHA-256 batches: k_sign_msg_group, warp
+//                                        / signature, spx_vgroup.cuh)
+//   k_sign_msg_wide warp / signature     the same for long messages (SHAKE; from how
+//                                        many bytes on: long_msg_bytes, engine.cu)
+//   k_sign_msg_pair 2 warps / 32 sigs    the same for long messages (SHA-256):
 //                                        schedule warp + rounds warp per message
 //   k_share         thread / (item, upper layer)  trees that items of one key share
 //   k_fors_sign     2^g lanes / FORS tree leaves (PRF+F), per-lane subtree stack,
@@ -23,7 +26,7 @@
 //   k_sign_finish   block / signature    WOTS signatures gathered from the recorded
 //                                        chains
 //
-// Verify: k_verify_msg (+ k_verify_msg_pair / _wide) -> k_verify_fors -> the
+// Verify: k_verify_msg or _group (+ k_verify_msg_pair / _wide) -> k_verify_fors -> the
 // hypertree: for tiny batches every chain run from all 16 start steps, then a
 // serial walk (k_vspec_cand + k_vspec_walk_*, spx_vsort.cuh); for SHA-256 up
 // to about 4 items an SM one launch of blocks that keep 2 to 8 items

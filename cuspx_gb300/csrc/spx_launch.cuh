@@ -461,13 +461,16 @@ struct Family {
     // none of these batches) and how many groups at most.  Simple f sets, 4
     // lanes: 128f 2048 items 1.384 ms (one group of 8 lanes 1.461), 4096 2.161
     // (a thread an item 2.20), 8192 3.586 / 3.649, but 12000 4.97 / 4.85; 192f
-    // 3000 items 2.71 / 3.01; 256f 3000 2.95 / 3.22, but 4096 3.77 / 3.68; the
+    // 3000 items 2.76 / 3.03, 5000 3.86 / 3.89, 6500 4.52 / 4.71, 8192 5.44 / 5.53
+    // (8193, a thread an item: 5.54); 256f 3000 2.95 / 3.22, but 4096 3.77 / 3.68; the
     // s sets, whose layers are few, lose (128s, 4096: 0.90 / 0.86).  Robust
     // sets, whose H masks the lanes share out, in two groups, 8 lanes at n = 32
     // (256f 3000 items 6.69 / 7.22, 8192 16.6 / 17.9; 256s 3000 3.51 / 3.89,
     // but 2048 2.76 / 2.62) and 4 at n < 32 (192f 6000 items 8.80 / 10.3, 12000
-    // 17.1 / 18.9; 128f 8192 7.30 / 7.73, but 4096 4.39 / 4.11; 192s 4200 2.56
-    // / 3.30), up to 32768 items, the largest measured.
+    // 17.1 / 18.8; 128f 8192 7.30 / 7.73, but 4096 4.39 / 4.11; 192s 4200 2.56
+    // / 3.30).  Their gain shrinks with the batch but had not ended at the largest
+    // measured (192f, 65536 items: 93.8 / 96.6 ms; 256f 49152: 101.0 / 102.8; 128s
+    // 65536: 19.3 / 20.1), so they have no upper end.
     static int side_lanes(const SetParams &P, uint32_t count, int &groups) {
         if (HF::kShake) return 0;
         if (!HF::kRobust) {

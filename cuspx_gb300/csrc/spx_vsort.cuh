@@ -512,9 +512,9 @@ __global__ void __launch_bounds__(128) k_vsort_chains(SetParams P, VerifyArgs A,
 // known up front, so k_vspec_cand computes every chain of every layer from
 // each of its 16 possible start steps at once, on SMs that a tiny batch
 // leaves idle (16 x d x len chain runs per item, 120 F per chain position),
-// and k_vspec_walk then walks the layers with T_len and the auth path only,
-// taking each chain's end by its digit: ~13 dependent units per layer
-// instead of ~20.
+// and k_vspec_walk_group (SHA-256) or _warp (SHAKE) then walks the layers with
+// T_len and the auth path only, taking each chain's end by its digit: ~13
+// dependent units per layer instead of ~20.
 // ---------------------------------------------------------------------------
 
 // thread per (start step, item, layer, chain): start-step-major, so a warp's
