@@ -358,13 +358,17 @@ struct Family {
         return g;
     }
 
+    static bool latency_mapping(uint32_t count, const Tuning &tu) {
+        return count <= (uint32_t)tu.chain_mode_max && count <= kChainModeItems;
+    }
+
     // First layer whose trees are looked for among the items (0: none).  A
     // layer of 8 trees per item still saves about 6% of its work if all items
     // have one key; the two memsets, k_share and k_share_leaves take 21 us at
     // 301 items and 25 to 50 from 1024 to 4096, so batches of the latency
     // mapping go without.
     static int share_layer(const SetParams &P, uint32_t count, const Tuning &tu, const ShareArgs &S) {
-        if (!S.tab || count <= 64 || count <= (uint32_t)tu.chain_mode_max) return 0;
+        if (!S.tab || count <= 64 || latency_mapping(count, tu)) return 0;
         return shared_layer0(P, count);
     }
 
@@ -423,8 +427,7 @@ struct Family {
         if (split) cudaEventRecord(fk->join, sf);
         {
             LeafArgs L{A.count, 0, P.d, A.sk, A.work, A.leaves, A.chains, A.ends, 0, 0, false, A.share, nullptr};
-            leaves(P, L, tu, s, pt, A.ends_trees,
-                   A.count <= (uint32_t)tu.chain_mode_max && A.count <= kChainModeItems);
+            leaves(P, L, tu, s, pt, A.ends_trees, latency_mapping(A.count, tu));
         }
         {
             TreeArgs T{A.count, 0, P.d, A.sk, A.work, A.leaves, A.roots, A.sig, A.share, nullptr};

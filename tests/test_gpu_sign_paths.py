@@ -306,3 +306,30 @@ def test_oneshot_inputs_packed_and_apart(setname):
                 assert list(got) == [0] * (count - 1) + [-1] * (count - 1)
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("count", [256, 257])
+def test_chain_mode_max_above_256_items(engine, count):
+    """a chain_mode_max above the sizes that it decides about: larger batches
+    still share trees"""
+    import numpy as np
+    import cuspx_gb300 as c
+    sid = engine.set_id("sha256-128f-simple")
+    z = c.set_sizes(sid)
+    pks, sks, msgs = _requests(engine, sid, count, 1, 16)
+    slab, offs, lens = c.pack_messages(msgs)
+    saved = engine.get_tuning(sid)
+    b = engine.batch(c.OP_SIGN, sid, count, len(slab), 1)
+    try:
+        engine.set_tuning(sid, chain_mode_max=4096)
+        b.profile()
+        b.upload(count, sks[0], 1, np.zeros(count, np.uint32), slab, len(slab), offs, lens)
+        b.run()
+        names = [k for k, _, _ in b.kernel_ms()]
+        out = np.zeros(count * z["sig"], np.uint8)
+        b.download(out)
+    finally:
+        b.close()
+        engine.set_tuning(sid, **saved)
+    assert ("k_share" in names) == (count > 256)
+    assert [out[i * z["sig"]:(i + 1) * z["sig"]].tobytes() for i in range(count)] == _in_pieces(engine, sid, sks, msgs)
