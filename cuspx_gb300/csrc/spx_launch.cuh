@@ -23,14 +23,14 @@ struct Tuning {
     int tree_warps = 4;      // warps per block for k_trees (upper bound)
     int chains_per_warp = 64;  // (item, chain) tasks per warp in k_verify_chains
     int verify_mode = 0;     // 0 layered kernels, 1 one thread per item over all layers,
-                             // 2 persistent hypertree kernel, 3 layered with sorted chains
+                             // 2 one launch over the hypertree, 3 layered with sorted chains
     int fors_lanes_log2 = 5; // lanes per FORS tree = 2^g (0: lane per tree, 5: warp per tree)
     int tree_mode = 0;       // 0 warp per XMSS tree, 1 lane per tree (subtrees of height <= 4)
     int chain_mode_max = 64; // sign batches of at most this many items take the T_len kernel of the
                              // lower latency; 0: XMSS leaves a lane each (up to kChainModeItems, and
                              // key generation)
-    int verify_slots = 4;    // most items per warp in the persistent verify kernel
-    int verify_item_max = 0; // batches of at most this many items verify one item per block
+    int verify_slots = 4;    // most items per warp in the persistent verify kernel (SHAKE)
+    int verify_item_max = 0; // batches of at most this many items verify in one launch
     int verify_claim_min = 1;// persistent verify: free lanes before chains are handed out
     int verify_groups = 4;   // sorted verify: item groups on their own streams (1..8)
     int verify_sorted_min = 0; // batches of at least this many items verify as verify_mode 3 (0: never by size)

@@ -94,7 +94,8 @@ typedef struct {
                              item) */
     int verify_sorted_min;/* verify batches of at least this many items run the sorted layered
                              verify whatever verify_mode says (0: only with verify_mode 3);
-                             batches up to verify_item_max still run one item per block */
+                             batches up to verify_item_max still run in one launch.  Decides
+                             before verify_spec_max */
     int verify_spec_max;  /* verify batches of at most this many items (0..64; 0: never) first
                              run every WOTS+ chain of every layer from each of its 16 possible
                              start steps in parallel, then walk the layers with T_len and the
